@@ -201,10 +201,13 @@ void launch_lu_step(const int* flist, int nf, int maxN, const FrontDev* fr, doub
 void launch_lu_solve(bool forward, const int* flist, int nf, int maxN, const FrontDev* fr,
                      const double* F, const int* ipiv, const int* dofs, double* X, int64_t ldx,
                      int nrhs, double* W, const int64_t* woff, cudaStream_t st);
-// Apply, upward part, of LU fronts (the downward part is launch_apply_down).
+// Apply of LU fronts, upward and downward part.
 void launch_lu_apply_up(const int* flist, int nf, const FrontDev* fr, const double* F,
                         const int* ipiv, const int* dofs, double* X, int64_t ldx, int nrhs,
                         double* W, const int64_t* woff, double* Tb, cudaStream_t st);
+void launch_lu_apply_down(const int* flist, int nf, const FrontDev* fr, const double* F,
+                          const int* dofs, int64_t ldx, int nrhs, double* W, const int64_t* woff,
+                          const double* Tb, cudaStream_t st);
 
 // Stencil assembly (width 1): recompute the CSR values of the rows of the
 // cells in [lo, hi) from the node coefficients; with `flag`, record which rows
@@ -238,16 +241,16 @@ template <class T>
 void launch_sep_gather(const int* slist, int ns, const SepDev* sp, const int* dofs, T* X,
                        int64_t ldx, int nrhs, const T* W, const int64_t* woff, const FrontDev* fr,
                        cudaStream_t st);
+// Factored-operator application of Cholesky fronts (kernels_apply.cu): both
+// launches over the fronts of all levels, in place on X; the boundary rows'
+// L21 t are left in W for the separator gathers.  apply_items lists the
+// (front, first column) and (front, first row) pairs.
+void apply_items(const std::vector<int>& n, const std::vector<int>& N, std::vector<int>& cols,
+                 std::vector<int>& rows);
 template <class T>
-void launch_apply_up(const int* flist, int nf, const FrontDev* fr, const T* F, const int* dofs, T* X,
-                     int64_t ldx, int nrhs, T* W, const int64_t* woff, T* Tb, cudaStream_t st);
-template <class T>
-void launch_apply_down(const int* flist, int nf, const FrontDev* fr, const T* F, const int* dofs,
-                       int64_t ldx, int nrhs, T* W, const int64_t* woff, const T* Tb,
-                       cudaStream_t st);
-template <class T>
-void launch_root_apply(int f, const FrontDev* fr, const T* F, const int* dofs, T* X, int64_t ldx,
-                       int nrhs, T* W, const int64_t* woff, cudaStream_t st);
+void launch_apply(const int* cols, int ncols, const int* rows, int nrows, const FrontDev* fr,
+                  const T* F, const int* dofs, T* X, int64_t ldx, int nrhs, T* W,
+                  const int64_t* woff, cudaStream_t st);
 
 // Vector kernels of the mixed-precision solve (kernels_vec.cu).
 void launch_diag_scale(const int* rp, const int* ci, const double* va, int n, double* s,

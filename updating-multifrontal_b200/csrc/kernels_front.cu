@@ -1077,72 +1077,20 @@ __global__ void __launch_bounds__(ST) k_sep_gather(const int* __restrict__ slist
   }
 }
 
-// Apply, upward part: t = L11^T b_piv + L21^T b_bd ; b_piv = L11 t ; T(piv) = t.
-template <class T>
-__device__ void front_apply_up(const FrontDev& d, const T* __restrict__ A, T* W,
-                               T* Tt, int nrhs) {
-  // W holds [b_piv; b_bd] (N x nrhs); Tt receives t (n x nrhs, ld n).
-  const int N = d.N, n = d.n, ld = d.ld, tid = threadIdx.x;
-  const int lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
-  for (int jc = warp; jc < n * nrhs; jc += nw) {
-    const int j = jc % n, c = jc / n;
-    const T* w = W + (int64_t)c * N;
-    T s = T(0);
-    for (int r = j + lane; r < N; r += 32) s += A[r + (int64_t)j * ld] * w[r];
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if (lane == 0) Tt[j + (int64_t)c * n] = s;
-  }
-  __syncthreads();
-  for (int idx = tid; idx < n * nrhs; idx += blockDim.x) {
-    const int r = idx % n, c = idx / n;
-    const T* t = Tt + (int64_t)c * n;
-    T s = T(0);
-    for (int j = 0; j <= r; j++) s += A[r + (int64_t)j * ld] * t[j];
-    W[r + (int64_t)c * N] = s;
-  }
-  __syncthreads();
-}
-
-template <class T>
-__global__ void __launch_bounds__(ST) k_apply_up(const int* __restrict__ flist,
-                                                 const FrontDev* __restrict__ fr,
-                                                 const T* __restrict__ F,
-                                                 const int* __restrict__ dofs, T* X,
-                                                 int64_t ldx, int nrhs, T* Wb,
-                                                 const int64_t* __restrict__ woff, T* Tb) {
-  const int f = flist[blockIdx.x];
-  const FrontDev d = fr[f];
-  T* W = Wb + woff[f] * nrhs;
-  const int* dl = dofs + d.dof_off;
-  for (int idx = threadIdx.x; idx < d.N * nrhs; idx += blockDim.x) {
-    const int i = idx % d.N, c = idx / d.N;
-    W[idx] = X[dl[i] + (int64_t)c * ldx];
-  }
-  __syncthreads();
-  T* Tt = W + (int64_t)d.N * nrhs;  // second half of the front's workspace
-  front_apply_up(d, F + d.off, W, Tt, nrhs);
-  for (int idx = threadIdx.x; idx < d.n * nrhs; idx += blockDim.x) {
-    const int i = idx % d.n, c = idx / d.n;
-    X[dl[i] + (int64_t)c * ldx] = W[i + (int64_t)c * d.N];
-    Tb[dl[i] + (int64_t)c * ldx] = Tt[i + (int64_t)c * d.n];
-  }
-}
-
-// Apply, downward part: W[n,N) = L21 t (t read from T by DOF).
-template <class T>
-__global__ void __launch_bounds__(ST) k_apply_down(const int* __restrict__ flist,
+// Apply, downward part, of a pivoted LU front: W[n,N) = L21 t (t read from T by DOF).
+__global__ void __launch_bounds__(ST) k_lu_apply_down(const int* __restrict__ flist,
                                                    const FrontDev* __restrict__ fr,
-                                                   const T* __restrict__ F,
+                                                   const double* __restrict__ F,
                                                    const int* __restrict__ dofs, int64_t ldx,
-                                                   int nrhs, T* Wb,
+                                                   int nrhs, double* Wb,
                                                    const int64_t* __restrict__ woff,
-                                                   const T* __restrict__ Tb) {
+                                                   const double* __restrict__ Tb) {
   const int f = flist[blockIdx.x];
   const FrontDev d = fr[f];
-  T* W = Wb + woff[f] * nrhs;
+  double* W = Wb + woff[f] * nrhs;
   const int* dl = dofs + d.dof_off;
-  const T* A = F + d.off;
-  T* Tt = W + (int64_t)d.N * nrhs;
+  const double* A = F + d.off;
+  double* Tt = W + (int64_t)d.N * nrhs;
   for (int idx = threadIdx.x; idx < d.n * nrhs; idx += blockDim.x) {
     const int i = idx % d.n, c = idx / d.n;
     Tt[i + (int64_t)c * d.n] = Tb[dl[i] + (int64_t)c * ldx];
@@ -1150,32 +1098,10 @@ __global__ void __launch_bounds__(ST) k_apply_down(const int* __restrict__ flist
   __syncthreads();
   for (int idx = threadIdx.x; idx < d.m * nrhs; idx += blockDim.x) {
     const int r = d.n + idx % d.m, c = idx / d.m;
-    const T* t = Tt + (int64_t)c * d.n;
-    T s = T(0);
+    const double* t = Tt + (int64_t)c * d.n;
+    double s = double(0);
     for (int j = 0; j < d.n; j++) s += A[r + (int64_t)j * d.ld] * t[j];
     W[r + (int64_t)c * d.N] = s;
-  }
-}
-
-template <class T>
-__global__ void __launch_bounds__(ST) k_root_apply(int f, const FrontDev* __restrict__ fr,
-                                                   const T* __restrict__ F,
-                                                   const int* __restrict__ dofs, T* X,
-                                                   int64_t ldx, int nrhs, T* Wb,
-                                                   const int64_t* __restrict__ woff) {
-  const FrontDev d = fr[f];
-  T* W = Wb + woff[f] * nrhs;
-  const int* dl = dofs + d.dof_off;
-  for (int idx = threadIdx.x; idx < d.N * nrhs; idx += blockDim.x) {
-    const int i = idx % d.N, c = idx / d.N;
-    W[idx] = X[dl[i] + (int64_t)c * ldx];
-  }
-  __syncthreads();
-  T* Tt = W + (int64_t)d.N * nrhs;
-  front_apply_up(d, F + d.off, W, Tt, nrhs);
-  for (int idx = threadIdx.x; idx < d.n * nrhs; idx += blockDim.x) {
-    const int i = idx % d.n, c = idx / d.n;
-    X[dl[i] + (int64_t)c * ldx] = W[i + (int64_t)c * d.N];
   }
 }
 
@@ -1327,7 +1253,7 @@ __global__ void __launch_bounds__(ST) k_lu_solve_bwd(const int* __restrict__ fli
 
 // Apply, upward part, of a pivoted LU front: u = U11 b_piv + U12 b_bd,
 // b_piv <- P^T L11 u (= A22 t with t = b_piv + XR b_bd), T(piv) = u; the
-// downward part W[n,N) = L21 u (= XL A22 t) is k_apply_down's.
+// downward part W[n,N) = L21 u (= XL A22 t) is k_lu_apply_down's.
 __global__ void __launch_bounds__(ST) k_lu_apply_up(const int* __restrict__ flist,
                                                     const FrontDev* __restrict__ fr,
                                                     const double* __restrict__ F,
@@ -1628,27 +1554,6 @@ void launch_root_solve(int f, int N, const FrontDev* fr, const T* F, const int* 
 }
 
 template <class T>
-void launch_apply_up(const int* flist, int nf, const FrontDev* fr, const T* F, const int* dofs, T* X,
-                     int64_t ldx, int nrhs, T* W, const int64_t* woff, T* Tb, cudaStream_t st) {
-  if (nf <= 0) return;
-  k_apply_up<T><<<nf, ST, 0, st>>>(flist, fr, F, dofs, X, ldx, nrhs, W, woff, Tb);
-  g_launches++;
-}
-template <class T>
-void launch_apply_down(const int* flist, int nf, const FrontDev* fr, const T* F, const int* dofs,
-                       int64_t ldx, int nrhs, T* W, const int64_t* woff, const T* Tb,
-                       cudaStream_t st) {
-  if (nf <= 0) return;
-  k_apply_down<T><<<nf, ST, 0, st>>>(flist, fr, F, dofs, ldx, nrhs, W, woff, Tb);
-  g_launches++;
-}
-template <class T>
-void launch_root_apply(int f, const FrontDev* fr, const T* F, const int* dofs, T* X, int64_t ldx,
-                       int nrhs, T* W, const int64_t* woff, cudaStream_t st) {
-  k_root_apply<T><<<1, ST, 0, st>>>(f, fr, F, dofs, X, ldx, nrhs, W, woff);
-  g_launches++;
-}
-template <class T>
 void launch_sep_gather(const int* slist, int ns, const SepDev* sp, const int* dofs, T* X,
                        int64_t ldx, int nrhs, const T* W, const int64_t* woff, const FrontDev* fr,
                        cudaStream_t st) {
@@ -1700,6 +1605,14 @@ void launch_lu_apply_up(const int* flist, int nf, const FrontDev* fr, const doub
   g_launches++;
 }
 
+void launch_lu_apply_down(const int* flist, int nf, const FrontDev* fr, const double* F,
+                          const int* dofs, int64_t ldx, int nrhs, double* W, const int64_t* woff,
+                          const double* Tb, cudaStream_t st) {
+  if (nf <= 0) return;
+  k_lu_apply_down<<<nf, ST, 0, st>>>(flist, fr, F, dofs, ldx, nrhs, W, woff, Tb);
+  g_launches++;
+}
+
 template <class T>
 cudaError_t launch_trail_syrk(const int* flist, int nf, const FrontDev* fr, T* F, int Ks, int w,
                               cudaStream_t st) {
@@ -1733,12 +1646,6 @@ cudaError_t launch_trail_syrk(const int* flist, int nf, const FrontDev* fr, T* F
                                     T*, int64_t, int, T*, const int64_t*, cudaStream_t);            \
   template void launch_root_solve<T>(int, int, const FrontDev*, const T*, const int*, T*, int64_t, \
                                      int, T*, const int64_t*, cudaStream_t);                        \
-  template void launch_apply_up<T>(const int*, int, const FrontDev*, const T*, const int*, T*,     \
-                                   int64_t, int, T*, const int64_t*, T*, cudaStream_t);             \
-  template void launch_apply_down<T>(const int*, int, const FrontDev*, const T*, const int*,       \
-                                     int64_t, int, T*, const int64_t*, const T*, cudaStream_t);     \
-  template void launch_root_apply<T>(int, const FrontDev*, const T*, const int*, T*, int64_t, int, \
-                                     T*, const int64_t*, cudaStream_t);                             \
   template void launch_sep_gather<T>(const int*, int, const SepDev*, const int*, T*, int64_t, int, \
                                      const T*, const int64_t*, const FrontDev*, cudaStream_t);      \
   template cudaError_t launch_trail_syrk<T>(const int*, int, const FrontDev*, T*, int, int,       \

@@ -366,6 +366,8 @@ struct mfgpu_handle {
   int* d_modbuf = nullptr;
   size_t capMod = 0;
   int* d_all = nullptr;      // every front id then every separator id, level order
+  int* d_apply = nullptr;    // apply items: (front, first column) then (front, first row) pairs
+  int nApplyCols = 0, nApplyRows = 0;
   int64_t woffTotal = 0;     // sum over fronts of 2N
   Plan full, upd;
   std::vector<int> tuned;    // per level of the full plan: kernel picked by mfgpu_autotune, or -1
@@ -404,6 +406,7 @@ struct mfgpu_handle {
       cudaFree(d_chunkrow);
       cudaFree(d_segchunk);
       cudaFree(d_all);
+      cudaFree(d_apply);
       cudaFree(d_dinv_off);
       cudaFree(d_ipiv);
       cudaFree(d_flow);
@@ -1288,36 +1291,29 @@ struct mfgpu_handle {
   void applySweeps(T* X, int64_t ldx, int nrhs, T* W, T* Tb) {
     const Schedule& s = *S;
     const T* F = (const T*)d_F;
-    auto up = [&](int ell) {
-      if (lu) {
-        mfgpu::launch_lu_apply_up(d_all + s.lv[ell].front0, s.lv[ell].nbox, d_fr, (const double*)F,
-                                  d_ipiv, d_dofs, (double*)X, ldx, nrhs, (double*)W, d_woff,
-                                  (double*)Tb, stream);
-        ck(cudaGetLastError(), "launch LU apply up (k_lu_apply_up)");
-      } else {
-        mfgpu::launch_apply_up<T>(d_all + s.lv[ell].front0, s.lv[ell].nbox, d_fr, F, d_dofs, X, ldx,
-                                  nrhs, W, d_woff, Tb, stream);
-        ck(cudaGetLastError(), "launch apply up (k_apply_up)");
-      }
-    };
-    for (int ell = s.levels - 1; ell >= 1; ell--) up(ell);
-    if (lu) {
-      up(0);
-    } else if (s.lv[0].nbox > 1) {   // several roots (a batch)
-      mfgpu::launch_apply_up<T>(d_all, s.lv[0].nbox, d_fr, F, d_dofs, X, ldx, nrhs, W, d_woff, Tb,
-                                stream);
-      ck(cudaGetLastError(), "launch apply up (k_apply_up)");
-    } else {
-      mfgpu::launch_root_apply<T>(0, d_fr, F, d_dofs, X, ldx, nrhs, W, d_woff, stream);
-      ck(cudaGetLastError(), "launch root apply (k_root_apply)");
-    }
-    for (int ell = 1; ell < s.levels; ell++) {
-      mfgpu::launch_apply_down<T>(d_all + s.lv[ell].front0, s.lv[ell].nbox, d_fr, F, d_dofs, ldx,
-                                  nrhs, W, d_woff, Tb, stream);
-      ck(cudaGetLastError(), "launch apply down (k_apply_down)");
+    auto gather = [&](int ell) {
       mfgpu::launch_sep_gather<T>(d_all + s.fronts.size() + s.lv[ell].sep0, s.lv[ell].nsep, d_sp,
                                   d_dofs, X, ldx, nrhs, W, d_woff, d_fr, stream);
       ck(cudaGetLastError(), "launch separator gather (k_sep_gather)");
+    };
+    if (!lu) {
+      mfgpu::launch_apply<T>(d_apply, nApplyCols, d_apply + 2 * (size_t)nApplyCols, nApplyRows,
+                             d_fr, F, d_dofs, X, ldx, nrhs, W, d_woff, stream);
+      ck(cudaGetLastError(), "launch apply (k_apply_t, k_apply_l)");
+      for (int ell = 1; ell < s.levels; ell++) gather(ell);
+      return;
+    }
+    for (int ell = s.levels - 1; ell >= 0; ell--) {
+      mfgpu::launch_lu_apply_up(d_all + s.lv[ell].front0, s.lv[ell].nbox, d_fr, (const double*)F,
+                                d_ipiv, d_dofs, (double*)X, ldx, nrhs, (double*)W, d_woff,
+                                (double*)Tb, stream);
+      ck(cudaGetLastError(), "launch LU apply up (k_lu_apply_up)");
+    }
+    for (int ell = 1; ell < s.levels; ell++) {
+      mfgpu::launch_lu_apply_down(d_all + s.lv[ell].front0, s.lv[ell].nbox, d_fr, (const double*)F,
+                                  d_dofs, ldx, nrhs, (double*)W, d_woff, (const double*)Tb, stream);
+      ck(cudaGetLastError(), "launch LU apply down (k_lu_apply_down)");
+      gather(ell);
     }
   }
 
@@ -1785,6 +1781,20 @@ int createFrom(std::unique_ptr<Schedule> sched, int n, const int* row_ptr, const
     }
     H.d_gbar = dalloc<unsigned>(1, "alloc grid barrier");
     H.d_all = dalloc<int>(all.size(), "alloc id list");
+    if (!H.lu) {
+      std::vector<int> nn, NN, cols, rows;
+      for (const mfgpu::Front& f : s.fronts) {
+        nn.push_back(f.n);
+        NN.push_back(f.N);
+      }
+      mfgpu::apply_items(nn, NN, cols, rows);
+      H.nApplyCols = (int)cols.size() / 2;
+      H.nApplyRows = (int)rows.size() / 2;
+      cols.insert(cols.end(), rows.begin(), rows.end());
+      H.d_apply = dalloc<int>(cols.size(), "alloc apply items");
+      ck(cudaMemcpy(H.d_apply, cols.data(), cols.size() * sizeof(int), cudaMemcpyHostToDevice),
+         "upload apply items");
+    }
     if (H.lu) H.d_ipiv = dalloc<int>(s.dofs.size(), "alloc LU pivots");
     ck(cudaMemcpy(H.d_val, val, H.nnz * sizeof(double), cudaMemcpyHostToDevice), "upload val");
     ck(cudaMemcpy(H.d_rp, row_ptr, (n + 1) * sizeof(int), cudaMemcpyHostToDevice), "upload rows");
