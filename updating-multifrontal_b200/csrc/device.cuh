@@ -78,6 +78,26 @@ __device__ __forceinline__ void grid_barrier(unsigned* count, unsigned& target, 
   __syncthreads();
 }
 
+// One element global -> shared without a register round trip (cp.async, so
+// that a thread has dozens of loads in flight); zero-filled when !take.
+__device__ __forceinline__ void cp_elem(float* dst, const float* src, bool take) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(
+                   (unsigned)__cvta_generic_to_shared(dst)),
+               "l"(src), "r"(take ? 4 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void cp_elem(double* dst, const double* src, bool take) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(
+                   (unsigned)__cvta_generic_to_shared(dst)),
+               "l"(src), "r"(take ? 8 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_wait() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
+
 constexpr int kTaskTile = 32;   // assembly tile edge
 constexpr int kPanel = 32;      // panel width of the partial Cholesky
 

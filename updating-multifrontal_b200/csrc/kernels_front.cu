@@ -817,243 +817,10 @@ __global__ void __launch_bounds__(kCT) k_trail_syrk(const int* __restrict__ flis
 }
 
 // ---------------------------------------------------------------------------
-// Solve / apply sweeps.  One CTA per front; W is the front's workspace (N x nrhs,
-// ld N) inside a shared buffer.
+// Separator gather of the sweeps, and the apply of pivoted LU fronts.  W is a
+// front's workspace (N x nrhs, ld N) inside a shared buffer.
 // ---------------------------------------------------------------------------
 constexpr int ST = 256;
-
-// Forward solve with the front's first n columns, right-looking over 32-column
-// blocks.  On exit W[0,n) = L11^{-1} b_piv and W[n,N) = -L21 W[0,n).  W is the
-// front's right-hand-side block (N x nrhs, ld N) in shared or global memory.
-// UNIT: L11 has a unit diagonal (the L of a pivoted LU front) and its stored
-// diagonal, U's, is not read.
-template <class T, int NR, bool UNIT = false>
-__device__ void front_forward(const FrontDev& d, const T* __restrict__ A, T* W,
-                              int nrhs) {
-  __shared__ T Ls[kPanel][kPanel + 1];
-  __shared__ T xs[kPanel][NR + 1];
-  const int N = d.N, n = d.n, ld = d.ld, tid = threadIdx.x;
-  const int lane = tid & 31, warp = tid >> 5;
-  for (int k = 0; k < n; k += kPanel) {
-    const int kb = min(kPanel, n - k);
-    for (int idx = tid; idx < kb * kb; idx += blockDim.x) {
-      const int i = idx % kb, j = idx / kb;
-      if (i >= j) Ls[i][j] = A[(k + i) + (int64_t)(k + j) * ld];
-    }
-    for (int idx = tid; idx < kb * nrhs; idx += blockDim.x) {
-      const int i = idx % kb, c = idx / kb;
-      xs[i][c] = W[k + i + (int64_t)c * N];
-    }
-    __syncthreads();
-    if (warp == 0) {
-      // column-oriented substitution: lane i owns row i of the block
-      for (int j = 0; j < kb; j++) {
-        if (!UNIT && lane == j) {
-          const T djj = Ls[j][j];
-#pragma unroll
-          for (int c = 0; c < NR; c++)
-            if (c < nrhs) xs[j][c] = xs[j][c] / djj;
-        }
-        __syncwarp();
-        if (lane > j && lane < kb) {
-          const T l = Ls[lane][j];
-#pragma unroll
-          for (int c = 0; c < NR; c++)
-            if (c < nrhs) xs[lane][c] -= l * xs[j][c];
-        }
-        __syncwarp();
-      }
-    }
-    __syncthreads();
-    for (int idx = tid; idx < kb * nrhs; idx += blockDim.x) {
-      const int i = idx % kb, c = idx / kb;
-      W[k + i + (int64_t)c * N] = xs[i][c];
-    }
-    // rows below the block: W(r, :) -= L(r, k:k+kb) x   (thread per row, coalesced L)
-    for (int r = k + kb + tid; r < N; r += blockDim.x) {
-      T acc[NR];
-#pragma unroll
-      for (int c = 0; c < NR; c++) acc[c] = T(0);
-      const T* Lr = A + r + (int64_t)k * ld;
-      if (kb == kPanel) {
-        // all 32 loads issued before the FMAs: memory-level parallelism
-        T l[kPanel];
-#pragma unroll
-        for (int t = 0; t < kPanel; t++) l[t] = Lr[(int64_t)t * ld];
-#pragma unroll
-        for (int t = 0; t < kPanel; t++)
-#pragma unroll
-          for (int c = 0; c < NR; c++) acc[c] = fma(l[t], xs[t][c], acc[c]);
-      } else {
-        for (int t = 0; t < kb; t++) {
-          const T l = Lr[(int64_t)t * ld];
-#pragma unroll
-          for (int c = 0; c < NR; c++) acc[c] = fma(l, xs[t][c], acc[c]);
-        }
-      }
-#pragma unroll
-      for (int c = 0; c < NR; c++)
-        if (c < nrhs) W[r + (int64_t)c * N] -= acc[c];
-    }
-    __syncthreads();
-  }
-}
-
-// Backward solve: W[0,n) <- L11^{-T} (W[0,n) - L21^T W[n,N)).
-template <class T, int NR>
-__device__ void front_backward(const FrontDev& d, const T* __restrict__ A, T* W,
-                               int nrhs) {
-  __shared__ T Ls[kPanel][kPanel + 1];
-  __shared__ T xs[kPanel][NR + 1];
-  const int N = d.N, n = d.n, ld = d.ld, tid = threadIdx.x;
-  const int lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
-  const int nblk = (n + kPanel - 1) / kPanel;
-  for (int bk = nblk - 1; bk >= 0; bk--) {
-    const int k = bk * kPanel;
-    const int kb = min(kPanel, n - k);
-    for (int idx = tid; idx < kb * kb; idx += blockDim.x) {
-      const int i = idx % kb, j = idx / kb;
-      if (i >= j) Ls[i][j] = A[(k + i) + (int64_t)(k + j) * ld];
-    }
-    // xs(j, c) = W(k+j, c) - sum_{r >= k+kb} L(r, k+j) W(r, c): warp per column
-    for (int j = warp; j < kb; j += nw) {
-      T acc[NR];
-#pragma unroll
-      for (int c = 0; c < NR; c++) acc[c] = T(0);
-      const T* Lc = A + (int64_t)(k + j) * ld;
-      int r = k + kb + lane;
-      for (; r + 96 < N; r += 128) {      // four independent loads in flight
-        const T l0 = Lc[r], l1 = Lc[r + 32], l2 = Lc[r + 64], l3 = Lc[r + 96];
-#pragma unroll
-        for (int c = 0; c < NR; c++)
-          if (c < nrhs) {
-            const T* w = W + (int64_t)c * N + r;
-            acc[c] = fma(l0, w[0], acc[c]);
-            acc[c] = fma(l1, w[32], acc[c]);
-            acc[c] = fma(l2, w[64], acc[c]);
-            acc[c] = fma(l3, w[96], acc[c]);
-          }
-      }
-      for (; r < N; r += 32) {
-        const T l = Lc[r];
-#pragma unroll
-        for (int c = 0; c < NR; c++)
-          if (c < nrhs) acc[c] = fma(l, W[r + (int64_t)c * N], acc[c]);
-      }
-#pragma unroll
-      for (int c = 0; c < NR; c++) {
-        T v = acc[c];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        if (lane == 0 && c < nrhs) xs[j][c] = W[k + j + (int64_t)c * N] - v;
-      }
-    }
-    __syncthreads();
-    if (warp == 0) {
-      for (int j = kb - 1; j >= 0; j--) {
-        if (lane == j) {
-          const T djj = Ls[j][j];
-#pragma unroll
-          for (int c = 0; c < NR; c++)
-            if (c < nrhs) xs[j][c] = xs[j][c] / djj;
-        }
-        __syncwarp();
-        if (lane < j) {
-          const T l = Ls[j][lane];
-#pragma unroll
-          for (int c = 0; c < NR; c++)
-            if (c < nrhs) xs[lane][c] -= l * xs[j][c];
-        }
-        __syncwarp();
-      }
-    }
-    __syncthreads();
-    for (int idx = tid; idx < kb * nrhs; idx += blockDim.x) {
-      const int i = idx % kb, c = idx / kb;
-      W[k + i + (int64_t)c * N] = xs[i][c];
-    }
-    __syncthreads();
-  }
-}
-
-// Shared-memory staging of a front's right-hand-side block when it fits.
-constexpr int kSolveSmemBytes = 200 * 1024;
-
-
-template <class T, int NR>
-__global__ void __launch_bounds__(ST) k_solve_fwd(const int* __restrict__ flist,
-                                                  const FrontDev* __restrict__ fr,
-                                                  const T* __restrict__ F,
-                                                  const int* __restrict__ dofs, T* X,
-                                                  int64_t ldx, int nrhs, T* Wb,
-                                                  const int64_t* __restrict__ woff, int use_smem) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  T* smW = reinterpret_cast<T*>(smraw);
-  const int f = flist[blockIdx.x];
-  const FrontDev d = fr[f];
-  T* Wg = Wb + woff[f] * nrhs;
-  T* W = use_smem ? smW : Wg;
-  const int* dl = dofs + d.dof_off;
-  for (int idx = threadIdx.x; idx < d.N * nrhs; idx += blockDim.x) {
-    const int i = idx % d.N, c = idx / d.N;
-    W[idx] = i < d.n ? X[dl[i] + (int64_t)c * ldx] : T(0);
-  }
-  __syncthreads();
-  front_forward<T, NR>(d, F + d.off, W, nrhs);
-  for (int idx = threadIdx.x; idx < d.N * nrhs; idx += blockDim.x) {
-    const int i = idx % d.N, c = idx / d.N;
-    if (i < d.n) X[dl[i] + (int64_t)c * ldx] = W[idx];
-    else if (use_smem) Wg[idx] = W[idx];    // boundary part for the separator gather
-  }
-}
-
-template <class T, int NR>
-__global__ void __launch_bounds__(ST) k_solve_bwd(const int* __restrict__ flist,
-                                                  const FrontDev* __restrict__ fr,
-                                                  const T* __restrict__ F,
-                                                  const int* __restrict__ dofs, T* X,
-                                                  int64_t ldx, int nrhs, T* Wb,
-                                                  const int64_t* __restrict__ woff, int use_smem) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  T* smW = reinterpret_cast<T*>(smraw);
-  const int f = flist[blockIdx.x];
-  const FrontDev d = fr[f];
-  T* W = use_smem ? smW : Wb + woff[f] * nrhs;
-  const int* dl = dofs + d.dof_off;
-  for (int idx = threadIdx.x; idx < d.N * nrhs; idx += blockDim.x) {
-    const int i = idx % d.N, c = idx / d.N;
-    W[idx] = X[dl[i] + (int64_t)c * ldx];
-  }
-  __syncthreads();
-  front_backward<T, NR>(d, F + d.off, W, nrhs);
-  for (int idx = threadIdx.x; idx < d.n * nrhs; idx += blockDim.x) {
-    const int i = idx % d.n, c = idx / d.n;
-    X[dl[i] + (int64_t)c * ldx] = W[i + (int64_t)c * d.N];
-  }
-}
-
-template <class T, int NR>
-__global__ void __launch_bounds__(ST) k_root_solve(int f, const FrontDev* __restrict__ fr,
-                                                   const T* __restrict__ F,
-                                                   const int* __restrict__ dofs, T* X,
-                                                   int64_t ldx, int nrhs, T* Wb,
-                                                   const int64_t* __restrict__ woff, int use_smem) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  T* smW = reinterpret_cast<T*>(smraw);
-  const FrontDev d = fr[f];
-  T* W = use_smem ? smW : Wb + woff[f] * nrhs;
-  const int* dl = dofs + d.dof_off;
-  for (int idx = threadIdx.x; idx < d.N * nrhs; idx += blockDim.x) {
-    const int i = idx % d.N, c = idx / d.N;
-    W[idx] = X[dl[i] + (int64_t)c * ldx];
-  }
-  __syncthreads();
-  front_forward<T, NR>(d, F + d.off, W, nrhs);
-  front_backward<T, NR>(d, F + d.off, W, nrhs);
-  for (int idx = threadIdx.x; idx < d.n * nrhs; idx += blockDim.x) {
-    const int i = idx % d.n, c = idx / d.n;
-    X[dl[i] + (int64_t)c * ldx] = W[i + (int64_t)c * d.N];
-  }
-}
 
 // X(sep) = (X(sep) + W_box0(sep rows)) + W_box1(sep rows), the reference's
 // per-box accumulation order (mf2d.cpp:992-1011, 1036-1047).
@@ -1102,152 +869,6 @@ __global__ void __launch_bounds__(ST) k_lu_apply_down(const int* __restrict__ fl
     double s = double(0);
     for (int j = 0; j < d.n; j++) s += A[r + (int64_t)j * d.ld] * t[j];
     W[r + (int64_t)c * d.N] = s;
-  }
-}
-
-// ---------------------------------------------------------------------------
-// Sweeps of pivoted LU fronts (nonsymmetric problems, FP64; factors from
-// kernels_lu.cu: P A22 = L11 U11, L21 = A12 U11^{-1}, U12 = L11^{-1} P A21).
-// The reference's upward step b_sk -= XL b_rd, b_rd <- A22^{-1} b_rd and
-// downward step b_rd -= XR b_sk (src/DE/mf2d.cpp:976-1054) become
-//   forward:  y = L11^{-1} P b_piv (kept as the pivot part), W[n,N) = -L21 y
-//   backward: x_piv = U11^{-1} (y - U12 x_bd)
-// since XL = L21 L11^{-1} P and XR = U11^{-1} U12.
-// ---------------------------------------------------------------------------
-
-// Backward solve: W[0,n) <- U11^{-1} (W[0,n) - U12 W[n,N)), upward over
-// 32-row blocks; U(k block, right of it) is read a column at a time (lanes
-// along the block's rows), warps splitting the columns.
-template <int NR>
-__device__ void front_backward_lu(const FrontDev& d, const double* __restrict__ A, double* W,
-                                  int nrhs) {
-  __shared__ double Us[kPanel][kPanel + 1];
-  __shared__ double xs[kPanel][NR + 1];
-  __shared__ double part[ST / 32][kPanel];
-  const int N = d.N, n = d.n, ld = d.ld, tid = threadIdx.x;
-  const int lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
-  const int nblk = (n + kPanel - 1) / kPanel;
-  for (int bk = nblk - 1; bk >= 0; bk--) {
-    const int k = bk * kPanel, kb = min(kPanel, n - k);
-    for (int idx = tid; idx < kb * kb; idx += blockDim.x) {
-      const int i = idx % kb, j = idx / kb;
-      if (i <= j) Us[i][j] = A[(k + i) + (int64_t)(k + j) * ld];
-    }
-    double acc[NR];
-#pragma unroll
-    for (int c = 0; c < NR; c++) acc[c] = 0.0;
-    if (lane < kb)
-      for (int r = k + kb + warp; r < N; r += nw) {
-        const double u = A[(k + lane) + (int64_t)r * ld];
-#pragma unroll
-        for (int c = 0; c < NR; c++)
-          if (c < nrhs) acc[c] = fma(u, W[r + (int64_t)c * N], acc[c]);
-      }
-#pragma unroll
-    for (int c = 0; c < NR; c++) {
-      if (c < nrhs) {
-        part[warp][lane] = acc[c];
-        __syncthreads();
-        if (warp == 0 && lane < kb) {
-          double s = 0.0;
-          for (int w = 0; w < nw; w++) s += part[w][lane];
-          xs[lane][c] = W[k + lane + (int64_t)c * N] - s;
-        }
-        __syncthreads();
-      }
-    }
-    if (warp == 0) {
-      for (int j = kb - 1; j >= 0; j--) {
-        if (lane == j) {
-          const double ujj = Us[j][j];
-#pragma unroll
-          for (int c = 0; c < NR; c++)
-            if (c < nrhs) xs[j][c] = xs[j][c] / ujj;
-        }
-        __syncwarp();
-        if (lane < j) {
-          const double u = Us[lane][j];
-#pragma unroll
-          for (int c = 0; c < NR; c++)
-            if (c < nrhs) xs[lane][c] -= u * xs[j][c];
-        }
-        __syncwarp();
-      }
-    }
-    __syncthreads();
-    for (int idx = tid; idx < kb * nrhs; idx += blockDim.x) {
-      const int i = idx % kb, c = idx / kb;
-      W[k + i + (int64_t)c * N] = xs[i][c];
-    }
-    __syncthreads();
-  }
-}
-
-template <int NR>
-__global__ void __launch_bounds__(ST) k_lu_solve_fwd(const int* __restrict__ flist,
-                                                     const FrontDev* __restrict__ fr,
-                                                     const double* __restrict__ F,
-                                                     const int* __restrict__ ipiv,
-                                                     const int* __restrict__ dofs, double* X,
-                                                     int64_t ldx, int nrhs, double* Wb,
-                                                     const int64_t* __restrict__ woff,
-                                                     int use_smem) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  double* smW = reinterpret_cast<double*>(smraw);
-  const int f = flist[blockIdx.x];
-  const FrontDev d = fr[f];
-  double* Wg = Wb + woff[f] * nrhs;
-  double* W = use_smem ? smW : Wg;
-  const int* dl = dofs + d.dof_off;
-  const int* pv = ipiv + d.dof_off;
-  for (int idx = threadIdx.x; idx < d.N * nrhs; idx += blockDim.x) {
-    const int i = idx % d.N, c = idx / d.N;
-    W[idx] = i < d.n ? X[dl[i] + (int64_t)c * ldx] : 0.0;
-  }
-  __syncthreads();
-  if (threadIdx.x < nrhs) {   // b_piv <- P b_piv: the swaps in factorization order
-    double* w = W + (int64_t)threadIdx.x * d.N;
-    for (int j = 0; j < d.n; j++) {
-      const int p = pv[j];
-      if (p != j) {
-        const double t = w[j];
-        w[j] = w[p];
-        w[p] = t;
-      }
-    }
-  }
-  __syncthreads();
-  front_forward<double, NR, true>(d, F + d.off, W, nrhs);
-  for (int idx = threadIdx.x; idx < d.N * nrhs; idx += blockDim.x) {
-    const int i = idx % d.N, c = idx / d.N;
-    if (i < d.n) X[dl[i] + (int64_t)c * ldx] = W[idx];
-    else if (use_smem) Wg[idx] = W[idx];    // boundary part for the separator gather
-  }
-}
-
-template <int NR>
-__global__ void __launch_bounds__(ST) k_lu_solve_bwd(const int* __restrict__ flist,
-                                                     const FrontDev* __restrict__ fr,
-                                                     const double* __restrict__ F,
-                                                     const int* __restrict__ dofs, double* X,
-                                                     int64_t ldx, int nrhs, double* Wb,
-                                                     const int64_t* __restrict__ woff,
-                                                     int use_smem) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  double* smW = reinterpret_cast<double*>(smraw);
-  const int f = flist[blockIdx.x];
-  const FrontDev d = fr[f];
-  double* W = use_smem ? smW : Wb + woff[f] * nrhs;
-  const int* dl = dofs + d.dof_off;
-  for (int idx = threadIdx.x; idx < d.N * nrhs; idx += blockDim.x) {
-    const int i = idx % d.N, c = idx / d.N;
-    W[idx] = X[dl[i] + (int64_t)c * ldx];
-  }
-  __syncthreads();
-  front_backward_lu<NR>(d, F + d.off, W, nrhs);
-  for (int idx = threadIdx.x; idx < d.n * nrhs; idx += blockDim.x) {
-    const int i = idx % d.n, c = idx / d.n;
-    X[dl[i] + (int64_t)c * ldx] = W[i + (int64_t)c * d.N];
   }
 }
 
@@ -1459,141 +1080,12 @@ void launch_front_small(const int* flist, int nf, int maxN, const FrontDev* fr, 
   g_launches++;
 }
 
-// Solve kernels are templated on a bound of the right-hand-side count and keep
-// the front's right-hand-side block in dynamic shared memory when the largest
-// front's fits.
-namespace {
-void smemFor(int maxN, int nrhs, size_t elem, size_t& sm, int& use) {
-  const size_t need = (size_t)maxN * nrhs * elem;
-  use = need <= (size_t)kSolveSmemBytes;
-  sm = use ? need : 0;
-}
-}  // namespace
-
-// Threads per CTA of the per-front sweeps: enough warps for the level's
-// largest front (a thread per row below the diagonal block, a warp per column
-// of the block), at least two and at most ST.  Small fronts (the leaves of a
-// batch of thousands of them) then leave room for more CTAs per SM; every
-// value is computed by the same operations in the same order whatever the
-// block size, so results do not depend on it.
-inline int sweep_threads(int maxN) { return std::min(ST, std::max(64, (maxN + 31) & ~31)); }
-
-template <class T>
-void launch_solve_fwd(const int* flist, int nf, int maxN, const FrontDev* fr, const T* F,
-                      const int* dofs, T* X, int64_t ldx, int nrhs, T* W, const int64_t* woff,
-                      cudaStream_t st) {
-  if (nf <= 0) return;
-  size_t sm;
-  int use;
-  smemFor(maxN, nrhs, sizeof(T), sm, use);
-  const int threads = sweep_threads(maxN);
-#define MFGPU_FWD(NR)                                                                          \
-  do {                                                                                         \
-    static const bool attr_ = (cudaFuncSetAttribute(k_solve_fwd<T, NR>,                     \
-                                                    cudaFuncAttributeMaxDynamicSharedMemorySize,  \
-                                                    kSolveSmemBytes),                             \
-                               true);                                                             \
-    (void)attr_;                                                                                  \
-    k_solve_fwd<T, NR><<<nf, threads, sm, st>>>(flist, fr, F, dofs, X, ldx, nrhs, W, woff, use);\
-  } while (0)
-  if (nrhs == 1) MFGPU_FWD(1);
-  else if (nrhs <= 4) MFGPU_FWD(4);
-  else if (nrhs <= 8) MFGPU_FWD(8);
-  else MFGPU_FWD(16);
-#undef MFGPU_FWD
-  g_launches++;
-}
-
-template <class T>
-void launch_solve_bwd(const int* flist, int nf, int maxN, const FrontDev* fr, const T* F,
-                      const int* dofs, T* X, int64_t ldx, int nrhs, T* W, const int64_t* woff,
-                      cudaStream_t st) {
-  if (nf <= 0) return;
-  size_t sm;
-  int use;
-  smemFor(maxN, nrhs, sizeof(T), sm, use);
-  const int threads = sweep_threads(maxN);
-#define MFGPU_BWD(NR)                                                                          \
-  do {                                                                                         \
-    static const bool attr_ = (cudaFuncSetAttribute(k_solve_bwd<T, NR>,                     \
-                                                    cudaFuncAttributeMaxDynamicSharedMemorySize,  \
-                                                    kSolveSmemBytes),                             \
-                               true);                                                             \
-    (void)attr_;                                                                                  \
-    k_solve_bwd<T, NR><<<nf, threads, sm, st>>>(flist, fr, F, dofs, X, ldx, nrhs, W, woff, use);\
-  } while (0)
-  if (nrhs == 1) MFGPU_BWD(1);
-  else if (nrhs <= 4) MFGPU_BWD(4);
-  else if (nrhs <= 8) MFGPU_BWD(8);
-  else MFGPU_BWD(16);
-#undef MFGPU_BWD
-  g_launches++;
-}
-
-template <class T>
-void launch_root_solve(int f, int N, const FrontDev* fr, const T* F, const int* dofs, T* X,
-                       int64_t ldx, int nrhs, T* W, const int64_t* woff, cudaStream_t st) {
-  size_t sm;
-  int use;
-  smemFor(N, nrhs, sizeof(T), sm, use);
-#define MFGPU_ROOT(NR)                                                                          \
-  do {                                                                                          \
-    static const bool attr_ = (cudaFuncSetAttribute(k_root_solve<T, NR>,                     \
-                                                    cudaFuncAttributeMaxDynamicSharedMemorySize,  \
-                                                    kSolveSmemBytes),                             \
-                               true);                                                             \
-    (void)attr_;                                                                                  \
-    k_root_solve<T, NR><<<1, ST, sm, st>>>(f, fr, F, dofs, X, ldx, nrhs, W, woff, use);         \
-  } while (0)
-  if (nrhs == 1) MFGPU_ROOT(1);
-  else if (nrhs <= 4) MFGPU_ROOT(4);
-  else if (nrhs <= 8) MFGPU_ROOT(8);
-  else MFGPU_ROOT(16);
-#undef MFGPU_ROOT
-  g_launches++;
-}
-
 template <class T>
 void launch_sep_gather(const int* slist, int ns, const SepDev* sp, const int* dofs, T* X,
                        int64_t ldx, int nrhs, const T* W, const int64_t* woff, const FrontDev* fr,
                        cudaStream_t st) {
   if (ns <= 0) return;
   k_sep_gather<T><<<ns, ST, 0, st>>>(slist, sp, dofs, X, ldx, nrhs, W, woff, fr);
-  g_launches++;
-}
-
-void launch_lu_solve(bool forward, const int* flist, int nf, int maxN, const FrontDev* fr,
-                     const double* F, const int* ipiv, const int* dofs, double* X, int64_t ldx,
-                     int nrhs, double* W, const int64_t* woff, cudaStream_t st) {
-  if (nf <= 0) return;
-  size_t sm;
-  int use;
-  smemFor(maxN, nrhs, sizeof(double), sm, use);
-  const int threads = sweep_threads(maxN);
-#define MFGPU_LU(NR)                                                                             \
-  do {                                                                                           \
-    if (forward) {                                                                               \
-      static const bool attr_ = (cudaFuncSetAttribute(k_lu_solve_fwd<NR>,                        \
-                                                      cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                                      kSolveSmemBytes),                            \
-                                 true);                                                            \
-      (void)attr_;                                                                               \
-      k_lu_solve_fwd<NR><<<nf, threads, sm, st>>>(flist, fr, F, ipiv, dofs, X, ldx, nrhs, W, woff, \
-                                                  use);                                          \
-    } else {                                                                                     \
-      static const bool attr_ = (cudaFuncSetAttribute(k_lu_solve_bwd<NR>,                        \
-                                                      cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                                      kSolveSmemBytes),                            \
-                                 true);                                                            \
-      (void)attr_;                                                                               \
-      k_lu_solve_bwd<NR><<<nf, threads, sm, st>>>(flist, fr, F, dofs, X, ldx, nrhs, W, woff, use); \
-    }                                                                                            \
-  } while (0)
-  if (nrhs == 1) MFGPU_LU(1);
-  else if (nrhs <= 4) MFGPU_LU(4);
-  else if (nrhs <= 8) MFGPU_LU(8);
-  else MFGPU_LU(16);
-#undef MFGPU_LU
   g_launches++;
 }
 
@@ -1640,12 +1132,6 @@ cudaError_t launch_trail_syrk(const int* flist, int nf, const FrontDev* fr, T* F
                                             int, int, int);                                         \
   template void launch_front_small<T>(const int*, int, int, const FrontDev*, T*, DevError*,        \
                                       cudaStream_t);                                                \
-  template void launch_solve_fwd<T>(const int*, int, int, const FrontDev*, const T*, const int*,   \
-                                    T*, int64_t, int, T*, const int64_t*, cudaStream_t);            \
-  template void launch_solve_bwd<T>(const int*, int, int, const FrontDev*, const T*, const int*,   \
-                                    T*, int64_t, int, T*, const int64_t*, cudaStream_t);            \
-  template void launch_root_solve<T>(int, int, const FrontDev*, const T*, const int*, T*, int64_t, \
-                                     int, T*, const int64_t*, cudaStream_t);                        \
   template void launch_sep_gather<T>(const int*, int, const SepDev*, const int*, T*, int64_t, int, \
                                      const T*, const int64_t*, const FrontDev*, cudaStream_t);      \
   template cudaError_t launch_trail_syrk<T>(const int*, int, const FrontDev*, T*, int, int,       \

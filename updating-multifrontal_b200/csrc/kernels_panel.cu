@@ -90,26 +90,6 @@ __device__ __forceinline__ void st4(double* p, double a, double b, double c, dou
   *reinterpret_cast<double2*>(p + 2) = make_double2(c, d);
 }
 
-// One element global -> shared without a register round trip (cp.async, so
-// that a thread has dozens of loads in flight); zero-filled when !take.
-__device__ __forceinline__ void cp_elem(float* dst, const float* src, bool take) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(
-                   (unsigned)__cvta_generic_to_shared(dst)),
-               "l"(src), "r"(take ? 4 : 0)
-               : "memory");
-}
-__device__ __forceinline__ void cp_elem(double* dst, const double* src, bool take) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(
-                   (unsigned)__cvta_generic_to_shared(dst)),
-               "l"(src), "r"(take ? 8 : 0)
-               : "memory");
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
-
 // One warp factors the jb x jb (jb <= 32) diagonal block at (j0, j0) of Ds
 // (row-major, stride S) in place: lane i holds row i in registers.  Four
 // columns at a time: their pivots and their mutual updates by shuffles, then
