@@ -148,6 +148,19 @@ int coop_outer();   // default outer panel width of the cooperative kernel
 // phases of outer panel K in the prefix table built with this outer width
 int coop_phases(int K, int maxn, int outer = 0);
 
+// Partial factorization of every front in flist as a dataflow of 64 x 64 tiles
+// (kernels_tile.cu).  tile_tasks appends a level's tasks (two ints each) and
+// the nf + 1 offsets of the fronts' block rows; done: rowoff[nf] + 1 ints of
+// scratch, cleared before each launch.  The inverses of the diagonal blocks
+// go to Dv where dinv_off[front] >= 0.
+constexpr int kTileBlock = 64;
+void tile_tasks(const std::vector<int>& n, const std::vector<int>& N, std::vector<int>& tasks,
+                std::vector<int>& rowoff);
+template <class T>
+cudaError_t launch_front_tiles(const int* flist, const FrontDev* fr, T* F, const int* tasks,
+                               int ntasks, const int* rowoff, int nrows, int* done, T* Dv,
+                               const int64_t* dinv_off, DevError* err, cudaStream_t st);
+
 // Tensor-core (tcgen05, TF32) trailing update of the mixed path after outer
 // panel K of every front in flist: C(k1:N, k1:N) -= P P^T with P the panel's
 // columns, split = 1 (TF32) or 3 (hi/lo three-term TF32, about FP32 accuracy).

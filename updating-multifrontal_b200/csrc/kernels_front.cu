@@ -1127,9 +1127,6 @@ cudaError_t launch_trail_syrk(const int* flist, int nf, const FrontDev* fr, T* F
 #define MFGPU_INSTANTIATE(T)                                                                      \
   template void launch_tasks<T>(const Task*, const int64_t*, int, int64_t, T*, T*, const int*,     \
                                 const int*, const double*, const int*, const double*, cudaStream_t); \
-  template cudaError_t launch_level_coop<T>(const int*, int, int, const FrontDev*, T*, DevError*,  \
-                                            T*, const int*, unsigned*, cudaStream_t, int, int, int, \
-                                            int, int, int);                                         \
   template void launch_front_small<T>(const int*, int, int, const FrontDev*, T*, DevError*,        \
                                       cudaStream_t);                                                \
   template void launch_sep_gather<T>(const int*, int, const SepDev*, const int*, T*, int64_t, int, \
@@ -1140,5 +1137,8 @@ cudaError_t launch_trail_syrk(const int* flist, int nf, const FrontDev* fr, T* F
 MFGPU_INSTANTIATE(double)
 MFGPU_INSTANTIATE(float)
 #undef MFGPU_INSTANTIATE
+template cudaError_t launch_level_coop<float>(const int*, int, int, const FrontDev*, float*,
+                                              DevError*, float*, const int*, unsigned*, cudaStream_t,
+                                              int, int, int, int, int, int);
 
 }  // namespace mfgpu

@@ -4,6 +4,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <climits>
 #include <cmath>
 #include <cstddef>
 #include <cstdio>
@@ -90,10 +91,13 @@ struct Plan {
     int64_t cpref0 = 0;   // offset of the cooperative kernel's phase prefixes in cpref
     int coopItems = 0;    // largest work-item count of any cooperative phase
     int coopOuter = 0;    // outer panel width the phase prefixes were built with (0: default)
+    int64_t tt0 = 0, tr0 = 0;   // tile tasks in ttask, block-row offsets in trow
+    int ntt = 0, nrows = 0;     // tile tasks, block rows of all fronts
     // A batch plan (several problems' fronts in one plan, the serving loop's)
     // factors a level's fronts in consecutive partitions, each with the kernel
     // its problems would get alone: `subs` holds them (f0, nf, maxN, maxn,
-    // cpref0, coopItems, coopOuter of a partition, its kernel in `kind`).
+    // cpref0, coopItems, coopOuter, tile tasks of a partition, its kernel in
+    // `kind`).
     // Empty: one partition, the level itself, kernel by the size rules.
     struct Sub;
     std::vector<Sub> subs;
@@ -105,6 +109,8 @@ struct Plan {
   std::vector<int64_t> pref;
   std::vector<int> ids;
   std::vector<int> cpref;
+  std::vector<int> ttask, trow;   // tile tasks (pairs) and block-row offsets
+  int maxRows = 0;                // most block rows of any tile launch
   int nfronts = 0;
   double flops = 0;
   // device copies
@@ -112,18 +118,51 @@ struct Plan {
   int64_t* d_pref = nullptr;
   int* d_ids = nullptr;
   int* d_cpref = nullptr;
-  size_t cap_tasks = 0, cap_pref = 0, cap_ids = 0, cap_cpref = 0;
+  int* d_ttask = nullptr;
+  int* d_trow = nullptr;
+  size_t cap_tasks = 0, cap_pref = 0, cap_ids = 0, cap_cpref = 0, cap_ttask = 0, cap_trow = 0;
 
   void release() {
     cudaFree(d_tasks);
     cudaFree(d_pref);
     cudaFree(d_ids);
     cudaFree(d_cpref);
+    cudaFree(d_ttask);
+    cudaFree(d_trow);
     d_tasks = nullptr;
     d_pref = nullptr;
     d_ids = nullptr;
     d_cpref = nullptr;
-    cap_tasks = cap_pref = cap_ids = cap_cpref = 0;
+    d_ttask = nullptr;
+    d_trow = nullptr;
+    cap_tasks = cap_pref = cap_ids = cap_cpref = cap_ttask = cap_trow = 0;
+  }
+
+  void clear(int levels) {
+    lv.assign(levels, Level());
+    tasks.clear();
+    pref.clear();
+    ids.clear();
+    real.clear();
+    cpref.clear();
+    ttask.clear();
+    trow.clear();
+    maxRows = 0;
+    nfronts = 0;
+    flops = 0;
+    tcPackBytes = 0;
+  }
+
+  // The tile tasks of fronts of n pivots and N rows, into L (a level or a
+  // partition of one).
+  template <class L>
+  void addTiles(L& l, const std::vector<int>& n, const std::vector<int>& N) {
+    l.tt0 = (int64_t)ttask.size();
+    l.tr0 = (int64_t)trow.size();
+    mfgpu::tile_tasks(n, N, ttask, trow);
+    l.ntt = (int)((ttask.size() - l.tt0) / 2);
+    l.nrows = trow.back();
+    maxRows = std::max(maxRows, l.nrows);
   }
 
   // A group is built by beginGroup, appendGroup (the tasks of some owners,
@@ -184,6 +223,8 @@ struct Plan {
     grow(d_pref, cap_pref, pref.size(), "alloc plan prefixes");
     grow(d_ids, cap_ids, ids.size(), "alloc plan ids");
     grow(d_cpref, cap_cpref, cpref.size(), "alloc plan phase prefixes");
+    grow(d_ttask, cap_ttask, ttask.size(), "alloc plan tile tasks");
+    grow(d_trow, cap_trow, trow.size(), "alloc plan block rows");
     if (!tasks.empty())
       ck(cudaMemcpyAsync(d_tasks, tasks.data(), tasks.size() * sizeof(Task), cudaMemcpyHostToDevice, st),
          "upload tasks");
@@ -197,6 +238,13 @@ struct Plan {
       ck(cudaMemcpyAsync(d_cpref, cpref.data(), cpref.size() * sizeof(int), cudaMemcpyHostToDevice,
                          st),
          "upload phase prefixes");
+    if (!ttask.empty())
+      ck(cudaMemcpyAsync(d_ttask, ttask.data(), ttask.size() * sizeof(int), cudaMemcpyHostToDevice,
+                         st),
+         "upload tile tasks");
+    if (!trow.empty())
+      ck(cudaMemcpyAsync(d_trow, trow.data(), trow.size() * sizeof(int), cudaMemcpyHostToDevice, st),
+         "upload block rows");
     // host vectors must outlive the async copies
     ck(cudaStreamSynchronize(st), "plan upload");
   }
@@ -207,6 +255,8 @@ struct Plan::Level::Sub {
   int maxN = 0, maxn = 0;
   int64_t cpref0 = 0;
   int coopItems = 0, coopOuter = 0;
+  int64_t tt0 = 0, tr0 = 0;
+  int ntt = 0, nrows = 0;
   int kind = -1;
 };
 
@@ -309,6 +359,8 @@ struct mfgpu_handle {
   void* d_tcpack = nullptr;    // tensor-core panel images (mixed path)
   void* d_pslot = nullptr;     // factored diagonal blocks of the panel-by-panel kernels
   size_t tcPackCap = 0;
+  int* d_done = nullptr;       // finished block columns per block row + the tile kernel's task counter
+  size_t capDone = 0;
   unsigned* d_gbar = nullptr;  // grid-barrier arrival counter of the cooperative kernels
   // Cooperative (flag-ordered) sweeps: per level, its forward / backward task
   // lists and flag offsets in d_flow; the ready flags of one launch in d_flags.
@@ -340,6 +392,7 @@ struct mfgpu_handle {
   int tcSub = 128;                 // mixed: sub-panel width inside each 512-column outer panel of a
                                    // tensor-core level (0 or 512: no sub-panels)
   int fusedMinFronts = 148;        // fewest fronts for the one-CTA-per-front kernel
+  int fusedMaxN = 128;             // largest front for it
   bool subpanel = true;            // tensor-core levels: sub-panels by k_diag_factor + k_panel_trsm
                                    // (MFGPU_SUBPANEL=0: by the cooperative kernel)
   int panelMaxN = 0;               // largest front of a level factored panel by panel (0: never;
@@ -420,6 +473,7 @@ struct mfgpu_handle {
     cudaFree(d_tcpack);
     cudaFree(d_pslot);
     cudaFree(d_gbar);
+    cudaFree(d_done);
     cudaFree(d_Wd);
     cudaFree(d_X);
     cudaFree(d_Td);
@@ -448,15 +502,7 @@ struct mfgpu_handle {
   // to a dirty front at their level are recomputed.
   void buildPlan(Plan& P, const std::vector<char>& dirtyFront) {
     const Schedule& s = *S;
-    P.lv.assign(s.levels, Plan::Level());
-    P.tasks.clear();
-    P.pref.clear();
-    P.ids.clear();
-    P.real.clear();
-    P.cpref.clear();
-    P.nfronts = 0;
-    P.flops = 0;
-    P.tcPackBytes = 0;
+    P.clear(s.levels);
     for (int ell = s.levels - 1; ell >= 0; ell--) {
       Plan::Level& L = P.lv[ell];
       std::vector<int> fl, sl;
@@ -486,16 +532,19 @@ struct mfgpu_handle {
       L.sadd0 = P.addGroup(s.sep_add_tasks, s.sep_task_ptr, sl, 0);
       L.sadd1 = P.addGroup(s.sep_add_tasks, s.sep_task_ptr, sl, 1);
       L.cpref0 = (int64_t)P.cpref.size();
-      // phase tables for every level the cooperative kernel can take (also the
-      // ones the size rules give to k_front_small: the autotuner may not)
-      if (!fl.empty() && mfgpu::coop_fits((int)fl.size())) {
-        std::vector<int> nn, NN;
-        for (int f : fl) {
-          nn.push_back(s.fronts[f].n);
-          NN.push_back(s.fronts[f].N);
-        }
+      // tile tasks for every level of the full plan (the autotuner may time any
+      // kernel), for the levels whose kernel they are otherwise; phase tables
+      // for the tensor-core levels
+      if (fl.empty() || lu || !mfgpu::coop_fits((int)fl.size())) continue;
+      std::vector<int> nn, NN;
+      for (int f : fl) {
+        nn.push_back(s.fronts[f].n);
+        NN.push_back(s.fronts[f].N);
+      }
+      if (&P == &full || ruleKernel(L) == LK_COOP) P.addTiles(L, nn, NN);
+      const bool tc = mixed && tcLevel(L);
+      if (tc || (mixed && &P == &full && tcCandidate(L))) {
         const int W = mfgpu::tc_outer();
-        const bool tc = mixed && tcLevel(L);
         L.coopOuter = tc && tcSub > 0 && tcSub < W ? tcSub : 0;
         std::vector<int> pp = mfgpu::coop_phase_prefix(nn, NN, L.maxn, L.coopOuter);
         P.cpref.insert(P.cpref.end(), pp.begin(), pp.end());
@@ -534,15 +583,7 @@ struct mfgpu_handle {
   // factored exactly as in a plan of its problem alone.
   void buildPlanBatch(Plan& P, const std::vector<BatchMember>& M) {
     const Schedule& s = *S;
-    P.lv.assign(s.levels, Plan::Level());
-    P.tasks.clear();
-    P.pref.clear();
-    P.ids.clear();
-    P.real.clear();
-    P.cpref.clear();
-    P.nfronts = 0;
-    P.flops = 0;
-    P.tcPackBytes = 0;
+    P.clear(s.levels);
     const int W = mfgpu::tc_outer();
     for (int ell = s.levels - 1; ell >= 0; ell--) {
       Plan::Level& L = P.lv[ell];
@@ -587,23 +628,22 @@ struct mfgpu_handle {
           }
         }
         u.nf = (int64_t)P.ids.size() - u.f0;
-        if (kd == LK_COOP || kd == LK_TC) {
-          u.coopOuter = kd == LK_TC && tcSub > 0 && tcSub < W ? tcSub : 0;
+        if (kd == LK_COOP) P.addTiles(u, nn, NN);
+        if (kd == LK_TC) {
+          u.coopOuter = tcSub > 0 && tcSub < W ? tcSub : 0;
           u.cpref0 = (int64_t)P.cpref.size();
           std::vector<int> pp = mfgpu::coop_phase_prefix(nn, NN, u.maxn, u.coopOuter);
           P.cpref.insert(P.cpref.end(), pp.begin(), pp.end());
           const size_t stride = nn.size() + 1;
           for (size_t q = 0; q + stride <= pp.size(); q += stride)
             u.coopItems = std::max(u.coopItems, pp[q + nn.size()]);
-          if (kd == LK_TC) {
-            const int w = u.coopOuter > 0 ? u.coopOuter : W;
-            for (int K = 0; K < u.maxn; K += w)
-              for (int ww : {w, W})
-                if (K % ww == 0)
-                  P.tcPackBytes = std::max(
-                      P.tcPackBytes,
-                      mfgpu::tc_pack_bytes((int)nn.size(), mfgpu::tc_pack_cap(nn, NN, K, ww)));
-          }
+          const int w = u.coopOuter > 0 ? u.coopOuter : W;
+          for (int K = 0; K < u.maxn; K += w)
+            for (int ww : {w, W})
+              if (K % ww == 0)
+                P.tcPackBytes = std::max(
+                    P.tcPackBytes,
+                    mfgpu::tc_pack_bytes((int)nn.size(), mfgpu::tc_pack_cap(nn, NN, K, ww)));
         }
         L.maxN = std::max(L.maxN, u.maxN);
         L.maxn = std::max(L.maxn, u.maxn);
@@ -701,10 +741,13 @@ struct mfgpu_handle {
     if (mfgpu::coop_fits((int)L.nf) && !(stepped && !mixed)) {
       c.push_back(LK_COOP);
       if (L.nf <= mfgpu::kMaxPanelFronts) c.push_back(LK_PANEL);
-      if (mixed && L.nf <= mfgpu::tc_max_fronts() && L.maxN >= 1024) c.push_back(LK_TC);
+      if (mixed && tcCandidate(L)) c.push_back(LK_TC);
     }
     if (c.empty()) c.push_back(ruleKernel(L));
     return c;
+  }
+  bool tcCandidate(const Plan::Level& L) const {
+    return L.nf <= mfgpu::tc_max_fronts() && L.maxN >= 1024;
   }
 
   // Panel-pack bytes a tensor-core run of level L needs (outer panels only when
@@ -790,7 +833,21 @@ struct mfgpu_handle {
     tcPackCap = bytes;
   }
 
-  // Partial factorization of the fronts of level ell with kernel `kind`.
+  void ensureDone(const Plan& P) {
+    const size_t need = (size_t)P.maxRows + 1;
+    if (need <= capDone) return;
+    dropGraphs(true, false);   // the captured factorization uses the old words
+    ck(cudaStreamSynchronize(stream), "sync before growing the block-row words");
+    cudaFree(d_done);
+    d_done = nullptr;
+    capDone = 0;
+    d_done = dalloc<int>(need, "alloc block-row words");
+    capDone = need;
+  }
+
+  // Partial factorization of the fronts of level ell with kernel `kind`, and
+  // the block inverses of the cooperative sweeps (which the tile kernel leaves
+  // itself).
   template <class T>
   void runLevelKernel(const Plan& P, const Plan::Level& L, int ell, int kind) {
     const Schedule& s = *S;
@@ -810,10 +867,10 @@ struct mfgpu_handle {
     } else if (kind == LK_COOP) {
       prof.flops[MFGPU_KC_COOP] += fl;
       prof.begin(MFGPU_KC_COOP, stream);
-      ck(mfgpu::launch_level_coop<T>(P.d_ids + L.f0, (int)L.nf, L.maxn, d_fr, F, d_err,
-                                     (T*)d_slots, P.d_cpref + L.cpref0, d_gbar, stream, 0, -1, 0,
-                                     1, L.coopItems, L.coopOuter),
-         "launch cooperative level factorization (k_level_coop)");
+      ck(mfgpu::launch_front_tiles<T>(P.d_ids + L.f0, d_fr, F, P.d_ttask + L.tt0, L.ntt,
+                                      P.d_trow + L.tr0, L.nrows, d_done, (T*)d_Dinv, d_dinv_off,
+                                      d_err, stream),
+         "launch level factorization by tiles (k_front_tiles)");
       prof.end(stream);
     } else if (kind == LK_STEPPED) {
       if (sizeof(T) != sizeof(double))
@@ -825,6 +882,11 @@ struct mfgpu_handle {
     } else if (kind == LK_PANEL) {
       prof.flops[MFGPU_KC_COOP] += fl;
       runPanel<T>(P, L);
+    }
+    if (kind != LK_COOP && L.nf > 0 && coopSweep(ell)) {
+      mfgpu::launch_diag_inv<T>(P.d_ids + L.f0, (int)L.nf, L.maxn, d_fr, F, (T*)d_Dinv, d_dinv_off,
+                                stream);
+      ck(cudaGetLastError(), "launch diagonal-block inverses (k_diag_inv)");
     }
   }
 
@@ -885,6 +947,7 @@ struct mfgpu_handle {
       for (int ell = 0; ell < s.levels && ell < (int)tuned.size(); ell++)
         if (tuned[ell] == LK_TC) pack = std::max(pack, levelPackBytes(P, P.lv[ell]));
     ensurePack(pack);
+    ensureDone(P);
     // the full factorization's schedule as one graph, from its second run on
     if (&P == &full && graphs && !prof.on && fullRuns++ > 0) {
       if (!fullGraph) fullGraph = capture([&] { enqueuePlanT<T>(P); });
@@ -917,23 +980,21 @@ struct mfgpu_handle {
           Ls.cpref0 = u.cpref0;
           Ls.coopItems = u.coopItems;
           Ls.coopOuter = u.coopOuter;
+          Ls.tt0 = u.tt0;
+          Ls.ntt = u.ntt;
+          Ls.tr0 = u.tr0;
+          Ls.nrows = u.nrows;
           runLevelKernel<T>(P, Ls, ell, u.kind);
         }
       }
-      finishLevel<T>(P, L, ell);
+      finishLevel<T>(P, L);
     }
     ck(cudaGetLastError(), "factor launch");
   }
 
-  // After a level's partial factorization: the cooperative sweeps' block
-  // inverses, then the separator accumulation.
+  // After a level's partial factorization: the separator accumulation.
   template <class T>
-  void finishLevel(const Plan& P, const Plan::Level& L, int ell) {
-    if (L.nf > 0 && coopSweep(ell)) {
-      mfgpu::launch_diag_inv<T>(P.d_ids + L.f0, (int)L.nf, L.maxn, d_fr, (T*)d_F, (T*)d_Dinv,
-                                d_dinv_off, stream);
-      ck(cudaGetLastError(), "launch diagonal-block inverses (k_diag_inv)");
-    }
+  void finishLevel(const Plan& P, const Plan::Level& L) {
     runGroup<T>(P, L.sadd0, groupBytes(P, L.sadd0));
     runGroup<T>(P, L.sadd1, groupBytes(P, L.sadd1));
   }
@@ -953,6 +1014,7 @@ struct mfgpu_handle {
       for (int c : levelCandidates(P.lv[ell]))
         if (c == LK_TC) pack = std::max(pack, levelPackBytes(P, P.lv[ell]));
     ensurePack(pack);
+    ensureDone(P);
     if (mixed) {
       mfgpu::launch_diag_scale(d_rp, d_ci, d_val, n, d_scale, d_iscale, stream);
       ck(cudaGetLastError(), "launch diagonal scaling");
@@ -986,7 +1048,7 @@ struct mfgpu_handle {
       }
       runGroup<T>(P, L.ftask, groupBytes(P, L.ftask));
       runLevelKernel<T>(P, L, ell, levelKernel(P, L, ell));
-      finishLevel<T>(P, L, ell);
+      finishLevel<T>(P, L);
     }
     prof.on = prof_on;
     ck(cudaGetLastError(), "factor launch");
@@ -995,11 +1057,14 @@ struct mfgpu_handle {
   }
 
   // One CTA per front (k_front_small) when the level has enough fronts to fill
-  // the GPU and each front's staged panel fits in shared memory; otherwise the
-  // cooperative kernel spreads every front of the level over all SMs (a
-  // localized update often leaves one or two fronts per level).
+  // the GPU and they are at most two tiles wide, where a tile's hand-offs cost
+  // more than they spread (256 fronts of 77 x 49: 52 us against 64); the tile
+  // kernel (k_front_tiles) otherwise, which also spreads the few large fronts
+  // of an uneven level (FP64, one CTA per front against tiles: 256 fronts of
+  // 377 x 125 526 against 380 us, 4096 of 285 x 225 5.09 against 4.47 ms).
   bool useFused(int nf, int maxN) const {
-    return mfgpu::small_front_fits(maxN, (int)esz) && (nf >= fusedMinFronts || maxN <= 64);
+    return mfgpu::small_front_fits(maxN, (int)esz) &&
+           ((nf >= fusedMinFronts && maxN <= fusedMaxN) || maxN <= 64);
   }
 
   // Mixed path: levels of large fronts run the cooperative kernel one outer
@@ -1154,7 +1219,7 @@ struct mfgpu_handle {
     ck(cudaStreamSynchronize(stream), "factor");
     if (e.code == 2 || e.code == 3) {
       throw CudaError(e.code == 2 ? "a tensor-core pipeline wait gave up (k_trail_tc)"
-                                  : "a cooperative kernel's grid barrier gave up",
+                                  : "a cooperative kernel's grid barrier or ready word gave up",
                       MFGPU_ERR_TIMEOUT);
     }
     if (e.code == 4) {
@@ -1651,7 +1716,10 @@ int createFrom(std::unique_ptr<Schedule> sched, int n, const int* row_ptr, const
   if (const char* e = getenv("MFGPU_VERBOSE")) h->prof.verbose = e[0] == '1';
   if (const char* e = getenv("MFGPU_TC_MIN_N")) h->tcMinN = atoi(e);
   if (const char* e = getenv("MFGPU_SOLVE_COOP_MIN_N")) h->solveCoopMinN = atoi(e);
-  if (const char* e = getenv("MFGPU_FUSED_MIN_FRONTS")) h->fusedMinFronts = atoi(e);
+  if (const char* e = getenv("MFGPU_FUSED_MIN_FRONTS")) {   // that many, of any size that fits
+    h->fusedMinFronts = atoi(e);
+    h->fusedMaxN = INT_MAX;
+  }
   auto splitOf = [](const char* e, int dflt) {
     const std::string v(e);
     return v == "1" || v == "tf32" ? 1 : v == "bf16" ? 2 : v == "3" ? 3 : dflt;
@@ -1809,6 +1877,7 @@ int createFrom(std::unique_ptr<Schedule> sched, int n, const int* row_ptr, const
     std::vector<char> dirty(s.fronts.size(), 1);
     H.buildPlan(H.full, dirty);
     H.full.upload(H.stream);
+    H.ensureDone(H.full);
     H.device_bytes = (int64_t)(s.front_elems + s.sep_elems) * (int64_t)H.esz + H.nnz * 8 +
                      (H.nnz + n + 1) * 4 + (int64_t)s.dofs.size() * 4;
   });
@@ -2897,6 +2966,7 @@ std::unique_ptr<mfgpu_handle> makeView(mfgpu_handle& B) {
   H.panelMaxN = B.panelMaxN;
   H.tcSub = B.tcSub;
   H.fusedMinFronts = B.fusedMinFronts;
+  H.fusedMaxN = B.fusedMaxN;
   H.d_scale = B.d_scale;
   H.d_iscale = B.d_iscale;
   H.nseg = B.nseg;
