@@ -30,8 +30,36 @@ std::atomic<long long> g_launches{0};
 
 namespace {
 
-// One warp per 32 x 32 tile of a task, kTaskWarps tiles per CTA.
+// Assembly, one warp per 32 x 32 tile of a task, kTaskWarps tiles per CTA.
+// Bound: HBM writes (every element of the fronts) for the leaf levels, the
+// chain of dependent loads (tile -> task -> DOFs -> CSR rows) for small levels.
+// So the tile's task is found by all lanes probing at once (three or four
+// rounds of loads for 100,000 tasks, not seventeen), the rows of a tile are
+// spread over the lanes, and block moves keep kTaskUnroll columns in flight.
+// Sparse tiles: a lane holds its row's CSR entries (eight at a time) in
+// registers and matches them against the tile's columns, broadcast one by one,
+// so each column is written as it is found.  Against a serial search and a
+// pass over all rows with every lane reading the same entries: 2D 1023^2
+// leaves 2.20 -> 1.29 ms; with the fronts, separator bases and both
+// accumulations of a level in two launches instead of four, the assemblies of
+// a 2D 127^2 factorization and update 549 -> 189 us.
 constexpr int kTaskWarps = 4;
+constexpr int kTaskUnroll = 8;
+
+// Last t in [0, n) with start[t] <= x (start[0] <= x), by a whole warp.
+__device__ __forceinline__ int warp_upper(const int64_t* __restrict__ start, int n, int64_t x,
+                                          int lane) {
+  int lo = 0, len = n;   // the answer is in [lo, lo + len)
+  while (len > 1) {
+    const int step = (len + 31) / 32;
+    const int at = lo + lane * step;
+    const bool le = lane * step < len && start[at] <= x;
+    const int k = __popc(__ballot_sync(0xffffffffu, le)) - 1;   // probes up to lane k hold
+    lo += k * step;
+    len = min(step, len - k * step);
+  }
+  return lo;
+}
 
 template <class T>
 __global__ void __launch_bounds__(32 * kTaskWarps) k_tasks(const Task* __restrict__ tasks,
@@ -47,79 +75,116 @@ __global__ void __launch_bounds__(32 * kTaskWarps) k_tasks(const Task* __restric
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t tile = ((int64_t)blockIdx.x + (int64_t)blockIdx.y * gridDim.x) * kTaskWarps + w;
   if (tile >= ntiles) return;
-  int t = 0;
-  if (lane == 0) {
-    int lo = 0, hi = ntasks - 1;   // last t with tstart[t] <= tile
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (tstart[mid] <= tile) lo = mid;
-      else hi = mid - 1;
-    }
-    t = lo;
-  }
-  t = __shfl_sync(0xffffffffu, t, 0);
+  const int t = warp_upper(tstart, ntasks, tile, lane);
   const Task Tk = tasks[t];
-  const int64_t local = tile - tstart[t];
+  const int local = (int)(tile - tstart[t]);
   const int tr = (Tk.rows + kTaskTile - 1) / kTaskTile;
-  const int i0 = (int)(local % tr) * kTaskTile;
-  const int j0 = (int)(local / tr) * kTaskTile;
+  const int i0 = (local % tr) * kTaskTile;
+  const int j0 = (local / tr) * kTaskTile;
   if (Tk.lower && i0 + kTaskTile - 1 < j0) return;
   T* dst = (Tk.dst_arena == AR_FRONT ? F : SA) + Tk.dst_off;
   const T* src = (Tk.src_arena == AR_FRONT ? F : SA) + Tk.src_off;
   const int rows = min(kTaskTile, Tk.rows - i0), cols = min(kTaskTile, Tk.cols - j0);
   T(*tb)[kTaskTile + 1] = sm[w];
   const int i = i0 + lane;   // this lane's row of the tile in the column-major writes
+  // first column this lane does not write (its row's diagonal in lower tiles)
+  const int jend = lane >= rows ? 0 : Tk.lower ? min(cols, i - j0 + 1) : cols;
+  T* d = dst + i + (int64_t)j0 * Tk.dst_ld;
   if (Tk.kind == TK_COPY && Tk.trans) {
     // dst(i, j) = src[j + i*ld]: read src rows with lanes along j, write dst
     // columns with lanes along i, through the warp's shared-memory tile
-    for (int ii = 0; ii < rows; ii++)
-      if (lane < cols) tb[ii][lane] = src[(j0 + lane) + (int64_t)(i0 + ii) * Tk.src_ld];
+    const T* sr = src + j0 + lane + (int64_t)i0 * Tk.src_ld;
+    for (int ii = 0; ii < rows; ii += kTaskUnroll) {
+      T v[kTaskUnroll];
+#pragma unroll
+      for (int q = 0; q < kTaskUnroll; q++)
+        v[q] = lane < cols && ii + q < rows ? sr[(int64_t)(ii + q) * Tk.src_ld] : T(0);
+#pragma unroll
+      for (int q = 0; q < kTaskUnroll; q++) tb[ii + q][lane] = v[q];
+    }
     __syncwarp();
-    if (lane < rows)
-      for (int jj = 0; jj < cols; jj++)
-        if (!Tk.lower || i >= j0 + jj) dst[i + (int64_t)(j0 + jj) * Tk.dst_ld] = tb[lane][jj];
+#pragma unroll 4
+    for (int jj = 0; jj < jend; jj++) d[(int64_t)jj * Tk.dst_ld] = tb[lane][jj];
     return;
   }
   if (Tk.kind == TK_SPARSE) {
-    // values of this task's matrix: src_off is the element offset of its CSR
-    // values (0 but for the serving loop's batches of several matrices)
+    // A(r, c) for the tile (Sparse::operator(), src/LinAlg/sparse.cpp:80-92).
+    // Values of this task's matrix: src_off is the element offset of its CSR
+    // values (0 but for the serving loop's batches of several matrices).
     va += Tk.src_off;
-    // A(r, c) for the tile (Sparse::operator(), src/LinAlg/sparse.cpp:80-92):
-    // lane j holds column DOF c_j; every row's CSR entries are read once (all
-    // lanes load the same addresses) and matched against the lanes' columns
     const int cj = lane < cols ? dofs[Tk.col_dof + j0 + lane] : -1;
+    const int rl = lane < rows ? dofs[Tk.row_dof + i] : 0;
     const double sc = (scale && lane < cols) ? scale[cj] : 1.0;
-    // row DOFs, row extents and row scales of the tile, one per lane
-    const int rl = lane < rows ? dofs[Tk.row_dof + i0 + lane] : 0;
-    const int pl0 = lane < rows ? rp[rl] : 0, pl1 = lane < rows ? rp[rl + 1] : 0;
-    const double srl = (scale && lane < rows) ? scale[rl] : 1.0;
-#pragma unroll 4
-    for (int ii = 0; ii < rows; ii++) {
-      const int p0 = __shfl_sync(0xffffffffu, pl0, ii), p1 = __shfl_sync(0xffffffffu, pl1, ii);
-      const double sr = __shfl_sync(0xffffffffu, srl, ii);
-      double v = 0.0;
+    const double sr = (scale && lane < rows) ? scale[rl] : 1.0;
+    const int p0 = lane < rows ? rp[rl] : 0, p1 = lane < rows ? rp[rl + 1] : 0;
+    const bool lng = __any_sync(0xffffffffu, p1 - p0 > 8);   // rows of wider stencils
+    if (lng)
+      for (int jj = 0; jj < cols; jj++) tb[lane][jj] = T(0);
+    for (int pb = p0;; pb += 8) {
+      int c[8];
+      double v[8];
 #pragma unroll
-      for (int q = 0; q < 8; q++)   // stencil rows are short: independent loads
-        if (p0 + q < p1 && ci[p0 + q] == cj) v = va[p0 + q];
-      for (int p = p0 + 8; p < p1; p++)
-        if (ci[p] == cj) v = va[p];
-      if (scale) v = v * sr * sc;   // symmetric diagonal scaling
-      tb[ii][lane] = (T)v;
+      for (int q = 0; q < 8; q++) c[q] = pb + q < p1 ? ci[pb + q] : -2;
+#pragma unroll
+      for (int q = 0; q < 8; q++) v[q] = pb + q < p1 ? va[pb + q] : 0.0;
+      for (int jj = 0; jj < cols; jj++) {
+        const int cc = __shfl_sync(0xffffffffu, cj, jj);
+        const double scj = __shfl_sync(0xffffffffu, sc, jj);
+        double x = 0.0;
+        bool hit = false;
+#pragma unroll
+        for (int q = 0; q < 8; q++)
+          if (c[q] == cc) {
+            x = v[q];
+            hit = true;
+          }
+        if (scale) x = x * sr * scj;   // symmetric diagonal scaling
+        if (lng) {
+          if (hit) tb[lane][jj] = (T)x;
+        } else if (jj < jend) {
+          d[(int64_t)jj * Tk.dst_ld] = (T)x;
+        }
+      }
+      if (!__any_sync(0xffffffffu, pb + 8 < p1)) break;
     }
-    __syncwarp();
-    if (lane < rows)
-      for (int jj = 0; jj < cols; jj++)
-        if (!Tk.lower || i >= j0 + jj) dst[i + (int64_t)(j0 + jj) * Tk.dst_ld] = tb[lane][jj];
+    if (lng)
+      for (int jj = 0; jj < jend; jj++) d[(int64_t)jj * Tk.dst_ld] = tb[lane][jj];
     return;
   }
-  if (lane >= rows) return;
-  for (int jj = 0; jj < cols; jj++) {
-    const int j = j0 + jj;
-    if (Tk.lower && i < j) continue;
-    T* d = dst + i + (int64_t)j * Tk.dst_ld;
-    if (Tk.kind == TK_ZERO) *d = T(0);
-    else if (Tk.kind == TK_COPY) *d = src[i + (int64_t)j * Tk.src_ld];
-    else *d = *d + src[i + (int64_t)j * Tk.src_ld];   // TK_ADD
+  if (Tk.kind == TK_ZERO) {
+#pragma unroll 8
+    for (int jj = 0; jj < jend; jj++) d[(int64_t)jj * Tk.dst_ld] = T(0);
+    return;
+  }
+  const T* s0 = src + i + (int64_t)j0 * Tk.src_ld;
+  if (Tk.kind == TK_COPY) {
+    for (int jj = 0; jj < jend; jj += kTaskUnroll) {
+      T v[kTaskUnroll];
+#pragma unroll
+      for (int q = 0; q < kTaskUnroll; q++)
+        if (jj + q < jend) v[q] = s0[(int64_t)(jj + q) * Tk.src_ld];
+#pragma unroll
+      for (int q = 0; q < kTaskUnroll; q++)
+        if (jj + q < jend) d[(int64_t)(jj + q) * Tk.dst_ld] = v[q];
+    }
+    return;
+  }
+  // TK_ADD, listed in pairs (the second has no tiles of its own):
+  // dst = (dst + box 0's block) + box 1's block, the reference's order
+  const Task T1 = tasks[t + 1];
+  const T* s1 = (T1.src_arena == AR_FRONT ? F : SA) + T1.src_off + i + (int64_t)j0 * T1.src_ld;
+  for (int jj = 0; jj < jend; jj += kTaskUnroll) {
+    T v[kTaskUnroll], a[kTaskUnroll], c[kTaskUnroll];
+#pragma unroll
+    for (int q = 0; q < kTaskUnroll; q++)
+      if (jj + q < jend) {
+        v[q] = d[(int64_t)(jj + q) * Tk.dst_ld];
+        a[q] = s0[(int64_t)(jj + q) * Tk.src_ld];
+        c[q] = s1[(int64_t)(jj + q) * T1.src_ld];
+      }
+#pragma unroll
+    for (int q = 0; q < kTaskUnroll; q++)
+      if (jj + q < jend) d[(int64_t)(jj + q) * Tk.dst_ld] = (v[q] + a[q]) + c[q];
   }
 }
 

@@ -87,7 +87,7 @@ struct Plan {
   struct Level {
     int64_t f0 = 0, nf = 0, s0 = 0, ns = 0;  // offsets into the id list
     int maxN = 0, maxn = 0;
-    Group ftask, sbase, sadd0, sadd1;
+    Group assemble, sadd;   // fronts and separators' base; separators' accumulation
     int64_t cpref0 = 0;   // offset of the cooperative kernel's phase prefixes in cpref
     int coopItems = 0;    // largest work-item count of any cooperative phase
     int coopOuter = 0;    // outer panel width the phase prefixes were built with (0: default)
@@ -166,7 +166,8 @@ struct Plan {
   }
 
   // A group is built by beginGroup, appendGroup (the tasks of some owners,
-  // optionally rewritten by fx), endGroup.
+  // optionally rewritten by fx), endGroup.  pairs: the owners' tasks come in
+  // pairs that one tile executes together, so the second one has no tiles.
   Group beginGroup() {
     Group g;
     g.task0 = (int64_t)tasks.size();
@@ -174,39 +175,24 @@ struct Plan {
     pref.push_back(0);
     return g;
   }
-  void appendGroup(Group& g, const std::vector<Task>& src, const std::vector<int64_t>& ptr,
-                   const std::vector<int>& owners, int pick /* -1 all, 0/1 add task k */,
+  void appendGroup(const std::vector<Task>& src, const std::vector<int64_t>& ptr,
+                   const std::vector<int>& owners, bool pairs,
                    const std::function<void(Task&)>& fx = nullptr) {
     int64_t acc = pref.back();
     for (int o : owners) {
-      int64_t a, b;
-      if (pick < 0) {
-        a = ptr[o];
-        b = ptr[o + 1];
-      } else {
-        a = 2 * (int64_t)o + pick;
-        b = a + 1;
-      }
+      const int64_t a = pairs ? 2 * (int64_t)o : ptr[o], b = pairs ? a + 2 : ptr[o + 1];
       for (int64_t t = a; t < b; t++) {
         tasks.push_back(src[t]);
         if (fx) fx(tasks.back());
-        acc += tilesOf(src[t]);
+        if (!pairs || t == a) acc += tilesOf(src[t]);
         pref.push_back(acc);
       }
     }
-    (void)g;
   }
   void endGroup(Group& g) {
     g.ntasks = (int64_t)tasks.size() - g.task0;
     g.ntiles = pref.back();
     if (g.ntasks == 0) pref.pop_back();
-  }
-  Group addGroup(const std::vector<Task>& src, const std::vector<int64_t>& ptr,
-                 const std::vector<int>& owners, int pick) {
-    Group g = beginGroup();
-    appendGroup(g, src, ptr, owners, pick);
-    endGroup(g);
-    return g;
   }
 
   void upload(cudaStream_t st) {
@@ -527,10 +513,13 @@ struct mfgpu_handle {
         P.flops += s.front_flops(s.fronts[f]);
       }
       P.nfronts += (int)fl.size();
-      L.ftask = P.addGroup(s.front_tasks, s.front_task_ptr, fl, -1);
-      L.sbase = P.addGroup(s.sep_tasks, s.sep_task_ptr, sl, -1);
-      L.sadd0 = P.addGroup(s.sep_add_tasks, s.sep_task_ptr, sl, 0);
-      L.sadd1 = P.addGroup(s.sep_add_tasks, s.sep_task_ptr, sl, 1);
+      L.assemble = P.beginGroup();
+      P.appendGroup(s.front_tasks, s.front_task_ptr, fl, false);
+      P.appendGroup(s.sep_tasks, s.sep_task_ptr, sl, false);
+      P.endGroup(L.assemble);
+      L.sadd = P.beginGroup();
+      P.appendGroup(s.sep_add_tasks, s.sep_task_ptr, sl, true);
+      P.endGroup(L.sadd);
       L.cpref0 = (int64_t)P.cpref.size();
       // tile tasks for every level of the full plan (the autotuner may time any
       // kernel), for the levels whose kernel they are otherwise; phase tables
@@ -658,23 +647,23 @@ struct mfgpu_handle {
           P.real.push_back(k);
         }
       L.ns = (int64_t)P.ids.size() - L.s0;
-      auto group = [&](const std::vector<Task>& src, const std::vector<int64_t>& ptr,
-                       const std::vector<std::vector<int>>& own, int pick) {
-        Group g = P.beginGroup();
+      auto append = [&](const std::vector<Task>& src, const std::vector<int64_t>& ptr,
+                        const std::vector<std::vector<int>>& own, bool pairs) {
         for (size_t m = 0; m < nm; m++) {
           const BatchMember& bm = M[m];
-          P.appendGroup(g, src, ptr, own[m], pick, [&bm](Task& t) {
+          P.appendGroup(src, ptr, own[m], pairs, [&bm](Task& t) {
             bm.move(t);
             if (t.kind == mfgpu::TK_SPARSE) t.src_off = bm.valoff;
           });
         }
-        P.endGroup(g);
-        return g;
       };
-      L.ftask = group(s.front_tasks, s.front_task_ptr, fl, -1);
-      L.sbase = group(s.sep_tasks, s.sep_task_ptr, sl, -1);
-      L.sadd0 = group(s.sep_add_tasks, s.sep_task_ptr, sl, 0);
-      L.sadd1 = group(s.sep_add_tasks, s.sep_task_ptr, sl, 1);
+      L.assemble = P.beginGroup();
+      append(s.front_tasks, s.front_task_ptr, fl, false);
+      append(s.sep_tasks, s.sep_task_ptr, sl, false);
+      P.endGroup(L.assemble);
+      L.sadd = P.beginGroup();
+      append(s.sep_add_tasks, s.sep_task_ptr, sl, true);
+      P.endGroup(L.sadd);
     }
   }
 
@@ -966,8 +955,7 @@ struct mfgpu_handle {
     for (int ell = s.levels - 1; ell >= 0; ell--) {
       const Plan::Level& L = P.lv[ell];
       prof.level = ell;
-      runGroup<T>(P, L.sbase, groupBytes(P, L.sbase));
-      runGroup<T>(P, L.ftask, groupBytes(P, L.ftask));
+      runGroup<T>(P, L.assemble, groupBytes(P, L.assemble));
       if (L.subs.empty()) {
         runLevelKernel<T>(P, L, ell, levelKernel(P, L, ell));
       } else {
@@ -995,8 +983,7 @@ struct mfgpu_handle {
   // After a level's partial factorization: the separator accumulation.
   template <class T>
   void finishLevel(const Plan& P, const Plan::Level& L) {
-    runGroup<T>(P, L.sadd0, groupBytes(P, L.sadd0));
-    runGroup<T>(P, L.sadd1, groupBytes(P, L.sadd1));
+    runGroup<T>(P, L.sadd, groupBytes(P, L.sadd));
   }
 
   // Full factorization that also picks each level's kernel by timing: per
@@ -1024,14 +1011,13 @@ struct mfgpu_handle {
     prof.on = false;
     for (int ell = s.levels - 1; ell >= 0; ell--) {
       const Plan::Level& L = P.lv[ell];
-      runGroup<T>(P, L.sbase, groupBytes(P, L.sbase));
       const std::vector<int> cand = levelCandidates(L);
       if (cand.size() > 1) {
         float best = 0;
         for (int c : cand) {
           float t = 0;
           for (int r = 0; r < std::max(1, reps); r++) {
-            runGroup<T>(P, L.ftask, groupBytes(P, L.ftask));
+            runGroup<T>(P, L.assemble, groupBytes(P, L.assemble));
             ck(cudaEventRecord(ev0, stream), "event");
             runLevelKernel<T>(P, L, ell, c);
             ck(cudaEventRecord(ev1, stream), "event");
@@ -1046,7 +1032,7 @@ struct mfgpu_handle {
           }
         }
       }
-      runGroup<T>(P, L.ftask, groupBytes(P, L.ftask));
+      runGroup<T>(P, L.assemble, groupBytes(P, L.assemble));
       runLevelKernel<T>(P, L, ell, levelKernel(P, L, ell));
       finishLevel<T>(P, L);
     }
