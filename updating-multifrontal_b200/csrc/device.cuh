@@ -13,8 +13,10 @@ struct FrontDev {
   int64_t off;      // element offset of the front (column-major, ld) in the arena
   int64_t dof_off;  // offset of [pivots..., boundary...] in the DOF table
   int n, m, N, ld;
+  int64_t rs_off;   // offset of the row scales of the front's matrix (0 but for the
+                    // serving loop's batches of several matrices)
 };
-static_assert(sizeof(FrontDev) == 32, "FrontDev layout");
+static_assert(sizeof(FrontDev) == 40, "FrontDev layout");
 
 // Per-separator descriptor for the solve/apply gathers.
 struct SepDev {
@@ -161,12 +163,14 @@ cudaError_t launch_front_tiles(const int* flist, const FrontDev* fr, T* F, const
                                int ntasks, const int* rowoff, int nrows, int* done, T* Dv,
                                const int64_t* dinv_off, DevError* err, cudaStream_t st);
 
-// Tensor-core (tcgen05, TF32) trailing update of the mixed path after outer
-// panel K of every front in flist: C(k1:N, k1:N) -= P P^T with P the panel's
-// columns, split = 1 (TF32) or 3 (hi/lo three-term TF32, about FP32 accuracy).
-// launch_tc_pack first writes P, split into TF32 hi / lo tensor-core images,
-// into `pack` (tc_pack_bytes(nf, cap) bytes, cap = tc_pack_cap(n, N, K, w));
-// launch_trail_tc then reads P only from there.
+// Tensor-core (tcgen05) trailing update of the mixed path after outer panel K
+// of every front in flist: C(k1:N, k1:N) -= P P^T with P the panel's columns,
+// split = 3 (three-term FP16 hi/lo products, about FP32 accuracy), 1 (TF32) or
+// 2 (BF16).  launch_tc_pack first writes P as tensor-core images into `pack`
+// (tc_pack_bytes(nf, cap) bytes, cap = tc_pack_cap(n, N, K, w)); launch_trail_tc
+// then reads P only from there.  rscale / dofs (split = 3): the power-of-two
+// scale of each DOF's row (launch_row_scale) and the DOF table; without them a
+// fixed scale for entries below 64 in magnitude.
 int tc_outer();
 int tc_max_fronts();
 // The panel is [K, K + w) (w a multiple of 32, at most tc_outer()); the
@@ -176,7 +180,8 @@ int64_t tc_tiles(const std::vector<int>& n, const std::vector<int>& N, int K, in
 int tc_pack_cap(const std::vector<int>& n, const std::vector<int>& N, int K, int w);
 size_t tc_pack_bytes(int nf, int cap);
 cudaError_t launch_tc_pack(const int* flist, int nf, int cap, const FrontDev* fr, const float* F,
-                           int K, int w, int split, void* pack, cudaStream_t st);
+                           int K, int w, int split, void* pack, cudaStream_t st,
+                           const float* rscale = nullptr, const int* dofs = nullptr);
 // Panel-by-panel partial Cholesky without grid barriers (kernels_panel.cu):
 // launch_subpanel turns the panel [Ks, Ks + w) of every front in flist into L
 // (w = panel_width(sizeof(T)): 64 FP64, 128 FP32; every earlier update
@@ -194,7 +199,8 @@ cudaError_t launch_trail_syrk(const int* flist, int nf, const FrontDev* fr, T* F
                               cudaStream_t st);
 cudaError_t launch_trail_tc(const int* flist, int nf, int64_t ntiles, const FrontDev* fr, float* F,
                             int K, int w, int cend, int split, int cap, const void* pack,
-                            DevError* err, cudaStream_t st);
+                            DevError* err, cudaStream_t st, const float* rscale = nullptr,
+                            const int* dofs = nullptr);
 
 // Cooperative sweeps over all fronts of one level (nrhs <= 16), ordered by
 // ready flags instead of grid barriers: forward = L11 solve and boundary update
@@ -288,6 +294,11 @@ void launch_apply(const int* cols, int ncols, const int* rows, int nrows, const 
 // Vector kernels of the mixed-precision solve (kernels_vec.cu).
 void launch_diag_scale(const int* rp, const int* ci, const double* va, int n, double* s,
                        double* is, cudaStream_t st);
+// r_i = 2^14 / sqrt(s_i a_ii s_i), rounded to a power of two so that the entries
+// of row i of the scaled matrix's Cholesky factor, at most that root, stay below
+// 2^14 in r_i L(i, :), for `count` matrices of nnz values each (n scales each).
+void launch_row_scale(const int* rp, const int* ci, const double* va, int n, int count, int64_t nnz,
+                      const double* s, float* r, cudaStream_t st);
 void launch_spmv(const int* rp, const int* ci, const double* va, int n, const double* x, int64_t ldx,
                  double* y, int64_t ldy, int nrhs, cudaStream_t st);
 void launch_residual(const int* rp, const int* ci, const double* va, int n, const double* b,

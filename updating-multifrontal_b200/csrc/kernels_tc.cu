@@ -12,12 +12,12 @@
 // is nearly all of the work.
 //
 // Two kernels per panel:
-//   * k_tc_pack writes the panel once, split into TF32 "hi" and "lo" parts
-//     (x = hi + lo, both exactly representable), as 8 KB images of 128 rows x
-//     16 columns in the K-major 64-byte-swizzled layout the tensor core reads:
-//     one CTA per (128-row block, 16-column chunk) reads its block coalesced
-//     from the column-major front and splits it in shared memory; per chunk
-//     the hi images of all row blocks are contiguous, then the lo images;
+//   * k_tc_pack writes the panel once, split into FP16 "hi" and "lo" parts
+//     (r x = hi + lo with a power of two r per row, below), as 8 KB images of
+//     128 rows x 32 columns in the K-major 64-byte-swizzled layout the tensor
+//     core reads: one CTA per (128-row block, 32-column chunk) reads its block
+//     coalesced from the column-major front and splits it in shared memory; per
+//     chunk the hi images of all row blocks are contiguous, then the lo images;
 //   * k_trail_tc, a persistent warp-specialised pipeline over 128 x 256 tiles
 //     of C (block row I of 128 rows, block column J of 256 columns, lower
 //     triangle only):
@@ -26,23 +26,36 @@
 //         blocks of the column block) into a ring of four shared-memory
 //         stages with bulk asynchronous copies (cp.async.bulk, completion
 //         counted in bytes on an mbarrier);
-//       - one MMA warp issues tcgen05.mma (kind::tf32, M = 128, N = 256,
-//         K = 8) from an elected lane into one of two tensor-memory
-//         accumulators (256 columns each, all of tensor memory):
-//             SPLIT = 3:  acc += hi_a hi_b^T + hi_a lo_b^T + lo_a hi_b^T
-//             SPLIT = 1:  acc += hi_a hi_b^T
-//             SPLIT = 2:  acc += a b^T in BF16 (kind::f16, K = 16; the pack
-//                         writes BF16 images of 32 columns, the same 8 KB size)
+//       - one MMA warp issues tcgen05.mma (M = 128, N = 256) from an elected
+//         lane into one of two tensor-memory accumulators (256 columns each,
+//         all of tensor memory):
+//             SPLIT = 3:  acc += hi_a hi_b^T + hi_a lo_b^T + lo_a hi_b^T in FP16
+//                         (kind::f16, K = 16)
+//             SPLIT = 1:  acc += a b^T in TF32 (kind::tf32, K = 8, images of 16
+//                         columns)
+//             SPLIT = 2:  acc += a b^T in BF16 (kind::f16, K = 16)
 //         and hands stages back to the producer with tcgen05.commit;
 //       - eight epilogue warps (two per accumulator lane quarter, 128 columns
 //         each, 32 at a time) read the accumulator with tcgen05.ld and
 //         subtract it from C in place; the first 32 values of C are loaded
 //         before the accumulator is ready.
 // A 256-column tile reads 25% fewer operand bytes per product than a 128 x 128
-// one, and 16-column stages keep three stages in flight.  MN-major TF32
-// operands would let the tensor core read the column-major front directly,
-// but they read back as zeros on sm_100a, hence the pack.  The three-term form
-// keeps products to about 2^-21 relative error, close to FP32.
+// one, and 48 KB stages keep three in flight.  MN-major TF32 operands would let
+// the tensor core read the column-major front directly, but they read back as
+// zeros on sm_100a, hence the pack.
+//
+// The three-term form takes FP16 parts because FP16 and TF32 carry the same 11
+// significant bits, so hi + lo keeps 22 of them either way and a product about
+// 2^-21, close to FP32, while FP16 runs at twice the rate and half the bytes.
+// What FP16 lacks is range, and a Cholesky factor needs little: the entries of
+// row i are at most sqrt(a_ii), so scaled by r_i = 2^14 / that bound (rounded to
+// a power of two, k_row_scale) they fill [0, 2^14], far below FP16's 65504, and
+// keep their 22 bits down to 2^-17 of the bound, an absolute 2^-39 of it below
+// (the sums they enter are rounded to FP32, 2^-24).  The epilogue divides by
+// r_i r_j exactly.  Against three-term TF32: updates of a 3D 95^3 factorization
+// and localized update 107 -> 77 ms, worst error against an FP64 product
+// (tests/cpp/tc_kernel_check.cu) 7.1e-6 -> 4.9e-6, residual after one refinement
+// step at 95^3 3.3e-10 -> 2.3e-10.
 //
 // Every mbarrier wait is bounded (kSpinLimit polls, or the limit the host put
 // in the error word); on expiry (or once another warp gave up) the kernel
@@ -50,6 +63,7 @@
 // its own copies and products in flight, releases its tensor memory and
 // returns.
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 
 #include <atomic>
 #include <cstdint>
@@ -65,14 +79,15 @@ namespace {
 constexpr int TM = 128;                    // C tile rows = accumulator lanes = image rows
 constexpr int TN = 256;                    // C tile columns = accumulator columns
 constexpr int TK = 16;                     // TF32: panel columns per chunk (64-byte image rows)
-constexpr int TK16 = 32;                   // BF16: panel columns per chunk (64-byte image rows)
+constexpr int TK16 = 32;                   // FP16, BF16: panel columns per chunk (64-byte image rows)
+constexpr float kPlainScale = 1024.0f;     // r without a row-scale table: entries below 64
 constexpr int NSTAGE = 4;                  // shared-memory stages
 constexpr int NACC = 2;                    // tensor-memory accumulators
 constexpr int MMA_WARP = 1;                // warp 0 produces, warp 1 issues the MMAs
 constexpr int EPI_WARP0 = 2;               // warps 2..9 run the epilogue
 constexpr int NEPI = 8;
 constexpr int TCT = (EPI_WARP0 + NEPI) * 32;   // 320 threads
-constexpr int IMG = TM * TK * 4;           // one image of 128 rows x 16 columns, 8 KB
+constexpr int IMG = TM * TK * 4;           // one image of 128 rows x 64 bytes, 8 KB
 constexpr int STAGE_BYTES = 6 * IMG;       // a_hi, a_lo, b_hi (2 blocks), b_lo (2 blocks)
 constexpr int kTcSmem = NSTAGE * STAGE_BYTES + 1024;   // + alignment slack
 constexpr int kMaxTcFronts = 1024;
@@ -87,15 +102,18 @@ __host__ __device__ constexpr int img_off(int m, int k) {
 }
 
 // Instruction descriptors: D = F32, both operands K-major, M = 128, N = 256;
-// A = B = TF32 (kind::tf32) or A = B = BF16 (kind::f16; never mixed types).
+// A = B = TF32 (kind::tf32), or A = B = BF16 or A = B = FP16 (kind::f16; never
+// mixed types).
 constexpr uint32_t kIdesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(TN >> 3) << 17) |
                             ((uint32_t)(TM >> 4) << 24);
 constexpr uint32_t kIdescBf16 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TN >> 3) << 17) |
                                 ((uint32_t)(TM >> 4) << 24);
 
-// Panel columns per chunk of each mode: SPLIT = 3 three-term TF32, 1 plain
-// TF32 (16 columns), 2 plain BF16 (one product, 32 columns).
-__host__ __device__ constexpr int chunk_cols(int split) { return split == 2 ? TK16 : TK; }
+constexpr uint32_t kIdescF16 = (1u << 4) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
+
+// Panel columns per chunk of each mode: SPLIT = 3 three-term FP16, 2 plain BF16
+// (32 columns), 1 plain TF32 (16 columns).
+__host__ __device__ constexpr int chunk_cols(int split) { return split == 1 ? TK : TK16; }
 
 // Panel geometry of a front for the panel [K, K + w): k1, 128-row blocks
 // below k1, 16-column chunks in [K, k1), the column bound cmax (cend < 0: N,
@@ -253,12 +271,13 @@ __device__ __forceinline__ void mma_tf32(uint32_t d_tmem, uint64_t a, uint64_t b
       "l"(a), "l"(b), "r"(kIdesc), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
 }
 
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t acc) {
+template <uint32_t IDESC>
+__device__ __forceinline__ void mma_16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t acc) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}" ::"r"(d_tmem),
-      "l"(a), "l"(b), "r"(kIdescBf16), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
+      "l"(a), "l"(b), "r"(IDESC), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
 }
 
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
@@ -297,6 +316,7 @@ struct TileInfo {
   float* A;
   int64_t ld;
   int N, k1, cmax, r0, c0, nch, nb, slot, I, J;
+  int64_t dof_off, rs_off;
 };
 
 __device__ __forceinline__ TileInfo tile_info(const int* pre, int nf, const int* flist,
@@ -319,6 +339,8 @@ __device__ __forceinline__ TileInfo tile_info(const int* pre, int nf, const int*
   t.nch = g.nch;
   t.nb = g.nb;
   t.slot = lo;
+  t.dof_off = d.dof_off;
+  t.rs_off = d.rs_off;
   tile_ij(tile - pre[lo], g.nb, g.nj, t.I, t.J);
   t.r0 = t.k1 + t.I * TM;
   t.c0 = t.k1 + t.J * TN;
@@ -326,15 +348,17 @@ __device__ __forceinline__ TileInfo tile_info(const int* pre, int nf, const int*
 }
 
 // Pack: CTA (x, i) = chunk c, row block b (x = c * nb + b) of front slot i:
-// rows k1 + 128 b + t (thread t), columns K + 16 c .. +15; zeros outside the
-// front and beyond k1.  Front slot i owns bytes [i * cap * 2 * IMG, +cap * 2 *
+// rows k1 + 128 b + t (thread t), columns K + tk c .. + tk - 1 (tk = 32 or 16);
+// zeros outside the front and beyond k1.  Front slot i owns bytes [i * cap * 2 * IMG, +cap * 2 *
 // IMG) of pack; inside, the hi image of (c, b) is image (2 c) * nb + b and the
 // lo image (2 c + 1) * nb + b.
 template <int SPLIT>
 __global__ void __launch_bounds__(128) k_tc_pack(const int* __restrict__ flist,
                                                  const FrontDev* __restrict__ fr,
                                                  const float* __restrict__ F, int K, int w,
-                                                 int cap, unsigned char* __restrict__ pack) {
+                                                 int cap, unsigned char* __restrict__ pack,
+                                                 const float* __restrict__ rscale,
+                                                 const int* __restrict__ dofs) {
   __shared__ __align__(1024) unsigned char img[2 * IMG];
   const FrontDev d = fr[flist[blockIdx.y]];
   constexpr int tk = chunk_cols(SPLIT);
@@ -363,29 +387,45 @@ __global__ void __launch_bounds__(128) k_tc_pack(const int* __restrict__ flist,
       *reinterpret_cast<uint4*>(img + t * 64 + ((q ^ ((t >> 1) & 3)) << 4)) =
           make_uint4(pk[0], pk[1], pk[2], pk[3]);
     }
+  } else if (SPLIT == 3) {
+    // FP16 hi and lo of the scaled entries, the same layout
+    const float r = !row_ok ? 0.0f : rscale ? rscale[d.rs_off + dofs[d.dof_off + row]] : kPlainScale;
+#pragma unroll
+    for (int q = 0; q < TK16 / 8; q++) {
+      float v[8];
+#pragma unroll
+      for (int j = 0; j < 8; j++)
+        v[j] = (row_ok && 8 * q + j < kend) ? __ldg(src + (int64_t)(8 * q + j) * d.ld) : 0.0f;
+      uint32_t hi[4], lo[4];
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const float x0 = v[2 * j] * r, x1 = v[2 * j + 1] * r;
+        const __half2 h = __floats2half2_rn(x0, x1);   // .x = x0 at the lower address
+        const float2 f = __half22float2(h);
+        const __half2 l = __floats2half2_rn(x0 - f.x, x1 - f.y);
+        hi[j] = *reinterpret_cast<const uint32_t*>(&h);
+        lo[j] = *reinterpret_cast<const uint32_t*>(&l);
+      }
+      unsigned char* at = img + t * 64 + ((q ^ ((t >> 1) & 3)) << 4);
+      *reinterpret_cast<uint4*>(at) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+      *reinterpret_cast<uint4*>(at + IMG) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    }
   } else {
 #pragma unroll
-  for (int q = 0; q < TK / 4; q++) {
-    float v[4];
+    for (int q = 0; q < TK / 4; q++) {
+      float v[4];
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int k = 4 * q + j;
-      v[j] = (row_ok && k < kend) ? __ldg(src + (int64_t)k * d.ld) : 0.0f;
+      for (int j = 0; j < 4; j++) {
+        const int k = 4 * q + j;
+        v[j] = (row_ok && k < kend) ? __ldg(src + (int64_t)k * d.ld) : 0.0f;
+      }
+      float4 h;
+      h.x = tf32_round(v[0]);
+      h.y = tf32_round(v[1]);
+      h.z = tf32_round(v[2]);
+      h.w = tf32_round(v[3]);
+      *reinterpret_cast<float4*>(img + img_off(t, 4 * q)) = h;
     }
-    float4 h, l;
-    h.x = tf32_round(v[0]);
-    h.y = tf32_round(v[1]);
-    h.z = tf32_round(v[2]);
-    h.w = tf32_round(v[3]);
-    *reinterpret_cast<float4*>(img + img_off(t, 4 * q)) = h;
-    if (SPLIT == 3) {
-      l.x = tf32_round(v[0] - h.x);
-      l.y = tf32_round(v[1] - h.y);
-      l.z = tf32_round(v[2] - h.z);
-      l.w = tf32_round(v[3] - h.w);
-      *reinterpret_cast<float4*>(img + IMG + img_off(t, 4 * q)) = l;
-    }
-  }
   }
   __syncthreads();
   unsigned char* base = pack + (int64_t)blockIdx.y * cap * 2 * IMG;
@@ -404,7 +444,9 @@ __global__ void __launch_bounds__(TCT, 1) k_trail_tc(const int* __restrict__ fli
                                                      const FrontDev* __restrict__ fr,
                                                      float* __restrict__ F, int K, int w, int cend,
                                                      int cap, const unsigned char* __restrict__ pack,
-                                                     DevError* err) {
+                                                     DevError* err,
+                                                     const float* __restrict__ rscale,
+                                                     const int* __restrict__ dofs) {
   extern __shared__ unsigned char tc_raw[];
   __shared__ uint64_t full[NSTAGE], empty[NSTAGE], acc_full[NACC], acc_empty[NACC], drain;
   __shared__ uint32_t tmem_base;
@@ -516,16 +558,16 @@ __global__ void __launch_bounds__(TCT, 1) k_trail_tc(const int* __restrict__ fli
           const uint32_t a_hi = in ? b_hi + ia * IMG : st, a_lo = in ? b_lo + ia * IMG : st + IMG;
 #pragma unroll
           for (int kk = 0; kk < 2; kk++) {
-            // K = 8 TF32 or K = 16 BF16 values: 32 bytes along the swizzled row
+            // K = 8 TF32 or K = 16 FP16 / BF16 values: 32 bytes along the swizzled row
             const uint32_t ko = kk * 32;
-            if (SPLIT == 2) {
-              mma_bf16(dacc, sw64_desc(a_hi + ko), sw64_desc(b_hi + ko), (c | kk) != 0);
-              continue;
-            }
-            mma_tf32(dacc, sw64_desc(a_hi + ko), sw64_desc(b_hi + ko), (c | kk) != 0);
-            if (SPLIT == 3) {
-              mma_tf32(dacc, sw64_desc(a_hi + ko), sw64_desc(b_lo + ko), 1u);
-              mma_tf32(dacc, sw64_desc(a_lo + ko), sw64_desc(b_hi + ko), 1u);
+            if (SPLIT == 1) {
+              mma_tf32(dacc, sw64_desc(a_hi + ko), sw64_desc(b_hi + ko), (c | kk) != 0);
+            } else if (SPLIT == 2) {
+              mma_16<kIdescBf16>(dacc, sw64_desc(a_hi + ko), sw64_desc(b_hi + ko), (c | kk) != 0);
+            } else {
+              mma_16<kIdescF16>(dacc, sw64_desc(a_hi + ko), sw64_desc(b_hi + ko), (c | kk) != 0);
+              mma_16<kIdescF16>(dacc, sw64_desc(a_hi + ko), sw64_desc(b_lo + ko), 1u);
+              mma_16<kIdescF16>(dacc, sw64_desc(a_lo + ko), sw64_desc(b_hi + ko), 1u);
             }
           }
           mma_commit(&empty[s]);
@@ -562,10 +604,19 @@ __global__ void __launch_bounds__(TCT, 1) k_trail_tc(const int* __restrict__ fli
       // accumulated, each later 32 once the previous ones are stored
       const int jmax = live ? min(row, ti.cmax - 1) - cb : -1;
       const uint32_t src = tmem + b * TN + half * (TN / 2) + ((uint32_t)(quarter * 32) << 16);
+      // FP16 parts: the accumulator holds r_i r_j times the product
+      const int* dl = dofs + ti.dof_off;
+      const float* rs = rscale ? rscale + ti.rs_off : nullptr;
+      float ir = 1.0f;
+      if (SPLIT == 3) ir = rs ? (live ? 1.0f / rs[dl[row]] : 0.0f) : 1.0f / kPlainScale;
       bool ok = true;
 #pragma unroll 1
       for (int h2 = 0; h2 < TN / 64; h2++) {
-        float cv[32];
+        float cv[32], ic = 1.0f;
+        if (SPLIT == 3) {
+          const int col = cb + 32 * h2 + lane;
+          ic = rs ? (col < ti.N ? 1.0f / rs[dl[col]] : 0.0f) : 1.0f / kPlainScale;
+        }
         const float* q = p + (int64_t)(32 * h2) * ti.ld;
 #pragma unroll
         for (int j = 0; j < 32; j++, q += ti.ld) cv[j] = 32 * h2 + j <= jmax ? *q : 0.0f;
@@ -582,8 +633,11 @@ __global__ void __launch_bounds__(TCT, 1) k_trail_tc(const int* __restrict__ fli
           uint32_t v[16];
           tmem_ld16(src + 32 * h2 + 16 * qb, v);
 #pragma unroll
-          for (int j = 0; j < 16; j++, wp += ti.ld)
-            if (32 * h2 + 16 * qb + j <= jmax) *wp = cv[16 * qb + j] - __uint_as_float(v[j]);
+          for (int j = 0; j < 16; j++, wp += ti.ld) {
+            const float inv = SPLIT == 3 ? ir * __shfl_sync(0xffffffffu, ic, 16 * qb + j) : 1.0f;
+            if (32 * h2 + 16 * qb + j <= jmax)
+              *wp = fmaf(-inv, __uint_as_float(v[j]), cv[16 * qb + j]);
+          }
         }
       }
       if (!ok) break;
@@ -638,24 +692,25 @@ int tc_setup() {   // thread-safe one-time set-up (static local initialisation)
 }  // namespace
 
 cudaError_t launch_tc_pack(const int* flist, int nf, int cap, const FrontDev* fr, const float* F,
-                           int K, int w, int split, void* pack, cudaStream_t st) {
+                           int K, int w, int split, void* pack, cudaStream_t st,
+                           const float* rscale, const int* dofs) {
   if (nf <= 0 || cap <= 0) return cudaSuccess;
   if (nf > 65535 || split < 1 || split > 3 || w <= 0 || w % chunk_cols(split) || w > kTcOuter)
     return cudaErrorInvalidValue;
   const dim3 grid((unsigned)cap, (unsigned)nf);
   if (split == 3)
-    k_tc_pack<3><<<grid, 128, 0, st>>>(flist, fr, F, K, w, cap, (unsigned char*)pack);
+    k_tc_pack<3><<<grid, 128, 0, st>>>(flist, fr, F, K, w, cap, (unsigned char*)pack, rscale, dofs);
   else if (split == 2)
-    k_tc_pack<2><<<grid, 128, 0, st>>>(flist, fr, F, K, w, cap, (unsigned char*)pack);
+    k_tc_pack<2><<<grid, 128, 0, st>>>(flist, fr, F, K, w, cap, (unsigned char*)pack, rscale, dofs);
   else
-    k_tc_pack<1><<<grid, 128, 0, st>>>(flist, fr, F, K, w, cap, (unsigned char*)pack);
+    k_tc_pack<1><<<grid, 128, 0, st>>>(flist, fr, F, K, w, cap, (unsigned char*)pack, rscale, dofs);
   g_launches++;
   return cudaGetLastError();
 }
 
 cudaError_t launch_trail_tc(const int* flist, int nf, int64_t ntiles, const FrontDev* fr, float* F,
                             int K, int w, int cend, int split, int cap, const void* pack,
-                            DevError* err, cudaStream_t st) {
+                            DevError* err, cudaStream_t st, const float* rscale, const int* dofs) {
   if (nf <= 0 || ntiles <= 0) return cudaSuccess;
   if (nf > kMaxTcFronts || split < 1 || split > 3 || !pack || w <= 0 ||
       w % chunk_cols(split) || w > kTcOuter)
@@ -663,13 +718,13 @@ cudaError_t launch_trail_tc(const int* flist, int nf, int64_t ntiles, const Fron
   const int grid = (int)std::min<int64_t>(ntiles, tc_setup());
   if (split == 3)
     k_trail_tc<3><<<grid, TCT, kTcSmem, st>>>(flist, nf, fr, F, K, w, cend, cap,
-                                              (const unsigned char*)pack, err);
+                                              (const unsigned char*)pack, err, rscale, dofs);
   else if (split == 2)
     k_trail_tc<2><<<grid, TCT, kTcSmem, st>>>(flist, nf, fr, F, K, w, cend, cap,
-                                              (const unsigned char*)pack, err);
+                                              (const unsigned char*)pack, err, rscale, dofs);
   else
     k_trail_tc<1><<<grid, TCT, kTcSmem, st>>>(flist, nf, fr, F, K, w, cend, cap,
-                                              (const unsigned char*)pack, err);
+                                              (const unsigned char*)pack, err, rscale, dofs);
   g_launches++;
   return cudaGetLastError();
 }

@@ -64,7 +64,12 @@ constexpr size_t tile_smem() {
 static_assert(B * DS <= 4 * KS * TS, "the diagonal tile's work array fits the stages");
 
 __device__ __forceinline__ double rsq(double x) { return rsqrt(x); }
-__device__ __forceinline__ float rsq(float x) { return rsqrtf(x); }
+// One Newton step on rsqrtf (up to two units off): L's diagonal, its reciprocal
+// and the inverse then agree to rounding.
+__device__ __forceinline__ float rsq(float x) {
+  const float r = rsqrtf(x);
+  return fmaf(0.5f * r, fmaf(-x * r, r, 1.0f), r);
+}
 
 // 16 bytes global -> shared through L2 only (L written by other SMs in this
 // launch), the last (16 - bytes) zero.

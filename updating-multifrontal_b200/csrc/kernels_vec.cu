@@ -32,6 +32,24 @@ __global__ void k_diag_scale(const int* __restrict__ rp, const int* __restrict__
   is[i] = r;
 }
 
+// Row scales of the three-term FP16 products (see device.cuh): matrix
+// blockIdx.y of the batch, a thread per row.  The slack keeps a row whose
+// diagonal is one to rounding at 2^14.
+__global__ void k_row_scale(const int* __restrict__ rp, const int* __restrict__ ci,
+                            const double* __restrict__ va, int n, int64_t nnz,
+                            const double* __restrict__ s, float* __restrict__ r) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  va += blockIdx.y * nnz;
+  double d = 0.0;
+  for (int p = rp[i]; p < rp[i + 1]; p++)
+    if (ci[p] == i) d = va[p];
+  const double b = sqrt(d > 0.0 ? d : 1.0) * s[i] * (1.0 - 1e-6);
+  int e;
+  frexp(b, &e);   // b < 2^e
+  r[i + (int64_t)blockIdx.y * n] = ldexpf(1.0f, 14 - max(-60, min(60, e)));
+}
+
 // y = A x, one thread per row and column (rows of a 5/7-point stencil are short).
 __global__ void k_spmv(const int* __restrict__ rp, const int* __restrict__ ci,
                        const double* __restrict__ va, int n, const double* __restrict__ x,
@@ -176,6 +194,12 @@ inline dim3 vgrid(int n, int nrhs) { return dim3((n + VT - 1) / VT, nrhs); }
 void launch_diag_scale(const int* rp, const int* ci, const double* va, int n, double* s,
                        double* is, cudaStream_t st) {
   k_diag_scale<<<(n + VT - 1) / VT, VT, 0, st>>>(rp, ci, va, n, s, is);
+  g_launches++;
+}
+
+void launch_row_scale(const int* rp, const int* ci, const double* va, int n, int count, int64_t nnz,
+                      const double* s, float* r, cudaStream_t st) {
+  k_row_scale<<<dim3((n + VT - 1) / VT, count), VT, 0, st>>>(rp, ci, va, n, nnz, s, r);
   g_launches++;
 }
 

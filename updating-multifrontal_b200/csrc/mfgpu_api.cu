@@ -386,6 +386,8 @@ struct mfgpu_handle {
   size_t esz = sizeof(double);     // bytes per factor element
   double* d_scale = nullptr;       // s = 1/sqrt(diag(A)) of the last full factorization
   double* d_iscale = nullptr;      // 1/s
+  float* d_rscale = nullptr;       // mixed: row scales of the tensor-core panels' FP16 parts
+  int nmat = 1;                    // matrices of d_val (the serving loop's batches: several)
   double *d_B = nullptr, *d_R = nullptr, *d_P = nullptr, *d_Q = nullptr, *d_Z = nullptr;
   size_t capB = 0, capR = 0, capP = 0, capQ = 0, capZ = 0;
   float* d_x32 = nullptr;
@@ -451,6 +453,7 @@ struct mfgpu_handle {
       cudaFree(d_flow);
     }
     cudaFree(d_flags);
+    cudaFree(d_rscale);
     cudaFree(d_Dinv);
     cudaFree(d_val);
     cudaFree(d_fr);
@@ -1004,6 +1007,7 @@ struct mfgpu_handle {
     ensureDone(P);
     if (mixed) {
       mfgpu::launch_diag_scale(d_rp, d_ci, d_val, n, d_scale, d_iscale, stream);
+      mfgpu::launch_row_scale(d_rp, d_ci, d_val, n, nmat, nnz, d_scale, d_rscale, stream);
       ck(cudaGetLastError(), "launch diagonal scaling");
     }
     clearErr();
@@ -1058,11 +1062,15 @@ struct mfgpu_handle {
   // the trailing update of each panel on the tensor cores.
   // A level also goes to the tensor cores with fronts of a quarter of tcMinN
   // when it has at least one front per SM (enough tiles to fill the GPU; 3D
-  // 127^3 level 3: 512 fronts, N <= 1981); levels with a few such fronts (the
-  // top of a 2D tree) stay on the cooperative kernel, which is faster there.
+  // 127^3 level 3: 512 fronts, N <= 1981), unless their panels fit one CTA's
+  // shared memory (N <= 1408): there, and in levels with a few such fronts (the
+  // top of a 2D tree), FP32 tiles cost little and round less (3D 95^3
+  // level 3, 512 fronts, N <= 1057: 3.4 ms on the tensor cores, 5.7 by tiles; the
+  // residual after one refinement step 4.8e-10 against 2.3e-10).
   bool tcLevel(const Plan::Level& L) const {
     if (tcMinN <= 0 || L.nf > mfgpu::tc_max_fronts()) return false;
-    return L.maxN >= tcMinN || (L.nf >= 148 && L.maxN >= tcMinN / 4);
+    return L.maxN >= tcMinN || (L.nf >= 148 && L.maxN >= tcMinN / 4 &&
+                                !mfgpu::small_front_fits(L.maxN, (int)esz));
   }
 
   // Tensor-core level (mixed path).  Per 512-column outer panel [K, K + 512):
@@ -1105,10 +1113,10 @@ struct mfgpu_handle {
         throw CudaError("tensor-core panel pack larger than planned", MFGPU_ERR_STATE);
       prof.begin(MFGPU_KC_TC, stream);
       ck(mfgpu::launch_tc_pack(P.d_ids + L.f0, (int)L.nf, cap, d_fr, (const float*)d_F, K0, pw,
-                               split, d_tcpack, stream),
+                               split, d_tcpack, stream, d_rscale, d_dofs),
          "launch tensor-core panel pack (k_tc_pack)");
       ck(mfgpu::launch_trail_tc(P.d_ids + L.f0, (int)L.nf, nt, d_fr, (float*)d_F, K0, pw, cend,
-                                split, cap, d_tcpack, d_err, stream),
+                                split, cap, d_tcpack, d_err, stream, d_rscale, d_dofs),
          "launch tensor-core update (k_trail_tc)");
       prof.end(stream);
     };
@@ -1184,7 +1192,19 @@ struct mfgpu_handle {
       mfgpu::launch_diag_scale(d_rp, d_ci, d_val, n, d_scale, d_iscale, stream);
       ck(cudaGetLastError(), "launch diagonal scaling");
     }
+    rowScales(P);
     runPlan(P);
+  }
+
+  // Row scales of the tensor-core panels for the current values.
+  void rowScales(const Plan& P) {
+    if (!mixed) return;
+    bool any = P.tcPackBytes > 0;
+    if (&P == &full)
+      for (int k : tuned) any |= k == LK_TC;
+    if (!any) return;
+    mfgpu::launch_row_scale(d_rp, d_ci, d_val, n, nmat, nnz, d_scale, d_rscale, stream);
+    ck(cudaGetLastError(), "launch row scales (k_row_scale)");
   }
 
   // Reset the error word before a call's launches (a memset, so it can be
@@ -1738,6 +1758,7 @@ int createFrom(std::unique_ptr<Schedule> sched, int n, const int* row_ptr, const
       H.nchunks = (int)chunkrow.size() - 1;
       H.d_scale = dalloc<double>(n, "alloc scaling");
       H.d_iscale = dalloc<double>(n, "alloc scaling");
+      H.d_rscale = dalloc<float>(n, "alloc row scales");
       H.d_sc = dalloc<double>(80 * (size_t)H.nseg, "alloc refinement scalars");
       H.d_active = dalloc<int>(16 * (size_t)H.nseg, "alloc refinement flags");
       H.d_segrow = dalloc<int>(segrow32.size(), "alloc segments");
@@ -2649,6 +2670,7 @@ struct mfgpu_server {
   unsigned char* d_DinvB = nullptr;
   FrontDev* d_frB = nullptr;
   int64_t* d_dinv_offB = nullptr;
+  float* d_rsB = nullptr;              // row scales, mixed precision
   std::thread worker;
   std::mutex mu;
   std::condition_variable cv_queue, cv_done;
@@ -2672,6 +2694,7 @@ struct mfgpu_server {
     cudaFree(d_DinvB);
     cudaFree(d_frB);
     cudaFree(d_dinv_offB);
+    cudaFree(d_rsB);
     cudaFree(d_coef);
     cudaFree(d_pool);
   }
@@ -2771,7 +2794,10 @@ struct mfgpu_server {
     double* own_val = V.d_val;
     void* own_Dinv = V.d_Dinv;
     int64_t* own_doff = V.d_dinv_off;
+    float* own_rs = V.d_rscale;
     auto restore = [&]() {
+      V.d_rscale = own_rs;
+      V.nmat = 1;
       V.d_fr = own_fr;
       V.d_val = own_val;
       V.d_Dinv = own_Dinv;
@@ -2826,6 +2852,7 @@ struct mfgpu_server {
         std::copy(base_table.begin(), base_table.end(), tb);
         int nd = 0;
         for (int f = 0; f < nF; f++) {
+          tb[f].rs_off = (int64_t)r * V.n;
           if (m.dirty[f]) {
             tb[f].off = b.poolF + b.fnew[f];
             nd++;
@@ -2858,6 +2885,8 @@ struct mfgpu_server {
       V.d_val = d_valB;
       V.d_Dinv = d_DinvB;
       V.d_dinv_off = d_dinv_offB;
+      V.d_rscale = d_rsB;
+      V.nmat = (int)batch.size();
       V.factorWith(nullptr, true, V.upd, false);
       V.checkDevError();
       restore();
@@ -3034,6 +3063,7 @@ int mfgpu_server_create(mfgpu_handle* base, const double* d_coef, const double* 
     S->d_DinvB = dalloc<unsigned char>(
         (size_t)slots * std::max<int64_t>(base->dinvElems, 1) * base->esz, "alloc batch inverses");
     S->d_frB = dalloc<FrontDev>((size_t)(slots + 1) * nF, "alloc batch front table");
+    if (base->mixed) S->d_rsB = dalloc<float>((size_t)slots * base->n, "alloc batch row scales");
     S->d_dinv_offB = dalloc<int64_t>((size_t)(slots + 1) * nF, "alloc batch inverse offsets");
   });
   if (st != MFGPU_OK) return st;
