@@ -154,14 +154,19 @@ int coop_phases(int K, int maxn, int outer = 0);
 // (kernels_tile.cu).  tile_tasks appends a level's tasks (two ints each) and
 // the nf + 1 offsets of the fronts' block rows; done: rowoff[nf] + 1 ints of
 // scratch, cleared before each launch.  The inverses of the diagonal blocks
-// go to Dv where dinv_off[front] >= 0.
+// go to Dv where dinv_off[front] >= 0.  kbeg (a multiple of 64) with the tasks of
+// tile_panel_tasks(n, N, kbeg, w): the panel [kbeg, kbeg + w) alone, panels in
+// order with the same `done`, every update by the columns left of it applied.
 constexpr int kTileBlock = 64;
 void tile_tasks(const std::vector<int>& n, const std::vector<int>& N, std::vector<int>& tasks,
                 std::vector<int>& rowoff);
+void tile_panel_tasks(const std::vector<int>& n, const std::vector<int>& N, int K, int w,
+                      std::vector<int>& tasks);
 template <class T>
 cudaError_t launch_front_tiles(const int* flist, const FrontDev* fr, T* F, const int* tasks,
                                int ntasks, const int* rowoff, int nrows, int* done, T* Dv,
-                               const int64_t* dinv_off, DevError* err, cudaStream_t st);
+                               const int64_t* dinv_off, DevError* err, cudaStream_t st,
+                               int kbeg = 0);
 
 // Tensor-core (tcgen05) trailing update of the mixed path after outer panel K
 // of every front in flist: C(k1:N, k1:N) -= P P^T with P the panel's columns,

@@ -16,8 +16,7 @@
 //                  substitution with L11 and those inverses: 128-row items
 //                  over a persistent grid of two CTAs per SM, 16 outputs
 //                  per thread in registers.
-// The trailing update then follows (k_trail_syrk here, the tensor-core update
-// on the mixed path's large levels).  The diagonal block is the only serial
+// The trailing update then follows (k_trail_syrk).  The diagonal block is the only serial
 // part and it is factored once, by one CTA; the panel below is plain
 // throughput work.  A non-positive pivot records error code 1 (front, column).
 #include <algorithm>

@@ -9,6 +9,10 @@
 //                       the inverse of the factor (diag_factor below);
 //   pivot tile (I, J)   A_IJ - sum_k L_Ik L_Jk^T, then times L_JJ^{-T};
 //   Schur tile (I, J)   A_IJ - sum_k L_Ik L_Jk^T over all pivot columns.
+// A launch may also cover one panel of block columns (kbeg: its first column):
+// the same pivot tiles, with the sums over the panel's columns only, for levels
+// whose trailing matrix takes each panel from another kernel (the tensor-core
+// levels of the mixed path).
 // Tiles are cut from row and column 0 of the front, so the block column that
 // holds the last pivots may hold boundary columns too: its tiles are listed
 // twice, once for the columns left of n, once for the Schur part.
@@ -325,7 +329,7 @@ __global__ void __launch_bounds__(TT, 3)
     k_front_tiles(const int* __restrict__ flist, const FrontDev* __restrict__ fr, T* __restrict__ F,
                   const int2* __restrict__ tasks, int ntasks, const int* __restrict__ rowoff,
                   int* done, int* counter, T* __restrict__ Dv,
-                  const int64_t* __restrict__ dinv_off, DevError* err) {
+                  const int64_t* __restrict__ dinv_off, DevError* err, int kbeg) {
   extern __shared__ __align__(16) unsigned char tile_raw[];
   T* sm = reinterpret_cast<T*>(tile_raw);
   __shared__ __align__(16) T q4[2][B][4];
@@ -398,9 +402,10 @@ __global__ void __launch_bounds__(TT, 3)
     });
     acc.zero();
     // stages of KS columns of block rows I and J
-    const int kend = schur ? n : c0, ns = (kend + KS - 1) / KS;
+    const int kend = schur ? n : c0, ns = (kend - kbeg + KS - 1) / KS;
+    auto block_of = [&](int s) { return (kbeg + s * KS) / B; };   // block column of stage s
     auto issue = [&](int s, int buf) {
-      const int k0 = s * KS;
+      const int k0 = kbeg + s * KS;
       T* X = sm + buf * 2 * KS * TS;
 #pragma unroll
       for (int o = 0; o < 2; o++) {
@@ -418,11 +423,11 @@ __global__ void __launch_bounds__(TT, 3)
     };
     int ready = 0;
     if (ns > 0) {
-      ready = wait(0);
+      ready = wait(block_of(0));
       issue(0, 0);
     }
     for (int s = 0; s < ns; s++) {
-      const bool more = s + 1 < ns, pre = more && (s + 1) * KS / B < ready;
+      const bool more = s + 1 < ns, pre = more && block_of(s + 1) < ready;
       if (pre) {
         issue(s + 1, (s + 1) & 1);
         cp_wait<1>();
@@ -438,7 +443,7 @@ __global__ void __launch_bounds__(TT, 3)
       }
       __syncthreads();
       if (more && !pre) {   // the next block column is not there yet: computed first, wait now
-        ready = wait((s + 1) * KS / B);
+        ready = wait(block_of(s + 1));
         issue(s + 1, (s + 1) & 1);
       }
     }
@@ -593,13 +598,28 @@ void tile_tasks(const std::vector<int>& n, const std::vector<int>& N, std::vecto
   }
 }
 
+// The pivot tiles of the block columns [K, K + w), diagonal tiles first.
+void tile_panel_tasks(const std::vector<int>& n, const std::vector<int>& N, int K, int w,
+                      std::vector<int>& tasks) {
+  for (int J = K / B; J < (K + w) / B; J++) {
+    for (size_t i = 0; i < n.size(); i++)
+      if (J * B < n[i]) tasks.insert(tasks.end(), {(int)i, J | (J << 15)});
+    for (size_t i = 0; i < n.size(); i++)
+      for (int I = J + 1; J * B < n[i] && I * B < N[i]; I++)
+        tasks.insert(tasks.end(), {(int)i, I | (J << 15)});
+  }
+}
+
 template <class T>
 cudaError_t launch_front_tiles(const int* flist, const FrontDev* fr, T* F, const int* tasks,
                                int ntasks, const int* rowoff, int nrows, int* done, T* Dv,
-                               const int64_t* dinv_off, DevError* err, cudaStream_t st) {
+                               const int64_t* dinv_off, DevError* err, cudaStream_t st, int kbeg) {
   if (ntasks <= 0) return cudaSuccess;
-  // done words and, behind them, the task counter
-  cudaError_t e = cudaMemsetAsync(done, 0, sizeof(int) * (size_t)(nrows + 1), st);
+  if (kbeg % B) return cudaErrorInvalidValue;
+  // done words and, behind them, the task counter; the words of a level
+  // factored by panels carry on from the panel before
+  cudaError_t e = kbeg == 0 ? cudaMemsetAsync(done, 0, sizeof(int) * (size_t)(nrows + 1), st)
+                            : cudaMemsetAsync(done + nrows, 0, sizeof(int), st);
   if (e != cudaSuccess) return e;
   static const int grid = []() {   // thread-safe one-time set-up: every resident CTA
     int dev = 0, sms = 0, per = 0;
@@ -612,16 +632,16 @@ cudaError_t launch_front_tiles(const int* flist, const FrontDev* fr, T* F, const
   }();
   k_front_tiles<T><<<std::min(grid, ntasks), TT, tile_smem<T>(), st>>>(
       flist, fr, F, reinterpret_cast<const int2*>(tasks), ntasks, rowoff, done, done + nrows, Dv,
-      dinv_off, err);
+      dinv_off, err, kbeg);
   g_launches++;
   return cudaGetLastError();
 }
 
 template cudaError_t launch_front_tiles<double>(const int*, const FrontDev*, double*, const int*, int,
                                                 const int*, int, int*, double*, const int64_t*,
-                                                DevError*, cudaStream_t);
+                                                DevError*, cudaStream_t, int);
 template cudaError_t launch_front_tiles<float>(const int*, const FrontDev*, float*, const int*, int,
                                                const int*, int, int*, float*, const int64_t*,
-                                               DevError*, cudaStream_t);
+                                               DevError*, cudaStream_t, int);
 
 }  // namespace mfgpu

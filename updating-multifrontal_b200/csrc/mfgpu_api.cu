@@ -93,6 +93,7 @@ struct Plan {
     int coopOuter = 0;    // outer panel width the phase prefixes were built with (0: default)
     int64_t tt0 = 0, tr0 = 0;   // tile tasks in ttask, block-row offsets in trow
     int ntt = 0, nrows = 0;     // tile tasks, block rows of all fronts
+    int64_t tp0 = 0;            // tensor-core levels: the outer panels' tile tasks, in tpanel
     // A batch plan (several problems' fronts in one plan, the serving loop's)
     // factors a level's fronts in consecutive partitions, each with the kernel
     // its problems would get alone: `subs` holds them (f0, nf, maxN, maxn,
@@ -110,6 +111,7 @@ struct Plan {
   std::vector<int> ids;
   std::vector<int> cpref;
   std::vector<int> ttask, trow;   // tile tasks (pairs) and block-row offsets
+  std::vector<int64_t> tpanel;    // per tensor-core level: offsets in ttask of its panels' tasks
   int maxRows = 0;                // most block rows of any tile launch
   int nfronts = 0;
   double flops = 0;
@@ -147,6 +149,7 @@ struct Plan {
     cpref.clear();
     ttask.clear();
     trow.clear();
+    tpanel.clear();
     maxRows = 0;
     nfronts = 0;
     flops = 0;
@@ -163,6 +166,26 @@ struct Plan {
     l.ntt = (int)((ttask.size() - l.tt0) / 2);
     l.nrows = trow.back();
     maxRows = std::max(maxRows, l.nrows);
+  }
+
+  // The same for a tensor-core level: the pivot tiles of each outer panel.
+  template <class L>
+  void addPanelTiles(L& l, const std::vector<int>& n, const std::vector<int>& N, int w) {
+    l.tr0 = (int64_t)trow.size();
+    int row = 0;
+    for (int x : N) {
+      trow.push_back(row);
+      row += (x + mfgpu::kTileBlock - 1) / mfgpu::kTileBlock;
+    }
+    trow.push_back(row);
+    l.nrows = row;
+    maxRows = std::max(maxRows, row);
+    l.tp0 = (int64_t)tpanel.size();
+    for (int K = 0; K < l.maxn; K += w) {
+      tpanel.push_back((int64_t)ttask.size());
+      mfgpu::tile_panel_tasks(n, N, K, w, ttask);
+    }
+    tpanel.push_back((int64_t)ttask.size());
   }
 
   // A group is built by beginGroup, appendGroup (the tasks of some owners,
@@ -243,6 +266,7 @@ struct Plan::Level::Sub {
   int coopItems = 0, coopOuter = 0;
   int64_t tt0 = 0, tr0 = 0;
   int ntt = 0, nrows = 0;
+  int64_t tp0 = 0;
   int kind = -1;
 };
 
@@ -379,8 +403,8 @@ struct mfgpu_handle {
                                    // tensor-core level (0 or 512: no sub-panels)
   int fusedMinFronts = 148;        // fewest fronts for the one-CTA-per-front kernel
   int fusedMaxN = 128;             // largest front for it
-  bool subpanel = true;            // tensor-core levels: sub-panels by k_diag_factor + k_panel_trsm
-                                   // (MFGPU_SUBPANEL=0: by the cooperative kernel)
+  bool subpanel = true;            // tensor-core levels: outer panels by tiles (MFGPU_SUBPANEL=0:
+                                   // sub-panels by the cooperative kernel)
   int panelMaxN = 0;               // largest front of a level factored panel by panel (0: never;
                                    // MFGPU_PANEL_MAX_N; the autotuner may still pick the kernel)
   size_t esz = sizeof(double);     // bytes per factor element
@@ -535,7 +559,11 @@ struct mfgpu_handle {
       }
       if (&P == &full || ruleKernel(L) == LK_COOP) P.addTiles(L, nn, NN);
       const bool tc = mixed && tcLevel(L);
-      if (tc || (mixed && &P == &full && tcCandidate(L))) {
+      if ((tc || (mixed && &P == &full && tcCandidate(L))) && subpanel) {
+        const int W = mfgpu::tc_outer();
+        P.addPanelTiles(L, nn, NN, W);
+        if (tc) P.tcPackBytes = std::max(P.tcPackBytes, packBytes(nn, NN, L.maxn, W));
+      } else if (tc || (mixed && &P == &full && tcCandidate(L))) {
         const int W = mfgpu::tc_outer();
         L.coopOuter = tc && tcSub > 0 && tcSub < W ? tcSub : 0;
         std::vector<int> pp = mfgpu::coop_phase_prefix(nn, NN, L.maxn, L.coopOuter);
@@ -621,7 +649,10 @@ struct mfgpu_handle {
         }
         u.nf = (int64_t)P.ids.size() - u.f0;
         if (kd == LK_COOP) P.addTiles(u, nn, NN);
-        if (kd == LK_TC) {
+        if (kd == LK_TC && subpanel) {
+          P.addPanelTiles(u, nn, NN, W);
+          P.tcPackBytes = std::max(P.tcPackBytes, packBytes(nn, NN, u.maxn, W));
+        } else if (kd == LK_TC) {
           u.coopOuter = tcSub > 0 && tcSub < W ? tcSub : 0;
           u.cpref0 = (int64_t)P.cpref.size();
           std::vector<int> pp = mfgpu::coop_phase_prefix(nn, NN, u.maxn, u.coopOuter);
@@ -740,6 +771,14 @@ struct mfgpu_handle {
   }
   bool tcCandidate(const Plan::Level& L) const {
     return L.nf <= mfgpu::tc_max_fronts() && L.maxN >= 1024;
+  }
+
+  // Panel-pack bytes of the outer panels of fronts of n pivots and N rows.
+  static size_t packBytes(const std::vector<int>& n, const std::vector<int>& N, int maxn, int W) {
+    size_t b = 0;
+    for (int K = 0; K < maxn; K += W)
+      b = std::max(b, mfgpu::tc_pack_bytes((int)n.size(), mfgpu::tc_pack_cap(n, N, K, W)));
+    return b;
   }
 
   // Panel-pack bytes a tensor-core run of level L needs (outer panels only when
@@ -875,7 +914,8 @@ struct mfgpu_handle {
       prof.flops[MFGPU_KC_COOP] += fl;
       runPanel<T>(P, L);
     }
-    if (kind != LK_COOP && L.nf > 0 && coopSweep(ell)) {
+    const bool tiles = kind == LK_COOP || (kind == LK_TC && subpanel);
+    if (!tiles && L.nf > 0 && coopSweep(ell)) {
       mfgpu::launch_diag_inv<T>(P.d_ids + L.f0, (int)L.nf, L.maxn, d_fr, F, (T*)d_Dinv, d_dinv_off,
                                 stream);
       ck(cudaGetLastError(), "launch diagonal-block inverses (k_diag_inv)");
@@ -975,6 +1015,7 @@ struct mfgpu_handle {
           Ls.ntt = u.ntt;
           Ls.tr0 = u.tr0;
           Ls.nrows = u.nrows;
+          Ls.tp0 = u.tp0;
           runLevelKernel<T>(P, Ls, ell, u.kind);
         }
       }
@@ -1073,15 +1114,16 @@ struct mfgpu_handle {
                                 !mfgpu::small_front_fits(L.maxN, (int)esz));
   }
 
-  // Tensor-core level (mixed path).  Per 512-column outer panel [K, K + 512):
-  // the cooperative kernel factors it one sub-panel [Ks, Ks + w) at a time
-  // (w = L.coopOuter, 32-column steps inside), and after each sub-panel the
-  // tensor cores update the outer panel's remaining columns [Ks + w, K + 512)
-  // of all rows below; then the tensor cores apply the whole outer panel to
-  // the trailing matrix.  With w = 512 (no sub-panels) only the trailing
-  // update remains.  Profile attribution: the tensor-core updates'
-  // algorithmic flops go to MFGPU_KC_TC, the rest of the level's flops
-  // (diagonal blocks, panel solves, in-sub-panel updates) to MFGPU_KC_COOP.
+  // Tensor-core level (mixed path).  Each 512-column outer panel [K, K + 512)
+  // is factored by one launch of FP32 tiles (k_front_tiles, 64-column steps
+  // ordered by ready words), then the tensor cores apply it to the trailing
+  // matrix.  (MFGPU_SUBPANEL=0: the cooperative kernel factors the panel one
+  // sub-panel of w = L.coopOuter columns at a time, the tensor cores updating
+  // the panel's remaining columns after each; w = 512: no sub-panels.)  Tiles
+  // against sub-panels of 128 columns (a diagonal-block, a panel-solve, a pack
+  // and an update launch each): PNPN.  Profile attribution: the tensor-core
+  // updates' algorithmic flops go to MFGPU_KC_TC, the rest of the level's flops
+  // to MFGPU_KC_COOP.
   void runTensorLevel(const Plan& P, const Plan::Level& L, double level_flops, int ell) {
     const Schedule& s = *S;
     const int split = tcSplit3Levels >= 0 && ell >= tcSplit3Levels ? tcSplitLow : tcSplit;
@@ -1120,22 +1162,26 @@ struct mfgpu_handle {
          "launch tensor-core update (k_trail_tc)");
       prof.end(stream);
     };
-    for (int K = 0; K < L.maxn; K += W) {
-      for (int Ks = K; Ks < K + W && Ks < L.maxn; Ks += w) {
+    for (int K = 0, pn = 0; K < L.maxn; K += W, pn++) {
+      if (subpanel) {
+        const int64_t t0 = P.tpanel[L.tp0 + pn], t1 = P.tpanel[L.tp0 + pn + 1];
         prof.begin(MFGPU_KC_COOP, stream);
-        if (subpanel && w == mfgpu::panel_width(sizeof(float)) && L.nf <= mfgpu::kMaxPanelFronts) {
-          ck(mfgpu::launch_subpanel<float>(P.d_ids + L.f0, (int)L.nf, d_fr, (float*)d_F, Ks, w,
-                                           (float*)d_pslot, d_err, stream),
-             "launch sub-panel factorization (k_diag_factor, k_panel_trsm)");
-        } else {
+        ck(mfgpu::launch_front_tiles<float>(P.d_ids + L.f0, d_fr, (float*)d_F, P.d_ttask + t0,
+                                            (int)((t1 - t0) / 2), P.d_trow + L.tr0, L.nrows, d_done,
+                                            (float*)d_Dinv, d_dinv_off, d_err, stream, K),
+           "launch panel factorization by tiles (k_front_tiles)");
+        prof.end(stream);
+      } else {
+        for (int Ks = K; Ks < K + W && Ks < L.maxn; Ks += w) {
+          prof.begin(MFGPU_KC_COOP, stream);
           ck(mfgpu::launch_level_coop<float>(P.d_ids + L.f0, (int)L.nf, L.maxn, d_fr, (float*)d_F,
                                              d_err, (float*)d_slots, P.d_cpref + L.cpref0, d_gbar,
                                              stream, Ks, Ks + w, phase0, 0, L.coopItems, w),
              "launch cooperative panel factorization (k_level_coop)");
+          prof.end(stream);
+          phase0 += mfgpu::coop_phases(Ks, L.maxn, w);
+          if (Ks + w < K + W) update(Ks, w, K + W);   // the outer panel's remaining columns
         }
-        prof.end(stream);
-        phase0 += mfgpu::coop_phases(Ks, L.maxn, w);
-        if (Ks + w < K + W) update(Ks, w, K + W);   // the outer panel's remaining columns
       }
       update(K, W, -1);   // the trailing matrix
     }
