@@ -6,11 +6,13 @@
 // (src/DE/mf2d.cpp:558-567).  Here each front is stored whole (column-major,
 // pivots first: [A22 A21; A12 A11]) and factored in place, right-looking, in
 // 32-column steps k:
-//   k_lu_panel       one CTA per front: columns [k, k + kb) over rows [k, N),
-//                    pivots chosen among the pivot rows [j, n) only (the
-//                    boundary rows are eliminated, never swapped, as in the
-//                    reference where A12 is outside dgetrf's matrix), row
-//                    swaps inside the panel, multipliers, in-panel update;
+//   k_lu_panel_rows  one CTA per front, up to 512 rows: columns [k, k + kb)
+//                    over rows [k, N), pivots chosen among the pivot rows
+//                    [j, n) only (the boundary rows are eliminated, never
+//                    swapped, as in the reference where A12 is outside dgetrf's
+//                    matrix), row swaps inside the panel, multipliers, in-panel
+//                    update; a row per thread, in registers;
+//   k_lu_panel       the same for more rows, in global memory;
 //   k_lu_swap_trsm   the panel's row swaps applied to every other column (the
 //                    L columns on the left too, LAPACK's convention, so that a
 //                    solve applies all swaps first), then U(k block, right) =
@@ -47,7 +49,104 @@ __device__ __forceinline__ void lu_report(DevError* err, int code, int front, in
   }
 }
 
-// Panel factorization with partial pivoting restricted to the pivot rows.
+// Panel factorization with partial pivoting restricted to the pivot rows, a row
+// of the panel per thread in registers (N - k <= blockDim.x <= 512).  Bound: the
+// chain of 32 pivot searches (latency).  A column costs two barriers: the warps'
+// candidates, then the pivot row and the row it changes places with through
+// shared memory; the updates touch registers only.  Panels of a 2D 127^2 tree
+// of width 2 (32 launches): 3738 us in global memory (five barriers a column, a
+// pass over the remaining columns in memory), 2128 us so; with the trailing
+// update's loads in flight together (1066 -> 308 us) factor + solve 4.99 -> 2.26 ms.
+constexpr int kLuPanelRows = 512;
+__global__ void __launch_bounds__(kLuPanelRows, 1)
+    k_lu_panel_rows(const int* __restrict__ flist, const FrontDev* __restrict__ fr,
+                    double* __restrict__ F, int* __restrict__ ipiv, int k, DevError* err) {
+  const int f = flist[blockIdx.x];
+  const FrontDev d = fr[f];
+  if (k >= d.n) return;
+  const int kb = min(kPanel, d.n - k), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nw = blockDim.x >> 5, i = k + tid;
+  const bool live = i < d.N;
+  double* A = F + d.off + (live ? i : 0) + (int64_t)k * d.ld;
+  __shared__ double prow[2][kPanel], jrow[2][kPanel];   // the pivot row, the row it replaces
+  __shared__ double wbest[2][kLuPanelRows / 32];
+  __shared__ int widx[2][kLuPanelRows / 32];
+  double row[kPanel];
+#pragma unroll
+  for (int c = 0; c < kPanel; c++) row[c] = live && c < kb ? A[(int64_t)c * d.ld] : 0.0;
+#pragma unroll
+  for (int jj = 0; jj < kPanel; jj++) {
+    if (jj < kb) {
+      const int j = k + jj, b = jj & 1;
+      // the first row of largest magnitude in column j among rows [j, n)
+      double best = -1.0;
+      int bi = d.n;
+      if (i >= j && i < d.n && fabs(row[jj]) > best) {
+        best = fabs(row[jj]);
+        bi = i;
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+        if (ob > best || (ob == best && oi < bi)) {
+          best = ob;
+          bi = oi;
+        }
+      }
+      if (lane == 0) {
+        wbest[b][warp] = best;
+        widx[b][warp] = bi;
+      }
+      __syncthreads();
+      best = lane < nw ? wbest[b][lane] : -1.0;
+      bi = lane < nw ? widx[b][lane] : d.n;
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) {   // at most 16 warps
+        const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+        if (ob > best || (ob == best && oi < bi)) {
+          best = ob;
+          bi = oi;
+        }
+      }
+      int p = __shfl_sync(0xffffffffu, bi, 0);
+      const double mag = __shfl_sync(0xffffffffu, best, 0);
+      if (!(mag > 0.0) || p >= d.n) {   // zero (or NaN) column: the pivot block is singular
+        if (tid == 0) lu_report(err, 4, f, j);
+        p = j;
+      }
+      if (tid == 0) ipiv[d.dof_off + j] = p;
+      if (i == p)
+#pragma unroll
+        for (int c = 0; c < kPanel; c++) prow[b][c] = row[c];
+      if (i == j && p != j)
+#pragma unroll
+        for (int c = 0; c < kPanel; c++) jrow[b][c] = row[c];
+      __syncthreads();
+      if (p != j) {
+        if (i == p)
+#pragma unroll
+          for (int c = 0; c < kPanel; c++) row[c] = jrow[b][c];
+        if (i == j)
+#pragma unroll
+          for (int c = 0; c < kPanel; c++) row[c] = prow[b][c];
+      }
+      if (i > j) {
+        const double djj = prow[b][jj];
+        const double l = row[jj] * (djj != 0.0 ? 1.0 / djj : 0.0);
+        row[jj] = l;
+#pragma unroll
+        for (int c = jj + 1; c < kPanel; c++) row[c] -= l * prow[b][c];
+      }
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < kPanel; c++)
+    if (live && c < kb) A[(int64_t)c * d.ld] = row[c];
+}
+
+// The same in global memory, for fronts with more rows.
 __global__ void __launch_bounds__(kLuPanelThreads) k_lu_panel(const int* __restrict__ flist,
                                                               const FrontDev* __restrict__ fr,
                                                               double* __restrict__ F,
@@ -204,13 +303,30 @@ __global__ void __launch_bounds__(128) k_lu_gemm(const int* __restrict__ flist,
   __shared__ double Xa[kLuTile * kLuS];   // Xa[i][t] = L(r0 + i, k + t)
   __shared__ double Xb[kLuTile * kLuS];   // Xb[j][t] = U(k + t, c0 + j)
   const int tid = threadIdx.x;
-  for (int idx = tid; idx < kLuTile * kPanel; idx += 128) {
-    const int i = idx % kLuTile, t = idx / kLuTile;
-    Xa[i * kLuS + t] = (t < kb && r0 + i < d.N) ? A[(r0 + i) + (int64_t)(k + t) * ld] : 0.0;
-  }
-  for (int idx = tid; idx < kLuTile * kPanel; idx += 128) {
-    const int t = idx % kPanel, j = idx / kPanel;
-    Xb[j * kLuS + t] = (t < kb && c0 + j < d.N) ? A[(k + t) + (int64_t)(c0 + j) * ld] : 0.0;
+  {   // all 32 loads of a thread in flight (clamped addresses, then a select)
+    double va[16], vb[16];
+    const int i = tid % kLuTile, t0 = tid / kLuTile;      // rows of L along the lanes
+    const int u = tid % kPanel, j0 = tid / kPanel;        // columns of U: rows k + u along the lanes
+#pragma unroll
+    for (int q = 0; q < 16; q++) {
+      const int t = t0 + 2 * q;
+      va[q] = A[t < kb && r0 + i < d.N ? (r0 + i) + (int64_t)(k + t) * ld : 0];
+    }
+#pragma unroll
+    for (int q = 0; q < 16; q++) {
+      const int j = j0 + 4 * q;
+      vb[q] = A[u < kb && c0 + j < d.N ? (k + u) + (int64_t)(c0 + j) * ld : 0];
+    }
+#pragma unroll
+    for (int q = 0; q < 16; q++) {
+      const int t = t0 + 2 * q;
+      Xa[i * kLuS + t] = t < kb && r0 + i < d.N ? va[q] : 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < 16; q++) {
+      const int j = j0 + 4 * q;
+      Xb[j * kLuS + u] = u < kb && c0 + j < d.N ? vb[q] : 0.0;
+    }
   }
   __syncthreads();
   const int lane = tid & 31, warp = tid >> 5, wi = warp >> 1, wj = warp & 1;
@@ -232,16 +348,28 @@ __global__ void __launch_bounds__(128) k_lu_gemm(const int* __restrict__ flist,
 #pragma unroll
       for (int b = 0; b < 4; b++) lu_dmma(acc[a][b][0], acc[a][b][1], fa[a], fb[b]);
   }
+  // C: all loads, then all stores
+  double cur[4][4][2];
 #pragma unroll
   for (int b = 0; b < 4; b++)
 #pragma unroll
     for (int q = 0; q < 2; q++) {
       const int c = c0 + wj * 32 + 8 * b + 2 * cc + q;
-      if (c >= d.N) continue;
 #pragma unroll
       for (int a = 0; a < 4; a++) {
         const int r = r0 + wi * 32 + 8 * a + rr;
-        if (r < d.N) A[r + (int64_t)c * ld] -= acc[a][b][q];
+        cur[a][b][q] = A[r < d.N && c < d.N ? r + (int64_t)c * ld : 0];
+      }
+    }
+#pragma unroll
+  for (int b = 0; b < 4; b++)
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      const int c = c0 + wj * 32 + 8 * b + 2 * cc + q;
+#pragma unroll
+      for (int a = 0; a < 4; a++) {
+        const int r = r0 + wi * 32 + 8 * a + rr;
+        if (r < d.N && c < d.N) A[r + (int64_t)c * ld] = cur[a][b][q] - acc[a][b][q];
       }
     }
 }
@@ -251,7 +379,10 @@ __global__ void __launch_bounds__(128) k_lu_gemm(const int* __restrict__ flist,
 void launch_lu_step(const int* flist, int nf, int maxN, const FrontDev* fr, double* F, int* ipiv,
                     int k, DevError* err, cudaStream_t st, int phase) {
   if (nf <= 0) return;
-  if (phase == 0) {
+  if (phase == 0 && maxN - k <= kLuPanelRows) {
+    const int threads = ((maxN - k + 31) / 32) * 32;
+    k_lu_panel_rows<<<nf, threads, 0, st>>>(flist, fr, F, ipiv, k, err);
+  } else if (phase == 0) {
     k_lu_panel<<<nf, kLuPanelThreads, 0, st>>>(flist, fr, F, ipiv, k, err);
   } else if (phase == 1) {
     const int gx = (maxN + kLuSwapThreads - 1) / kLuSwapThreads;
