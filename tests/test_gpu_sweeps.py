@@ -34,6 +34,21 @@ def test_solve_matches_a_sparse_direct_solve(N, nrhs, precision, tol):
         assert rel(x[:, c], ref[:, c]) < tol
 
 
+@pytest.mark.parametrize("N", [(31, 33), (77, 39), (130, 70), (28, 21, 23), (31, 31, 31)])
+@pytest.mark.parametrize("nrhs", [1, 3, 8, 9, 16, 19])
+@pytest.mark.parametrize("precision,tol", [(MFGPU_FP64, 1e-11), (MFGPU_MIXED, 1e-8)])
+def test_flag_ordered_sweeps_match_a_sparse_direct_solve(monkeypatch, N, nrhs, precision, tol):
+    """The flag-ordered sweeps on every level with a front of 48 or more rows:
+    block edges at 64, pivot and boundary rows in one block, fronts of one block."""
+    monkeypatch.setenv("MFGPU_SOLVE_COOP_MIN_N", "48")
+    _, A, b = problem(len(N), N, seed=8, nrhs=nrhs)
+    F = (MF2D if len(N) == 2 else MF3D)(A, *N, 1, 4, precision=precision)
+    F.Factor()
+    x, ref = F.Solve(b.T), _solve(A, b.T)
+    for c in range(nrhs):
+        assert rel(x[:, c], ref[:, c]) < tol
+
+
 @pytest.mark.parametrize("N,width", [((31, 33), 2), ((77, 39), 2), ((50, 41), 3), ((13, 11, 12), 2)])
 @pytest.mark.parametrize("nrhs", [1, 3, 6, 16])
 def test_lu_solve_matches_a_sparse_direct_solve(N, width, nrhs):

@@ -465,19 +465,316 @@ __global__ void __launch_bounds__(SCT) k_solve_flow_bwd(const int* __restrict__ 
   }
 }
 
+// ---------------------------------------------------------------------------
+// The same sweeps in FP64 on the FP64 tensor cores (mma.sync m8n8k4), eight
+// right-hand sides a product, up to NT = 2 products.  Warp w owns rows (columns,
+// backward) 8 w .. 8 w + 7 of the task's 64; its operand fragments of L come
+// straight from global memory (forward four columns of 64 bytes, backward eight
+// columns of 64 bytes a load), so an element of L is loaded once for all
+// right-hand sides, and a lane's state is two values per product instead of a
+// sum per right-hand side: 16 right-hand sides fit the registers of two CTAs an
+// SM where the scalar form spilled with one.  Bound: HBM for many blocks, the
+// chain of blocks (flag, 64 x 64 product, inverse product) for one front.
+// Against the scalar form: 3D 63^3, 16 right-hand sides, forward 6.05 -> 1.64
+// ms, backward 7.65 -> 1.78 ms; 2D 1023^2, 4, 428 -> 192 and 420 -> 228 us; 3D 79
+// x 63 x 50, one, 1287 -> 992 and 1181 -> 954 us.
+// ---------------------------------------------------------------------------
+constexpr int MS = 12;           // right-hand-side stride in shared memory per 8 (no bank conflicts)
+
+__device__ __forceinline__ void mma884(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
+}
+
+// c[t] += A x for 64 columns: a[s] is the lane's fragment of columns 4 s .. + 3,
+// x(k, rhs) at xs[k * MS * NT + rhs] (rhs 8 t + ..: 12 t + ..).  Two chains.
+template <int NT>
+__device__ __forceinline__ void mma_block(double (&c)[NT][2][2], const double (&a)[16],
+                                          const double* xs, int rr, int cc) {
+#pragma unroll
+  for (int s = 0; s < 16; s++)
+#pragma unroll
+    for (int t = 0; t < NT; t++)
+      mma884(c[t][s & 1], a[s], xs[(4 * s + cc) * (MS * NT) + MS * t + rr]);
+}
+
+// x(k, rhs) of 64 rows into shared memory, zero outside [0, nr) x [0, nrhs).
+template <int NT, class Get>
+__device__ __forceinline__ void stage_rhs(double* xs, int nr, int nrhs, Get&& get) {
+  for (int idx = threadIdx.x; idx < SB * 8 * NT; idx += SCT) {
+    const int r = idx & (SB - 1), c = idx / SB;
+    xs[r * (MS * NT) + MS * (c >> 3) + (c & 7)] = r < nr && c < nrhs ? get(r, c) : 0.0;
+  }
+}
+
+template <int NT>
+__global__ void __launch_bounds__(SCT, 2)
+    k_flow_fwd64(const int* __restrict__ flist, const FrontDev* __restrict__ fr,
+                 const double* __restrict__ F, const int* __restrict__ dofs, double* X, int64_t ldx,
+                 int nrhs, double* Wb, const int64_t* __restrict__ woff,
+                 const double* __restrict__ Dv, const int64_t* __restrict__ dinv_off,
+                 const int2* __restrict__ tasks, int ntasks, const int* __restrict__ flagoff,
+                 int* flags, DevError* err) {
+  __shared__ double xs[2][SB * MS * NT];
+  const int tid = threadIdx.x, lane = tid & 31, w8 = 8 * (tid >> 5), rr = lane >> 2, cc = lane & 3;
+  for (int t = blockIdx.x; t < ntasks; t += gridDim.x) {
+    const int2 tk = tasks[t];
+    const int i = tk.x, R = tk.y, f = flist[i];
+    const FrontDev d = fr[f];
+    double* W = Wb + woff[f] * nrhs;
+    double* Y = W + (int64_t)d.N * nrhs;
+    const int* dl = dofs + d.dof_off;
+    const int* fl = flags + flagoff[i];
+    const int nb = cdiv(d.n, SB);
+    const bool piv = R < nb;
+    const int row0 = piv ? R * SB : d.n + (R - nb) * SB;
+    const int rows = min(SB, (piv ? d.n : d.N) - row0);
+    const int jmax = piv ? R : nb;
+    const bool live = w8 + rr < rows;
+    // this lane's row, first column cc (dead rows read the block's first row)
+    const double* Ar = F + d.off + row0 + (live ? w8 + rr : 0) + (int64_t)min(cc, d.N - 1) * d.ld;
+    double acc[NT][2][2];
+#pragma unroll
+    for (int q = 0; q < NT; q++) acc[q][0][0] = acc[q][0][1] = acc[q][1][0] = acc[q][1][1] = 0.0;
+    auto load = [&](double (&a)[16], int j) {   // L(row, block j)
+      const int c0 = j * SB + cc;
+#pragma unroll
+      for (int s = 0; s < 16; s++)
+        a[s] = Ar[c0 + 4 * s < d.n ? (int64_t)(j * SB + 4 * s) * d.ld : 0];
+      if (j * SB + SB > d.n)
+#pragma unroll
+        for (int s = 0; s < 16; s++)
+          if (c0 + 4 * s >= d.n) a[s] = 0.0;
+    };
+    auto solved = [&](int j) {
+      return [&, j](int r, int c) {
+        return j * SB + r < d.n ? ldcg(Y + j * SB + r + (int64_t)c * d.N) : 0.0;
+      };
+    };
+    double a[16], an[16];
+    if (jmax > 0) load(a, 0);
+    for (int j = 0; j < jmax - 1; j++) {
+      if (tid == 0) flow_wait(fl + j, err);
+      __syncthreads();
+      stage_rhs<NT>(xs[j & 1], SB, nrhs, solved(j));
+      load(an, j + 1);                          // the next block in flight
+      __syncthreads();
+      mma_block<NT>(acc, a, xs[j & 1], rr, cc);
+#pragma unroll
+      for (int s = 0; s < 16; s++) a[s] = an[s];
+    }
+    // before the last wait: the inverse (in `an`) and the right-hand side
+    double b[NT][2];
+    if (piv) {
+      const double* D = Dv + dinv_off[f] + (int64_t)R * 2 * SB * SB + w8 + rr + cc * SB;
+#pragma unroll
+      for (int s = 0; s < 16; s++) an[s] = D[4 * s * SB];
+#pragma unroll
+      for (int q = 0; q < NT; q++)
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+          const int c = 8 * q + 2 * cc + e;
+          b[q][e] = live && c < nrhs ? X[dl[row0 + w8 + rr] + (int64_t)c * ldx] : 0.0;
+        }
+    }
+    if (jmax > 0) {
+      const int j = jmax - 1;
+      if (tid == 0) flow_wait(fl + j, err);
+      __syncthreads();
+      stage_rhs<NT>(xs[j & 1], SB, nrhs, solved(j));
+      __syncthreads();
+      mma_block<NT>(acc, a, xs[j & 1], rr, cc);
+    }
+    if (!piv) {
+#pragma unroll
+      for (int q = 0; q < NT; q++)
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+          const int c = 8 * q + 2 * cc + e;
+          if (live && c < nrhs)
+            W[row0 + w8 + rr + (int64_t)c * d.N] = -(acc[q][0][e] + acc[q][1][e]);
+        }
+      __syncthreads();                          // xs is free for the next task
+      continue;
+    }
+    // y_R = Dinv_R (b_R - acc)
+    double* ws = xs[jmax & 1];
+#pragma unroll
+    for (int q = 0; q < NT; q++)
+#pragma unroll
+      for (int e = 0; e < 2; e++)
+        ws[(w8 + rr) * (MS * NT) + MS * q + 2 * cc + e] =
+            live ? b[q][e] - (acc[q][0][e] + acc[q][1][e]) : 0.0;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < NT; q++) acc[q][0][0] = acc[q][0][1] = acc[q][1][0] = acc[q][1][1] = 0.0;
+    mma_block<NT>(acc, an, ws, rr, cc);
+#pragma unroll
+    for (int q = 0; q < NT; q++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const int c = 8 * q + 2 * cc + e;
+        const double y = acc[q][0][e] + acc[q][1][e];
+        if (live && c < nrhs) {
+          Y[row0 + w8 + rr + (int64_t)c * d.N] = y;
+          X[dl[row0 + w8 + rr] + (int64_t)c * ldx] = y;
+        }
+      }
+    __syncthreads();
+    if (tid == 0) flow_publish(flags + flagoff[i] + R);
+  }
+}
+
+// Backward: row blocks of 64 from row 0, so that a fragment takes two rows a
+// load (rows 8 s + 2 cc and + 1 of columns rr; the products take them as two
+// steps of four rows 8 s + {0, 2, 4, 6} and {1, 3, 5, 7}).  Blocks from the last
+// one up: boundary rows from X, pivot rows from Y as their flags come up; the
+// block holding the last pivots may hold both.
+template <int NT>
+__global__ void __launch_bounds__(SCT, 2)
+    k_flow_bwd64(const int* __restrict__ flist, const FrontDev* __restrict__ fr,
+                 const double* __restrict__ F, const int* __restrict__ dofs, double* X, int64_t ldx,
+                 int nrhs, double* Wb, const int64_t* __restrict__ woff,
+                 const double* __restrict__ Dv, const int64_t* __restrict__ dinv_off,
+                 const int2* __restrict__ tasks, int ntasks, const int* __restrict__ flagoff,
+                 int* flags, DevError* err) {
+  __shared__ double xs[2][SB * MS * NT];
+  const int tid = threadIdx.x, lane = tid & 31, w8 = 8 * (tid >> 5), rr = lane >> 2, cc = lane & 3;
+  for (int t = blockIdx.x; t < ntasks; t += gridDim.x) {
+    const int2 tk = tasks[t];
+    const int i = tk.x, j = tk.y, f = flist[i];
+    const FrontDev d = fr[f];
+    double* Y = Wb + woff[f] * nrhs + (int64_t)d.N * nrhs;
+    const int* dl = dofs + d.dof_off;
+    const int* fl = flags + flagoff[i];
+    const int nb = cdiv(d.n, SB), nbr = cdiv(d.N, SB), col0 = j * SB, kbj = min(SB, d.n - col0);
+    const bool live = w8 + rr < kbj;
+    const double* Lc = F + d.off + (int64_t)(col0 + (live ? w8 + rr : 0)) * d.ld + 2 * cc;
+    double acc[NT][2][2];
+#pragma unroll
+    for (int q = 0; q < NT; q++) acc[q][0][0] = acc[q][0][1] = acc[q][1][0] = acc[q][1][1] = 0.0;
+    // rows of block R this task takes: below its pivots, inside the front
+    auto load = [&](double (&a)[16], int R) {
+      const int r0 = R * SB, lo = R == j ? d.n : r0;
+      if (lo == r0 && r0 + SB <= d.N) {
+#pragma unroll
+        for (int s = 0; s < 8; s++) {
+          const double2 v = *reinterpret_cast<const double2*>(Lc + r0 + 8 * s);
+          a[2 * s] = v.x;
+          a[2 * s + 1] = v.y;
+        }
+      } else {
+#pragma unroll
+        for (int s = 0; s < 8; s++)
+#pragma unroll
+          for (int e = 0; e < 2; e++) {
+            const int r = r0 + 8 * s + 2 * cc + e;
+            a[2 * s + e] = r >= lo && r < d.N ? Lc[r0 + 8 * s + e] : 0.0;
+          }
+      }
+    };
+    auto stage = [&](double* x, int R) {        // x(row, rhs) in the fragments' row order
+      const int r0 = R * SB, lo = R == j ? d.n : r0;
+      for (int idx = tid; idx < SB * 8 * NT; idx += SCT) {
+        const int r = idx & (SB - 1), c = idx / SB, g = r0 + r;
+        double v = 0.0;
+        if (g >= lo && g < d.N && c < nrhs)
+          v = g < d.n ? ldcg(Y + g + (int64_t)c * d.N) : X[dl[g] + (int64_t)c * ldx];
+        const int k = (r & ~7) + 4 * (r & 1) + ((r & 7) >> 1);
+        x[k * (MS * NT) + MS * (c >> 3) + (c & 7)] = v;
+      }
+    };
+    // last block this task reads last: the one after it, or its own boundary rows
+    const int Rlast = (d.n & (SB - 1)) && j == nb - 1 && d.N > d.n ? j : j + 1;
+    double a[16], an[16];
+    if (Rlast < nbr) load(a, nbr - 1);
+    for (int R = nbr - 1; R > Rlast; R--) {
+      if (R < nb) {
+        if (tid == 0) flow_wait(fl + R, err);
+        __syncthreads();
+      }
+      stage(xs[R & 1], R);
+      load(an, R - 1);
+      __syncthreads();
+      mma_block<NT>(acc, a, xs[R & 1], rr, cc);
+#pragma unroll
+      for (int s = 0; s < 16; s++) a[s] = an[s];
+    }
+    // before the last wait: the inverse's transpose (in `an`) and y_j
+    const double* D = Dv + dinv_off[f] + (int64_t)j * 2 * SB * SB + SB * SB + w8 + rr + cc * SB;
+#pragma unroll
+    for (int s = 0; s < 16; s++) an[s] = D[4 * s * SB];
+    double b[NT][2];
+#pragma unroll
+    for (int q = 0; q < NT; q++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const int c = 8 * q + 2 * cc + e;
+        b[q][e] = live && c < nrhs ? X[dl[col0 + w8 + rr] + (int64_t)c * ldx] : 0.0;
+      }
+    if (Rlast < nbr) {
+      if (Rlast < nb && Rlast > j) {
+        if (tid == 0) flow_wait(fl + Rlast, err);
+        __syncthreads();
+      }
+      stage(xs[Rlast & 1], Rlast);
+      __syncthreads();
+      mma_block<NT>(acc, a, xs[Rlast & 1], rr, cc);
+    }
+    // x_j = Dinv_j^T (y_j - acc)
+    double* ws = xs[(Rlast + 1) & 1];
+#pragma unroll
+    for (int q = 0; q < NT; q++)
+#pragma unroll
+      for (int e = 0; e < 2; e++)
+        ws[(w8 + rr) * (MS * NT) + MS * q + 2 * cc + e] =
+            live ? b[q][e] - (acc[q][0][e] + acc[q][1][e]) : 0.0;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < NT; q++) acc[q][0][0] = acc[q][0][1] = acc[q][1][0] = acc[q][1][1] = 0.0;
+    mma_block<NT>(acc, an, ws, rr, cc);
+#pragma unroll
+    for (int q = 0; q < NT; q++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const int c = 8 * q + 2 * cc + e;
+        const double x = acc[q][0][e] + acc[q][1][e];
+        if (live && c < nrhs) {
+          Y[col0 + w8 + rr + (int64_t)c * d.N] = x;
+          X[dl[col0 + w8 + rr] + (int64_t)c * ldx] = x;
+        }
+      }
+    __syncthreads();
+    if (tid == 0) flow_publish(flags + flagoff[i] + j);
+  }
+}
+
 // Persistent grid: every CTA the SMs hold at once (a cooperative launch checks
 // that they are all resident, which the flag waits rely on).  As many CTAs as
 // fit, so that the row blocks of a long chain (a root front has hundreds) each
 // get their own CTA from the start and accumulate the solved blocks as they
 // come, instead of queueing behind other tasks of the same CTA.
-template <class K>
-int flowGrid(K kern) {
+int flowGrid(const void* kern) {
   int dev = 0, sms = 0, per = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, SCT, 0);
   return sms * std::max(1, per);
 }
+
+// Kernels of a direction and bound of the right-hand-side count: the scalar
+// form in FP32, the tensor-core form in FP64.
+template <class T, int NR>
+struct FlowKernels {
+  static const void* fwd() { return (const void*)k_solve_flow_fwd<T, NR>; }
+  static const void* bwd() { return (const void*)k_solve_flow_bwd<T, NR>; }
+};
+template <int NR>
+struct FlowKernels<double, NR> {
+  static const void* fwd() { return (const void*)k_flow_fwd64<NR / 8>; }
+  static const void* bwd() { return (const void*)k_flow_bwd64<NR / 8>; }
+};
 
 template <class T, int NR>
 cudaError_t launchFlowSolve(bool fwd, const int* flist, const FrontDev* fr, const T* F,
@@ -487,19 +784,16 @@ cudaError_t launchFlowSolve(bool fwd, const int* flist, const FrontDev* fr, cons
                             int nflags, DevError* err, cudaStream_t st) {
   cudaError_t me = cudaMemsetAsync(flags, 0, sizeof(int) * (size_t)std::max(1, nflags), st);
   if (me != cudaSuccess) return me;
-  static const int gf = flowGrid(k_solve_flow_fwd<T, NR>);   // thread-safe one-time set-up
-  static const int gb = flowGrid(k_solve_flow_bwd<T, NR>);
+  using K = FlowKernels<T, NR>;
+  static const int gf = flowGrid(K::fwd());   // thread-safe one-time set-up
+  static const int gb = flowGrid(K::bwd());
   const int grid = std::max(1, std::min(fwd ? gf : gb, ntasks));
   void* args[] = {(void*)&flist, (void*)&fr,    (void*)&F,      (void*)&dofs,    (void*)&X,
                   (void*)&ldx,   (void*)&nrhs,  (void*)&W,      (void*)&woff,    (void*)&Dv,
                   (void*)&dinv_off, (void*)&tasks, (void*)&ntasks, (void*)&flagoff, (void*)&flags,
                   (void*)&err};
   g_launches++;
-  if (fwd)
-    return cudaLaunchCooperativeKernel((const void*)k_solve_flow_fwd<T, NR>, dim3(grid), dim3(SCT),
-                                       args, 0, st);
-  return cudaLaunchCooperativeKernel((const void*)k_solve_flow_bwd<T, NR>, dim3(grid), dim3(SCT),
-                                     args, 0, st);
+  return cudaLaunchCooperativeKernel(fwd ? K::fwd() : K::bwd(), dim3(grid), dim3(SCT), args, 0, st);
 }
 
 }  // namespace
@@ -541,8 +835,10 @@ cudaError_t launch_solve_flow(bool forward, const int* flist, const FrontDev* fr
 #define MFGPU_FLOW(NRV)                                                                           \
   return launchFlowSolve<T, NRV>(forward, flist, fr, F, dofs, X, ldx, nrhs, W, woff, Dv, dinv_off, \
                                  tk, ntasks, flagoff, flags, nflags, err, st)
-  if (nrhs == 1) MFGPU_FLOW(1);
-  if (nrhs <= 4) MFGPU_FLOW(4);
+  if constexpr (sizeof(T) == sizeof(float)) {
+    if (nrhs == 1) MFGPU_FLOW(1);
+    if (nrhs <= 4) MFGPU_FLOW(4);
+  }
   if (nrhs <= 8) MFGPU_FLOW(8);
   MFGPU_FLOW(16);
 #undef MFGPU_FLOW
