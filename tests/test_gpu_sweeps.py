@@ -49,6 +49,29 @@ def test_flag_ordered_sweeps_match_a_sparse_direct_solve(monkeypatch, N, nrhs, p
         assert rel(x[:, c], ref[:, c]) < tol
 
 
+@pytest.mark.parametrize("nrhs", [1, 5, 16])
+@pytest.mark.parametrize("precision,tol", [(MFGPU_FP64, 1e-11), (MFGPU_MIXED, 1e-8)])
+def test_large_fronts_of_a_level_of_many(monkeypatch, tmp_path, nrhs, precision, tol):
+    """A leaf level of 1024 fronts whose last ones are several times larger: those
+    go to the flag-ordered sweeps.  A factor saved under another split of the
+    level loads and solves as well."""
+    N = (270, 150)
+    monkeypatch.setenv("MFGPU_SOLVE_COOP_MIN_N", "120")
+    _, A, b = problem(2, N, seed=9, nrhs=nrhs)
+    F = MF2D(A, *N, 1, 4, precision=precision)
+    F.Factor()
+    x, ref = F.Solve(b.T), _solve(A, b.T)
+    for c in range(nrhs):
+        assert rel(x[:, c], ref[:, c]) < tol
+    F.save(tmp_path / "f")
+    monkeypatch.setenv("MFGPU_SOLVE_COOP_MIN_N", "200")
+    G = MF2D(A, *N, 1, 4, precision=precision)
+    G.load(tmp_path / "f")
+    y = G.Solve(b.T)
+    for c in range(nrhs):
+        assert rel(y[:, c], ref[:, c]) < tol
+
+
 @pytest.mark.parametrize("N,width", [((31, 33), 2), ((77, 39), 2), ((50, 41), 3), ((13, 11, 12), 2)])
 @pytest.mark.parametrize("nrhs", [1, 3, 6, 16])
 def test_lu_solve_matches_a_sparse_direct_solve(N, width, nrhs):

@@ -374,9 +374,13 @@ struct mfgpu_handle {
   unsigned* d_gbar = nullptr;  // grid-barrier arrival counter of the cooperative kernels
   // Cooperative (flag-ordered) sweeps: per level, its forward / backward task
   // lists and flag offsets in d_flow; the ready flags of one launch in d_flags.
+  // In a level of more fronts than one flow launch takes, its large fronts
+  // (`list`, in d_flow) go there and the others (`rest`) to the per-front sweeps.
   struct FlowLevel {
     int64_t fwd = 0, bwd = 0, flagoff = 0;
     int nfwd = 0, nbwd = 0, nflags = 0;
+    int64_t list = -1, rest = -1;   // -1: every front of the level
+    int nrest = 0, restMaxN = 0;
   };
   std::vector<FlowLevel> flow;
   int* d_flow = nullptr;       // shared with serving-loop views
@@ -915,7 +919,7 @@ struct mfgpu_handle {
       runPanel<T>(P, L);
     }
     const bool tiles = kind == LK_COOP || (kind == LK_TC && subpanel);
-    if (!tiles && L.nf > 0 && coopSweep(ell)) {
+    if (!tiles && L.nf > 0 && hasFlow(ell)) {
       mfgpu::launch_diag_inv<T>(P.d_ids + L.f0, (int)L.nf, L.maxn, d_fr, F, (T*)d_Dinv, d_dinv_off,
                                 stream);
       ck(cudaGetLastError(), "launch diagonal-block inverses (k_diag_inv)");
@@ -1028,6 +1032,23 @@ struct mfgpu_handle {
   template <class T>
   void finishLevel(const Plan& P, const Plan::Level& L) {
     runGroup<T>(P, L.sadd, groupBytes(P, L.sadd));
+  }
+
+  // The flag-ordered sweeps' block inverses of every front that has some, from
+  // the factor in place.
+  void formBlockInverses() {
+    for (int ell = 0; ell < S->levels; ell++) {
+      if (!hasFlow(ell)) continue;
+      const int* fl = d_all + S->lv[ell].front0;
+      if (mixed)
+        mfgpu::launch_diag_inv<float>(fl, S->lv[ell].nbox, lvMaxn[ell], d_fr, (const float*)d_F,
+                                      (float*)d_Dinv, d_dinv_off, stream);
+      else
+        mfgpu::launch_diag_inv<double>(fl, S->lv[ell].nbox, lvMaxn[ell], d_fr, (const double*)d_F,
+                                       (double*)d_Dinv, d_dinv_off, stream);
+      ck(cudaGetLastError(), "launch diagonal-block inverses (k_diag_inv)");
+    }
+    ck(cudaStreamSynchronize(stream), "block inverses");
   }
 
   // Full factorization that also picks each level's kernel by timing: per
@@ -1339,33 +1360,58 @@ struct mfgpu_handle {
     return solveCoopMinN > 0 && lvMaxN[ell] >= solveCoopMinN &&
            S->lv[ell].nbox <= mfgpu::solve_coop_max_fronts();
   }
+  // The large fronts of a level too numerous for coopSweep (ragged grids leave
+  // their remainder to the last boxes, so leaf levels of thousands of small
+  // fronts hold a few large ones); empty when they are too many as well.
+  // One CTA's sweep of such a front holds up the level: 2D 700 x 333 mixed (4096
+  // leaves, one of 1348 x 1260), factor + solve 6.38 -> 5.66 ms.
+  std::vector<int> largeFronts(int ell) const {
+    std::vector<int> big;
+    if (solveCoopMinN <= 0 || lvMaxN[ell] < solveCoopMinN || coopSweep(ell) ||
+        S->lv[ell].nbox > 32768)   // (a launch of k_diag_inv covers a level's fronts)
+      return big;
+    for (int b = 0; b < S->lv[ell].nbox; b++)
+      if (S->fronts[S->lv[ell].front0 + b].N >= solveCoopMinN) big.push_back(S->lv[ell].front0 + b);
+    if ((int)big.size() > mfgpu::solve_coop_max_fronts()) big.clear();
+    return big;
+  }
+  bool hasFlow(int ell) const { return ell < (int)flow.size() && flow[ell].nfwd > 0; }
 
   template <class T>
   void sweepLevel(bool forward, int ell, T* X, int64_t ldx, int nrhs, T* W) {
     const Schedule& s = *S;
     const T* F = (const T*)d_F;
     const int* fl = d_all + s.lv[ell].front0;
-    const int nf = s.lv[ell].nbox;
+    int nf = s.lv[ell].nbox;
     if (lu) {
       if (sizeof(T) != sizeof(double)) throw CudaError("LU fronts are FP64 only", MFGPU_ERR_ARG);
       mfgpu::launch_lu_solve(forward, fl, nf, lvMaxN[ell], d_fr, (const double*)F, d_ipiv, d_dofs,
                              (double*)X, ldx, nrhs, (double*)W, d_woff, stream);
       ck(cudaGetLastError(), forward ? "launch LU forward sweep (k_lu_solve_fwd)"
                                      : "launch LU backward sweep (k_lu_solve_bwd)");
-    } else if (coopSweep(ell)) {
+      return;
+    }
+    int maxN = lvMaxN[ell];
+    if (hasFlow(ell)) {
       const FlowLevel& q = flow[ell];
-      ck(mfgpu::launch_solve_flow<T>(forward, fl, d_fr, F, d_dofs, X, ldx, nrhs, W, d_woff,
+      const int* big = q.list < 0 ? fl : d_flow + q.list;
+      ck(mfgpu::launch_solve_flow<T>(forward, big, d_fr, F, d_dofs, X, ldx, nrhs, W, d_woff,
                                      (const T*)d_Dinv, d_dinv_off,
                                      d_flow + (forward ? q.fwd : q.bwd), forward ? q.nfwd : q.nbwd,
                                      d_flow + q.flagoff, d_flags, q.nflags, d_err, stream),
          forward ? "launch cooperative forward sweep (k_solve_flow_fwd)"
                  : "launch cooperative backward sweep (k_solve_flow_bwd)");
-    } else if (forward) {
-      mfgpu::launch_solve_fwd<T>(fl, nf, lvMaxN[ell], d_fr, F, d_dofs, X, ldx, nrhs, W, d_woff,
+      if (q.list < 0) return;
+      fl = d_flow + q.rest;
+      nf = q.nrest;
+      maxN = q.restMaxN;
+    }
+    if (forward) {
+      mfgpu::launch_solve_fwd<T>(fl, nf, maxN, d_fr, F, d_dofs, X, ldx, nrhs, W, d_woff,
                                  stream);
       ck(cudaGetLastError(), "launch forward sweep (k_solve_fwd)");
     } else {
-      mfgpu::launch_solve_bwd<T>(fl, nf, lvMaxN[ell], d_fr, F, d_dofs, X, ldx, nrhs, W, d_woff,
+      mfgpu::launch_solve_bwd<T>(fl, nf, maxN, d_fr, F, d_dofs, X, ldx, nrhs, W, d_woff,
                                  stream);
       ck(cudaGetLastError(), "launch backward sweep (k_solve_bwd)");
     }
@@ -1839,8 +1885,16 @@ int createFrom(std::unique_ptr<Schedule> sched, int n, const int* row_ptr, const
       std::vector<int64_t> doff(s.fronts.size(), -1);
       int64_t cur = 0;
       const int B = mfgpu::kDinvBlock;
+      std::vector<char> flowFront(s.fronts.size(), 0);
+      std::vector<std::vector<int>> big(s.levels);
+      for (int ell = 0; ell < s.levels; ell++) {
+        big[ell] = H.largeFronts(ell);
+        for (int f : big[ell]) flowFront[f] = 1;
+        for (int b = 0; b < s.lv[ell].nbox && H.coopSweep(ell); b++)
+          flowFront[s.lv[ell].front0 + b] = 1;
+      }
       for (size_t i = 0; i < s.fronts.size(); i++)
-        if (H.coopSweep(s.fronts[i].level)) {
+        if (flowFront[i]) {
           doff[i] = cur;
           cur += (int64_t)((s.fronts[i].n + B - 1) / B) * 2 * B * B;
         }
@@ -1851,14 +1905,28 @@ int createFrom(std::unique_ptr<Schedule> sched, int n, const int* row_ptr, const
       std::vector<int> tab;
       H.flow.assign(s.levels, mfgpu_handle::FlowLevel());
       for (int ell = 0; ell < s.levels; ell++) {
-        if (!H.coopSweep(ell)) continue;
-        std::vector<int> nn, NN, fw, bw, fo;
+        if (!H.coopSweep(ell) && big[ell].empty()) continue;
+        std::vector<int> nn, NN, fw, bw, fo, rest;
+        mfgpu_handle::FlowLevel& q = H.flow[ell];
         for (int b = 0; b < s.lv[ell].nbox; b++) {
-          nn.push_back(s.fronts[s.lv[ell].front0 + b].n);
-          NN.push_back(s.fronts[s.lv[ell].front0 + b].N);
+          const int f = s.lv[ell].front0 + b;
+          if (flowFront[f]) {
+            nn.push_back(s.fronts[f].n);
+            NN.push_back(s.fronts[f].N);
+          } else {
+            rest.push_back(f);
+            q.restMaxN = std::max(q.restMaxN, s.fronts[f].N);
+          }
         }
         mfgpu::flow_tasks(nn, NN, fw, bw, fo);
-        mfgpu_handle::FlowLevel& q = H.flow[ell];
+        if (!big[ell].empty()) {
+          q.list = (int64_t)tab.size();
+          tab.insert(tab.end(), big[ell].begin(), big[ell].end());
+          q.rest = (int64_t)tab.size();
+          q.nrest = (int)rest.size();
+          tab.insert(tab.end(), rest.begin(), rest.end());
+          if (tab.size() % 2) tab.push_back(0);   // the pairs below are 8-byte aligned
+        }
         q.fwd = (int64_t)tab.size();
         q.nfwd = (int)fw.size() / 2;
         tab.insert(tab.end(), fw.begin(), fw.end());
@@ -2430,8 +2498,7 @@ int mfgpu_load(mfgpu_handle* h, const char* path) {
                        : hd.n != me.n || hd.nnz != me.nnz || hd.pattern != me.pattern
                            ? "matrix size or sparsity pattern"
                        : hd.front_elems != me.front_elems || hd.sep_elems != me.sep_elems ||
-                               hd.dinv_elems != me.dinv_elems || hd.nfronts != me.nfronts ||
-                               hd.nseps != me.nseps
+                               hd.nfronts != me.nfronts || hd.nseps != me.nseps
                            ? "elimination-tree schedule"
                            : nullptr;
     if (what)
@@ -2439,15 +2506,28 @@ int mfgpu_load(mfgpu_handle* h, const char* path) {
                       MFGPU_ERR_ARG);
     ck(cudaStreamSynchronize(h->stream), "sync before load");
     h->factored = false;
+    // block inverses saved for another set of fronts (other sweep thresholds,
+    // an earlier build) are read over and formed anew
+    const bool same = hd.dinv_elems == me.dinv_elems;
+    auto blocks = facBlocks(h);
+    if (!same) {
+      for (size_t i = 0; i < blocks.size();)
+        if (blocks[i].first == h->d_Dinv) blocks.erase(blocks.begin() + i);
+        else i++;
+      if (hd.dinv_elems > 0)
+        blocks.insert(h->lu ? blocks.end() - 1 : blocks.end(),
+                      {nullptr, (size_t)hd.dinv_elems * h->esz});
+    }
     std::vector<unsigned char> buf;
     uint64_t sum = kFnvBasis;
-    for (const auto& blk : facBlocks(h)) {
+    for (const auto& blk : blocks) {
       for (size_t o = 0; o < blk.second; o += kFacChunk) {
         const size_t len = std::min(kFacChunk, blk.second - o);
         buf.resize(len);
         if (fread(buf.data(), 1, len, f.get()) != len)
           throw CudaError(std::string("factor file ") + path + " is truncated", MFGPU_ERR_ARG);
         sum = fnv64(sum, buf.data(), len);
+        if (!blk.first) continue;
         ck(cudaMemcpy((unsigned char*)blk.first + o, buf.data(), len, cudaMemcpyHostToDevice),
            "copy factor to device");
       }
@@ -2455,6 +2535,7 @@ int mfgpu_load(mfgpu_handle* h, const char* path) {
     uint64_t want = 0;
     if (fread(&want, sizeof want, 1, f.get()) != 1 || want != sum)
       throw CudaError(std::string("factor file ") + path + " fails its checksum", MFGPU_ERR_ARG);
+    if (!same) h->formBlockInverses();
     h->stats = mfgpu_stats{};
     h->factored = true;
   });
