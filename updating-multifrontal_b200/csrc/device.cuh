@@ -105,10 +105,12 @@ constexpr int kPanel = 32;      // panel width of the partial Cholesky
 
 // Kernel launch wrappers.  T = double (FP64 path) or float (mixed path).
 
-// Assembly tasks: tstart has ntasks+1 exclusive prefix sums of tile counts.
-// `scale` (may be null) multiplies sparse entries a_rc by scale[r] * scale[c].
+// Assembly: a warp per tile, tiles[i] = (task, tile row | tile column << 16).
+// staged: some tile needs shared memory (a transposed copy, or a sparse tile of
+// a matrix with rows of more than eight entries).  `scale` (may be null)
+// multiplies sparse entries a_rc by scale[r] * scale[c].
 template <class T>
-void launch_tasks(const Task* tasks, const int64_t* tstart, int ntasks, int64_t ntiles, T* fronts,
+void launch_tasks(const Task* tasks, const int2* tiles, int64_t ntiles, bool staged, T* fronts,
                   T* seps, const int* rp, const int* ci, const double* va, const int* dofs,
                   const double* scale, cudaStream_t st);
 

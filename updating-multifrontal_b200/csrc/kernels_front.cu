@@ -33,64 +33,45 @@ namespace {
 // Assembly, one warp per 32 x 32 tile of a task, kTaskWarps tiles per CTA.
 // Bound: HBM writes (every element of the fronts) for the leaf levels, the
 // chain of dependent loads (tile -> task -> DOFs -> CSR rows) for small levels.
-// So the tile's task is found by all lanes probing at once (three or four
-// rounds of loads for 100,000 tasks, not seventeen), the rows of a tile are
-// spread over the lanes, and block moves keep kTaskUnroll columns in flight.
+// So a tile names its task and place (no search), the rows of a tile are spread
+// over the lanes, block moves keep kTaskUnroll columns in flight, and launches
+// without transposed copies take no shared memory (twice the warps an SM).
 // Sparse tiles: a lane holds its row's CSR entries (eight at a time) in
 // registers and matches them against the tile's columns, broadcast one by one,
-// so each column is written as it is found.  Against a serial search and a
-// pass over all rows with every lane reading the same entries: 2D 1023^2
-// leaves 2.20 -> 1.29 ms; with the fronts, separator bases and both
-// accumulations of a level in two launches instead of four, the assemblies of
-// a 2D 127^2 factorization and update 549 -> 189 us.
+// so each column is written as it is found.  Against a serial search through
+// tile prefixes, a pass over all rows with every lane reading the same entries,
+// and four launches a level: 2D 1023^2 leaves 2.20 -> 0.78 ms, a 2D 127^2 step's
+// assemblies 549 -> 184 us.
 constexpr int kTaskWarps = 4;
 constexpr int kTaskUnroll = 8;
 
-// Last t in [0, n) with start[t] <= x (start[0] <= x), by a whole warp.
-__device__ __forceinline__ int warp_upper(const int64_t* __restrict__ start, int n, int64_t x,
-                                          int lane) {
-  int lo = 0, len = n;   // the answer is in [lo, lo + len)
-  while (len > 1) {
-    const int step = (len + 31) / 32;
-    const int at = lo + lane * step;
-    const bool le = lane * step < len && start[at] <= x;
-    const int k = __popc(__ballot_sync(0xffffffffu, le)) - 1;   // probes up to lane k hold
-    lo += k * step;
-    len = min(step, len - k * step);
-  }
-  return lo;
-}
-
-template <class T>
+template <class T, bool STAGED>
 __global__ void __launch_bounds__(32 * kTaskWarps) k_tasks(const Task* __restrict__ tasks,
-                                                           const int64_t* __restrict__ tstart,
-                                                           int ntasks, int64_t ntiles,
-                                                           T* __restrict__ F, T* __restrict__ SA,
+                                                           const int2* __restrict__ tiles,
+                                                           int64_t ntiles, T* __restrict__ F,
+                                                           T* __restrict__ SA,
                                                            const int* __restrict__ rp,
                                                            const int* __restrict__ ci,
                                                            const double* __restrict__ va,
                                                            const int* __restrict__ dofs,
                                                            const double* __restrict__ scale) {
-  __shared__ T sm[kTaskWarps][kTaskTile][kTaskTile + 1];
+  __shared__ T sm[STAGED ? kTaskWarps : 1][STAGED ? kTaskTile : 1][kTaskTile + 1];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t tile = ((int64_t)blockIdx.x + (int64_t)blockIdx.y * gridDim.x) * kTaskWarps + w;
   if (tile >= ntiles) return;
-  const int t = warp_upper(tstart, ntasks, tile, lane);
+  const int2 at = tiles[tile];
+  const int t = at.x;
   const Task Tk = tasks[t];
-  const int local = (int)(tile - tstart[t]);
-  const int tr = (Tk.rows + kTaskTile - 1) / kTaskTile;
-  const int i0 = (local % tr) * kTaskTile;
-  const int j0 = (local / tr) * kTaskTile;
-  if (Tk.lower && i0 + kTaskTile - 1 < j0) return;
+  const int i0 = (at.y & 0xffff) * kTaskTile, j0 = (int)((unsigned)at.y >> 16) * kTaskTile;
   T* dst = (Tk.dst_arena == AR_FRONT ? F : SA) + Tk.dst_off;
   const T* src = (Tk.src_arena == AR_FRONT ? F : SA) + Tk.src_off;
   const int rows = min(kTaskTile, Tk.rows - i0), cols = min(kTaskTile, Tk.cols - j0);
-  T(*tb)[kTaskTile + 1] = sm[w];
+  T(*tb)[kTaskTile + 1] = sm[STAGED ? w : 0];
   const int i = i0 + lane;   // this lane's row of the tile in the column-major writes
   // first column this lane does not write (its row's diagonal in lower tiles)
   const int jend = lane >= rows ? 0 : Tk.lower ? min(cols, i - j0 + 1) : cols;
   T* d = dst + i + (int64_t)j0 * Tk.dst_ld;
-  if (Tk.kind == TK_COPY && Tk.trans) {
+  if (STAGED && Tk.kind == TK_COPY && Tk.trans) {
     // dst(i, j) = src[j + i*ld]: read src rows with lanes along j, write dst
     // columns with lanes along i, through the warp's shared-memory tile
     const T* sr = src + j0 + lane + (int64_t)i0 * Tk.src_ld;
@@ -117,7 +98,7 @@ __global__ void __launch_bounds__(32 * kTaskWarps) k_tasks(const Task* __restric
     const double sc = (scale && lane < cols) ? scale[cj] : 1.0;
     const double sr = (scale && lane < rows) ? scale[rl] : 1.0;
     const int p0 = lane < rows ? rp[rl] : 0, p1 = lane < rows ? rp[rl + 1] : 0;
-    const bool lng = __any_sync(0xffffffffu, p1 - p0 > 8);   // rows of wider stencils
+    const bool lng = STAGED && __any_sync(0xffffffffu, p1 - p0 > 8);   // rows of wider stencils
     if (lng)
       for (int jj = 0; jj < cols; jj++) tb[lane][jj] = T(0);
     for (int pb = p0;; pb += 8) {
@@ -145,7 +126,7 @@ __global__ void __launch_bounds__(32 * kTaskWarps) k_tasks(const Task* __restric
           d[(int64_t)jj * Tk.dst_ld] = (T)x;
         }
       }
-      if (!__any_sync(0xffffffffu, pb + 8 < p1)) break;
+      if (!lng || !__any_sync(0xffffffffu, pb + 8 < p1)) break;
     }
     if (lng)
       for (int jj = 0; jj < jend; jj++) d[(int64_t)jj * Tk.dst_ld] = tb[lane][jj];
@@ -1002,15 +983,20 @@ __global__ void __launch_bounds__(ST) k_lu_apply_up(const int* __restrict__ flis
 }  // namespace
 
 template <class T>
-void launch_tasks(const Task* tasks, const int64_t* tstart, int ntasks, int64_t ntiles, T* fronts,
+void launch_tasks(const Task* tasks, const int2* tiles, int64_t ntiles, bool staged, T* fronts,
                   T* seps, const int* rp, const int* ci, const double* va, const int* dofs,
                   const double* scale, cudaStream_t st) {
-  if (ntasks <= 0 || ntiles <= 0) return;
+  if (ntiles <= 0) return;
   const int64_t blocks = (ntiles + kTaskWarps - 1) / kTaskWarps;
   const int64_t gx = blocks < 65535 * 32 ? blocks : 65535 * 32;
   const int64_t gy = (blocks + gx - 1) / gx;
-  k_tasks<T><<<dim3((unsigned)gx, (unsigned)gy), 32 * kTaskWarps, 0, st>>>(
-      tasks, tstart, ntasks, ntiles, fronts, seps, rp, ci, va, dofs, scale);
+  const dim3 grid((unsigned)gx, (unsigned)gy);
+  if (staged)
+    k_tasks<T, true><<<grid, 32 * kTaskWarps, 0, st>>>(tasks, tiles, ntiles, fronts, seps, rp, ci,
+                                                       va, dofs, scale);
+  else
+    k_tasks<T, false><<<grid, 32 * kTaskWarps, 0, st>>>(tasks, tiles, ntiles, fronts, seps, rp, ci,
+                                                        va, dofs, scale);
   g_launches++;
 }
 
@@ -1190,7 +1176,7 @@ cudaError_t launch_trail_syrk(const int* flist, int nf, const FrontDev* fr, T* F
 }
 
 #define MFGPU_INSTANTIATE(T)                                                                      \
-  template void launch_tasks<T>(const Task*, const int64_t*, int, int64_t, T*, T*, const int*,     \
+  template void launch_tasks<T>(const Task*, const int2*, int64_t, bool, T*, T*, const int*,       \
                                 const int*, const double*, const int*, const double*, cudaStream_t); \
   template void launch_front_small<T>(const int*, int, int, const FrontDev*, T*, DevError*,        \
                                       cudaStream_t);                                                \

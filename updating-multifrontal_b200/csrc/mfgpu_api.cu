@@ -70,15 +70,10 @@ T* dalloc(size_t count, const char* what) {
   return static_cast<T*>(p);
 }
 
-int64_t tilesOf(const Task& t) {
-  const int64_t a = (t.rows + mfgpu::kTaskTile - 1) / mfgpu::kTaskTile;
-  const int64_t b = (t.cols + mfgpu::kTaskTile - 1) / mfgpu::kTaskTile;
-  return a * b;
-}
-
-// A group of tasks executed by one launch.
+// A group of tasks executed by one launch, a warp per tile.
 struct Group {
-  int64_t task0 = 0, ntasks = 0, pref0 = 0, ntiles = 0;
+  int64_t task0 = 0, ntasks = 0, tile0 = 0, ntiles = 0;
+  bool staged = false;   // some tile goes through shared memory
 };
 
 // Everything one factorization pass needs: per level the fronts and separators
@@ -107,7 +102,7 @@ struct Plan {
   std::vector<Level> lv;
   std::vector<int> real;    // batch plans: the schedule's front id of each entry of `ids`
   std::vector<Task> tasks;
-  std::vector<int64_t> pref;
+  std::vector<int2> tiles;  // (task of the group, tile row | tile column << 16)
   std::vector<int> ids;
   std::vector<int> cpref;
   std::vector<int> ttask, trow;   // tile tasks (pairs) and block-row offsets
@@ -117,33 +112,33 @@ struct Plan {
   double flops = 0;
   // device copies
   Task* d_tasks = nullptr;
-  int64_t* d_pref = nullptr;
+  int2* d_tiles = nullptr;
   int* d_ids = nullptr;
   int* d_cpref = nullptr;
   int* d_ttask = nullptr;
   int* d_trow = nullptr;
-  size_t cap_tasks = 0, cap_pref = 0, cap_ids = 0, cap_cpref = 0, cap_ttask = 0, cap_trow = 0;
+  size_t cap_tasks = 0, cap_tiles = 0, cap_ids = 0, cap_cpref = 0, cap_ttask = 0, cap_trow = 0;
 
   void release() {
     cudaFree(d_tasks);
-    cudaFree(d_pref);
+    cudaFree(d_tiles);
     cudaFree(d_ids);
     cudaFree(d_cpref);
     cudaFree(d_ttask);
     cudaFree(d_trow);
     d_tasks = nullptr;
-    d_pref = nullptr;
+    d_tiles = nullptr;
     d_ids = nullptr;
     d_cpref = nullptr;
     d_ttask = nullptr;
     d_trow = nullptr;
-    cap_tasks = cap_pref = cap_ids = cap_cpref = cap_ttask = cap_trow = 0;
+    cap_tasks = cap_tiles = cap_ids = cap_cpref = cap_ttask = cap_trow = 0;
   }
 
   void clear(int levels) {
     lv.assign(levels, Level());
     tasks.clear();
-    pref.clear();
+    tiles.clear();
     ids.clear();
     real.clear();
     cpref.clear();
@@ -191,31 +186,35 @@ struct Plan {
   // A group is built by beginGroup, appendGroup (the tasks of some owners,
   // optionally rewritten by fx), endGroup.  pairs: the owners' tasks come in
   // pairs that one tile executes together, so the second one has no tiles.
+  // wide: the matrix has rows of more than eight entries.
   Group beginGroup() {
     Group g;
     g.task0 = (int64_t)tasks.size();
-    g.pref0 = (int64_t)pref.size();
-    pref.push_back(0);
+    g.tile0 = (int64_t)tiles.size();
     return g;
   }
-  void appendGroup(const std::vector<Task>& src, const std::vector<int64_t>& ptr,
-                   const std::vector<int>& owners, bool pairs,
+  void appendGroup(Group& g, const std::vector<Task>& src, const std::vector<int64_t>& ptr,
+                   const std::vector<int>& owners, bool pairs, bool wide,
                    const std::function<void(Task&)>& fx = nullptr) {
-    int64_t acc = pref.back();
+    const int E = mfgpu::kTaskTile;
     for (int o : owners) {
       const int64_t a = pairs ? 2 * (int64_t)o : ptr[o], b = pairs ? a + 2 : ptr[o + 1];
       for (int64_t t = a; t < b; t++) {
-        tasks.push_back(src[t]);
+        const Task& T = src[t];
+        const int id = (int)((int64_t)tasks.size() - g.task0);
+        tasks.push_back(T);
         if (fx) fx(tasks.back());
-        if (!pairs || t == a) acc += tilesOf(src[t]);
-        pref.push_back(acc);
+        if (pairs && t != a) continue;
+        g.staged |= (T.kind == mfgpu::TK_COPY && T.trans) || (wide && T.kind == mfgpu::TK_SPARSE);
+        for (int j = 0; j * E < T.cols; j++)
+          for (int i = T.lower ? j : 0; i * E < T.rows; i++)   // (nothing above the diagonal)
+            tiles.push_back(make_int2(id, i | (j << 16)));
       }
     }
   }
   void endGroup(Group& g) {
     g.ntasks = (int64_t)tasks.size() - g.task0;
-    g.ntiles = pref.back();
-    if (g.ntasks == 0) pref.pop_back();
+    g.ntiles = (int64_t)tiles.size() - g.tile0;
   }
 
   void upload(cudaStream_t st) {
@@ -229,7 +228,7 @@ struct Plan {
       cap = c;
     };
     grow(d_tasks, cap_tasks, tasks.size(), "alloc plan tasks");
-    grow(d_pref, cap_pref, pref.size(), "alloc plan prefixes");
+    grow(d_tiles, cap_tiles, tiles.size(), "alloc plan tiles");
     grow(d_ids, cap_ids, ids.size(), "alloc plan ids");
     grow(d_cpref, cap_cpref, cpref.size(), "alloc plan phase prefixes");
     grow(d_ttask, cap_ttask, ttask.size(), "alloc plan tile tasks");
@@ -237,9 +236,10 @@ struct Plan {
     if (!tasks.empty())
       ck(cudaMemcpyAsync(d_tasks, tasks.data(), tasks.size() * sizeof(Task), cudaMemcpyHostToDevice, st),
          "upload tasks");
-    if (!pref.empty())
-      ck(cudaMemcpyAsync(d_pref, pref.data(), pref.size() * sizeof(int64_t), cudaMemcpyHostToDevice, st),
-         "upload prefixes");
+    if (!tiles.empty())
+      ck(cudaMemcpyAsync(d_tiles, tiles.data(), tiles.size() * sizeof(int2), cudaMemcpyHostToDevice,
+                         st),
+         "upload tiles");
     if (!ids.empty())
       ck(cudaMemcpyAsync(d_ids, ids.data(), ids.size() * sizeof(int), cudaMemcpyHostToDevice, st),
          "upload ids");
@@ -343,6 +343,7 @@ struct mfgpu_handle {
   int n = 0;
   int64_t nnz = 0;
   std::vector<int> h_rowptr, h_colind;
+  bool longRows = false;       // some row of the matrix has more than eight entries
 
   void* d_F = nullptr;             // front arena (double or float)
   void* d_Sep = nullptr;           // separator arena (double or float)
@@ -545,11 +546,11 @@ struct mfgpu_handle {
       }
       P.nfronts += (int)fl.size();
       L.assemble = P.beginGroup();
-      P.appendGroup(s.front_tasks, s.front_task_ptr, fl, false);
-      P.appendGroup(s.sep_tasks, s.sep_task_ptr, sl, false);
+      P.appendGroup(L.assemble, s.front_tasks, s.front_task_ptr, fl, false, longRows);
+      P.appendGroup(L.assemble, s.sep_tasks, s.sep_task_ptr, sl, false, longRows);
       P.endGroup(L.assemble);
       L.sadd = P.beginGroup();
-      P.appendGroup(s.sep_add_tasks, s.sep_task_ptr, sl, true);
+      P.appendGroup(L.sadd, s.sep_add_tasks, s.sep_task_ptr, sl, true, longRows);
       P.endGroup(L.sadd);
       L.cpref0 = (int64_t)P.cpref.size();
       // tile tasks for every level of the full plan (the autotuner may time any
@@ -685,33 +686,32 @@ struct mfgpu_handle {
           P.real.push_back(k);
         }
       L.ns = (int64_t)P.ids.size() - L.s0;
-      auto append = [&](const std::vector<Task>& src, const std::vector<int64_t>& ptr,
+      auto append = [&](Group& g, const std::vector<Task>& src, const std::vector<int64_t>& ptr,
                         const std::vector<std::vector<int>>& own, bool pairs) {
         for (size_t m = 0; m < nm; m++) {
           const BatchMember& bm = M[m];
-          P.appendGroup(src, ptr, own[m], pairs, [&bm](Task& t) {
+          P.appendGroup(g, src, ptr, own[m], pairs, longRows, [&bm](Task& t) {
             bm.move(t);
             if (t.kind == mfgpu::TK_SPARSE) t.src_off = bm.valoff;
           });
         }
       };
       L.assemble = P.beginGroup();
-      append(s.front_tasks, s.front_task_ptr, fl, false);
-      append(s.sep_tasks, s.sep_task_ptr, sl, false);
+      append(L.assemble, s.front_tasks, s.front_task_ptr, fl, false);
+      append(L.assemble, s.sep_tasks, s.sep_task_ptr, sl, false);
       P.endGroup(L.assemble);
       L.sadd = P.beginGroup();
-      append(s.sep_add_tasks, s.sep_task_ptr, sl, true);
+      append(L.sadd, s.sep_add_tasks, s.sep_task_ptr, sl, true);
       P.endGroup(L.sadd);
     }
   }
 
   template <class T>
   void runGroup(const Plan& P, const Group& g, int64_t bytes) {
-    if (g.ntasks == 0 || g.ntiles == 0) return;
+    if (g.ntiles == 0) return;
     prof.begin(MFGPU_KC_ASSEMBLE, stream);
-    mfgpu::launch_tasks<T>(P.d_tasks + g.task0, P.d_pref + g.pref0, (int)g.ntasks, g.ntiles,
-                           (T*)d_F, (T*)d_Sep, d_rp, d_ci, d_val, d_dofs, mixed ? d_scale : nullptr,
-                           stream);
+    mfgpu::launch_tasks<T>(P.d_tasks + g.task0, P.d_tiles + g.tile0, g.ntiles, g.staged, (T*)d_F,
+                           (T*)d_Sep, d_rp, d_ci, d_val, d_dofs, mixed ? d_scale : nullptr, stream);
     ck(cudaGetLastError(), "launch assembly (k_tasks)");
     prof.end(stream);
     if (prof.on) prof.bytes[MFGPU_KC_ASSEMBLE] += (double)bytes;
@@ -1832,6 +1832,7 @@ int createFrom(std::unique_ptr<Schedule> sched, int n, const int* row_ptr, const
   if (h->lu) h->solveCoopMinN = 0;   // LU fronts use the per-front sweeps
   h->h_rowptr.assign(row_ptr, row_ptr + n + 1);
   h->h_colind.assign(col_ind, col_ind + h->nnz);
+  for (int i = 0; i < n; i++) h->longRows |= row_ptr[i + 1] - row_ptr[i] > 8;
   int st = guarded(h.get(), [&]() {
     mfgpu_handle& H = *h;
     ck(cudaStreamCreateWithFlags(&H.own, cudaStreamNonBlocking), "create stream");
@@ -3090,6 +3091,7 @@ std::unique_ptr<mfgpu_handle> makeView(mfgpu_handle& B) {
   H.device = B.device;
   H.n = B.n;
   H.nnz = B.nnz;
+  H.longRows = B.longRows;
   H.d_F = B.d_F;
   H.d_Sep = B.d_Sep;
   H.d_rp = B.d_rp;
