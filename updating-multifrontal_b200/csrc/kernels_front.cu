@@ -462,8 +462,8 @@ __device__ __forceinline__ void row_trsm(double (&x)[kPanel], const double (*L)[
 // Fused partial factorization, one CTA per front (fronts up to kSmallMaxN).
 // The panel of each step is staged in shared memory for the tensor-core update.
 // ---------------------------------------------------------------------------
-template <class T>
-__global__ void __launch_bounds__(256, 2) k_front_small(const int* __restrict__ flist,
+template <class T, int NT>
+__global__ void __launch_bounds__(NT, 512 / NT) k_front_small(const int* __restrict__ flist,
                                                      const FrontDev* __restrict__ fr,
                                                      T* __restrict__ F, DevError* err) {
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -488,7 +488,7 @@ __global__ void __launch_bounds__(256, 2) k_front_small(const int* __restrict__ 
       Psm[rr * kPS + t] = (rr < M && t < kb) ? A[(r0 + rr) + (int64_t)(k + t) * ld] : T(0);
     }
     __syncthreads();
-    for (int R0 = warp * 32; R0 < Mp; R0 += 256) warp_trsm_block(Psm, R0, Li, kb, A, ld, r0, k, M, lane);
+    for (int R0 = warp * 32; R0 < Mp; R0 += NT) warp_trsm_block(Psm, R0, Li, kb, A, ld, r0, k, M, lane);
     __syncthreads();
     const int TT = Mp >> 5;
     const int ntile = TT * (TT + 1) / 2;
@@ -504,7 +504,7 @@ __global__ void __launch_bounds__(256, 2) k_front_small(const int* __restrict__ 
       __syncwarp();
       if (r0 < d.n) warp_factor_inv(A, ld, r0, min(kPanel, d.n - r0), Ls, Li, Dinv, err, f);
     } else {
-      for (int t = warp; t < ntile; t += 7) {   // warps 1..7 take tiles 1, 2, ...
+      for (int t = warp; t < ntile; t += NT / 32 - 1) {   // the other warps take tiles 1, 2, ...
         int I, J;
         tri_index(t, I, J);
         T acc[4][4][2];
@@ -1115,19 +1115,29 @@ cudaError_t launch_level_coop(const int* flist, int nf, int maxn, const FrontDev
   return e;
 }
 
+// 128 threads a front when no front has more than four 32-row blocks (four CTAs
+// an SM overlap their diagonal blocks' chains: the leaves of 24 2D problems, 1.45
+// -> 0.96 ms), 256 otherwise.
+template <class T, int NT>
+void front_small(const int* flist, int nf, size_t sm, const FrontDev* fr, T* F, DevError* err,
+                 cudaStream_t st) {
+  // the largest dynamic size any launch asks for, set once (launches from
+  // several host threads must not race on the attribute)
+  static const bool attr = (cudaFuncSetAttribute(k_front_small<T, NT>,
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 200 * 1024),
+                            true);
+  (void)attr;
+  k_front_small<T, NT><<<nf, NT, sm, st>>>(flist, fr, F, err);
+}
+
 template <class T>
 void launch_front_small(const int* flist, int nf, int maxN, const FrontDev* fr, T* F, DevError* err,
                         cudaStream_t st) {
   if (nf <= 0) return;
   const size_t sm = (size_t)((maxN + 31) & ~31) * kPS * sizeof(T);
-  // the largest dynamic size any launch asks for, set once (launches from
-  // several host threads must not race on the attribute)
-  static const bool attr = (cudaFuncSetAttribute(k_front_small<T>,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 200 * 1024),
-                            true);
-  (void)attr;
-  k_front_small<T><<<nf, 256, sm, st>>>(flist, fr, F, err);
+  if (maxN <= 128) front_small<T, 128>(flist, nf, sm, fr, F, err, st);
+  else front_small<T, 256>(flist, nf, sm, fr, F, err, st);
   g_launches++;
 }
 
