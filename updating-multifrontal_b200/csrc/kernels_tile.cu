@@ -208,6 +208,17 @@ struct Acc<float> {
   }
 };
 
+// Four consecutive values from 16-byte aligned shared memory.
+__device__ __forceinline__ void ld4s(const float* p, float (&v)[4]) {
+  const float4 q = *reinterpret_cast<const float4*>(p);
+  v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+}
+__device__ __forceinline__ void ld4s(const double* p, double (&v)[4]) {
+  const double2 a = *reinterpret_cast<const double2*>(p);
+  const double2 b = *reinterpret_cast<const double2*>(p + 2);
+  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
+
 // Cholesky factor of the 64 x 64 block in w (column c at w[c * DS], rows 0 ..
 // 63, lower triangle, zeros above) over its first kb columns, and beside it
 // the same column operations on the 64 rows of an identity (rows 64 .. 127),
@@ -291,33 +302,29 @@ __device__ int diag_factor(T* w, int kb, T (*q4)[B][4], T (*d4)[4][4]) {
     for (int c = 0; c < 32; c++) w[(c0 + c) * DS + tid] = c0 + c < kb ? row[c] : T(0);
     __syncthreads();
     if (h == 0 && kb > 32) {
-      // columns 32 .. 63 of every row: - X(:, 0:32) L(32:64, 0:32)^T, 8 columns
-      // and 8 rows a thread
-      const int rg = (tid & 15) * 4, cg = 32 + (tid >> 4) * 4;   // rows rg .. + 3, + 64; 4 columns
-      T a[8][4];
+      // columns 32 .. 63: - X(:, 0:32) L(32:64, 0:32)^T for the rows that have
+      // some, 32 .. 63 of the block and the first 32 of the identity, 4 x 4 a thread
+      const int rg = 32 + (tid & 15) * 4, cg = 32 + (tid >> 4) * 4;
+      T a[4][4];
 #pragma unroll
-      for (int i = 0; i < 8; i++)
+      for (int i = 0; i < 4; i++)
 #pragma unroll
         for (int j = 0; j < 4; j++) a[i][j] = T(0);
-#pragma unroll 4
+#pragma unroll 8
       for (int t = 0; t < 32; t++) {
-        T xr[8], yc[4];
+        T xr[4], yc[4];
+        ld4s(w + t * DS + rg, xr);
+        ld4s(w + t * DS + cg, yc);
 #pragma unroll
-        for (int i = 0; i < 8; i++) xr[i] = w[t * DS + (i >> 2) * B + rg + (i & 3)];
-#pragma unroll
-        for (int j = 0; j < 4; j++) yc[j] = w[t * DS + cg + j];
-#pragma unroll
-        for (int i = 0; i < 8; i++)
+        for (int i = 0; i < 4; i++)
 #pragma unroll
           for (int j = 0; j < 4; j++) a[i][j] = fma(xr[i], yc[j], a[i][j]);
       }
 #pragma unroll
       for (int j = 0; j < 4; j++)
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-          const int rw = (i >> 2) * B + rg + (i & 3);
-          if (rw >= cg + j) w[(cg + j) * DS + rw] -= a[i][j];   // (entries above stay zero)
-        }
+        for (int i = 0; i < 4; i++)
+          if (rg + i >= cg + j) w[(cg + j) * DS + rg + i] -= a[i][j];   // (entries above stay zero)
       __syncthreads();
     }
   }
@@ -477,6 +484,7 @@ __global__ void __launch_bounds__(TT, 3)
           if (r0 + r < N && (r >= c || r < kb))
             P[(int64_t)c * ld] = r >= c ? sm[c * DS + r] : sm[c * DS + B + r];
       }
+      publish(J + 1);
       if (dinv_off[f] >= 0) {
         T* D = Dv + dinv_off[f] + (int64_t)J * 2 * B * B;
         for (int idx = tid; idx < B * B; idx += TT) {
@@ -486,7 +494,6 @@ __global__ void __launch_bounds__(TT, 3)
           D[idx] = in ? sm[r * DS + B + c] : T(0);           // Linv(r, c)
         }
       }
-      publish(J + 1);
       continue;
     }
     // times L_JJ^{-T}
