@@ -479,7 +479,7 @@ __global__ void __launch_bounds__(SCT) k_solve_flow_bwd(const int* __restrict__ 
 // ms, backward 7.65 -> 1.78 ms; 2D 1023^2, 4, 428 -> 192 and 420 -> 228 us; 3D 79
 // x 63 x 50, one, 1287 -> 992 and 1181 -> 954 us.
 // ---------------------------------------------------------------------------
-constexpr int MS = 12;           // right-hand-side stride in shared memory per 8 (no bank conflicts)
+constexpr int MS = 12;           // row stride of 8 right-hand sides in shared memory (no bank conflicts)
 
 __device__ __forceinline__ void mma884(double (&c)[2], double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
@@ -488,15 +488,27 @@ __device__ __forceinline__ void mma884(double (&c)[2], double a, double b) {
 }
 
 // c[t] += A x for 64 columns: a[s] is the lane's fragment of columns 4 s .. + 3,
-// x(k, rhs) at xs[k * MS * NT + rhs] (rhs 8 t + ..: 12 t + ..).  Two chains.
+// x(k, 8 t + rhs) at xs[t * SB * MS + k * MS + rhs], in four chains (a product's
+// result takes 65 cycles).
 template <int NT>
-__device__ __forceinline__ void mma_block(double (&c)[NT][2][2], const double (&a)[16],
+__device__ __forceinline__ void mma_block(double (&c)[NT][4][2], const double (&a)[16],
                                           const double* xs, int rr, int cc) {
 #pragma unroll
   for (int s = 0; s < 16; s++)
 #pragma unroll
     for (int t = 0; t < NT; t++)
-      mma884(c[t][s & 1], a[s], xs[(4 * s + cc) * (MS * NT) + MS * t + rr]);
+      mma884(c[t][s & 3], a[s], xs[t * SB * MS + (4 * s + cc) * MS + rr]);
+}
+
+template <int NT>
+__device__ __forceinline__ void mma_zero(double (&c)[NT][4][2]) {
+#pragma unroll
+  for (int t = 0; t < NT; t++)
+#pragma unroll
+    for (int s = 0; s < 4; s++) c[t][s][0] = c[t][s][1] = 0.0;
+}
+__device__ __forceinline__ double mma_sum(const double (&c)[4][2], int e) {
+  return (c[0][e] + c[1][e]) + (c[2][e] + c[3][e]);
 }
 
 // x(k, rhs) of 64 rows into shared memory, zero outside [0, nr) x [0, nrhs).
@@ -504,7 +516,7 @@ template <int NT, class Get>
 __device__ __forceinline__ void stage_rhs(double* xs, int nr, int nrhs, Get&& get) {
   for (int idx = threadIdx.x; idx < SB * 8 * NT; idx += SCT) {
     const int r = idx & (SB - 1), c = idx / SB;
-    xs[r * (MS * NT) + MS * (c >> 3) + (c & 7)] = r < nr && c < nrhs ? get(r, c) : 0.0;
+    xs[(c >> 3) * SB * MS + r * MS + (c & 7)] = r < nr && c < nrhs ? get(r, c) : 0.0;
   }
 }
 
@@ -534,9 +546,8 @@ __global__ void __launch_bounds__(SCT, 2)
     const bool live = w8 + rr < rows;
     // this lane's row, first column cc (dead rows read the block's first row)
     const double* Ar = F + d.off + row0 + (live ? w8 + rr : 0) + (int64_t)min(cc, d.N - 1) * d.ld;
-    double acc[NT][2][2];
-#pragma unroll
-    for (int q = 0; q < NT; q++) acc[q][0][0] = acc[q][0][1] = acc[q][1][0] = acc[q][1][1] = 0.0;
+    double acc[NT][4][2];
+    mma_zero(acc);
     auto load = [&](double (&a)[16], int j) {   // L(row, block j)
       const int c0 = j * SB + cc;
 #pragma unroll
@@ -593,7 +604,7 @@ __global__ void __launch_bounds__(SCT, 2)
         for (int e = 0; e < 2; e++) {
           const int c = 8 * q + 2 * cc + e;
           if (live && c < nrhs)
-            W[row0 + w8 + rr + (int64_t)c * d.N] = -(acc[q][0][e] + acc[q][1][e]);
+            W[row0 + w8 + rr + (int64_t)c * d.N] = -mma_sum(acc[q], e);
         }
       __syncthreads();                          // xs is free for the next task
       continue;
@@ -604,18 +615,17 @@ __global__ void __launch_bounds__(SCT, 2)
     for (int q = 0; q < NT; q++)
 #pragma unroll
       for (int e = 0; e < 2; e++)
-        ws[(w8 + rr) * (MS * NT) + MS * q + 2 * cc + e] =
-            live ? b[q][e] - (acc[q][0][e] + acc[q][1][e]) : 0.0;
+        ws[q * SB * MS + (w8 + rr) * MS + 2 * cc + e] =
+            live ? b[q][e] - mma_sum(acc[q], e) : 0.0;
     __syncthreads();
-#pragma unroll
-    for (int q = 0; q < NT; q++) acc[q][0][0] = acc[q][0][1] = acc[q][1][0] = acc[q][1][1] = 0.0;
+    mma_zero(acc);
     mma_block<NT>(acc, an, ws, rr, cc);
 #pragma unroll
     for (int q = 0; q < NT; q++)
 #pragma unroll
       for (int e = 0; e < 2; e++) {
         const int c = 8 * q + 2 * cc + e;
-        const double y = acc[q][0][e] + acc[q][1][e];
+        const double y = mma_sum(acc[q], e);
         if (live && c < nrhs) {
           Y[row0 + w8 + rr + (int64_t)c * d.N] = y;
           X[dl[row0 + w8 + rr] + (int64_t)c * ldx] = y;
@@ -651,9 +661,8 @@ __global__ void __launch_bounds__(SCT, 2)
     const int nb = cdiv(d.n, SB), nbr = cdiv(d.N, SB), col0 = j * SB, kbj = min(SB, d.n - col0);
     const bool live = w8 + rr < kbj;
     const double* Lc = F + d.off + (int64_t)(col0 + (live ? w8 + rr : 0)) * d.ld + 2 * cc;
-    double acc[NT][2][2];
-#pragma unroll
-    for (int q = 0; q < NT; q++) acc[q][0][0] = acc[q][0][1] = acc[q][1][0] = acc[q][1][1] = 0.0;
+    double acc[NT][4][2];
+    mma_zero(acc);
     // rows of block R this task takes: below its pivots, inside the front
     auto load = [&](double (&a)[16], int R) {
       const int r0 = R * SB, lo = R == j ? d.n : r0;
@@ -682,7 +691,7 @@ __global__ void __launch_bounds__(SCT, 2)
         if (g >= lo && g < d.N && c < nrhs)
           v = g < d.n ? ldcg(Y + g + (int64_t)c * d.N) : X[dl[g] + (int64_t)c * ldx];
         const int k = (r & ~7) + 4 * (r & 1) + ((r & 7) >> 1);
-        x[k * (MS * NT) + MS * (c >> 3) + (c & 7)] = v;
+        x[(c >> 3) * SB * MS + k * MS + (c & 7)] = v;
       }
     };
     // last block this task reads last: the one after it, or its own boundary rows
@@ -728,18 +737,17 @@ __global__ void __launch_bounds__(SCT, 2)
     for (int q = 0; q < NT; q++)
 #pragma unroll
       for (int e = 0; e < 2; e++)
-        ws[(w8 + rr) * (MS * NT) + MS * q + 2 * cc + e] =
-            live ? b[q][e] - (acc[q][0][e] + acc[q][1][e]) : 0.0;
+        ws[q * SB * MS + (w8 + rr) * MS + 2 * cc + e] =
+            live ? b[q][e] - mma_sum(acc[q], e) : 0.0;
     __syncthreads();
-#pragma unroll
-    for (int q = 0; q < NT; q++) acc[q][0][0] = acc[q][0][1] = acc[q][1][0] = acc[q][1][1] = 0.0;
+    mma_zero(acc);
     mma_block<NT>(acc, an, ws, rr, cc);
 #pragma unroll
     for (int q = 0; q < NT; q++)
 #pragma unroll
       for (int e = 0; e < 2; e++) {
         const int c = 8 * q + 2 * cc + e;
-        const double x = acc[q][0][e] + acc[q][1][e];
+        const double x = mma_sum(acc[q], e);
         if (live && c < nrhs) {
           Y[col0 + w8 + rr + (int64_t)c * d.N] = x;
           X[dl[col0 + w8 + rr] + (int64_t)c * ldx] = x;
