@@ -215,14 +215,14 @@ cudaError_t launch_trail_tc(const int* flist, int nf, int64_t ntiles, const Fron
 // and scattering to X themselves.  flow_tasks builds a level's task lists
 // (front slot, block) pairs, forward R-major and backward by distance from
 // each front's last block, and the per-front offsets of the ready flags
-// (flagoff[nf] = flags needed); `flags` is cleared before every launch.
+// (flagoff[nf] = flags needed); `flags`: flow_scratch_bytes(flags, element
+// bytes) of scratch for the flags and the solved blocks, reset by every launch.
 int solve_coop_max_fronts();
+size_t flow_scratch_bytes(int nflags, int elem_bytes);
 void flow_tasks(const std::vector<int>& n, const std::vector<int>& N, std::vector<int>& fwd,
                 std::vector<int>& bwd, std::vector<int>& flagoff);
 // The sweeps apply each 64 x 64 pivot block through its explicit inverse (Dv,
-// per front at dinv_off, written by launch_diag_inv after the front is
-// factored) and keep solved blocks in the second half of the front's
-// workspace, where other tasks read them.
+// per front at dinv_off, written by the tile kernel or launch_diag_inv).
 template <class T>
 cudaError_t launch_solve_flow(bool forward, const int* flist, const FrontDev* fr, const T* F,
                               const int* dofs, T* X, int64_t ldx, int nrhs, T* W,

@@ -23,8 +23,8 @@
 //
 // W is the front's right-hand-side block (N x nrhs, ld N) in the same
 // workspace the per-front kernels use, so the separator gathers between
-// levels are unchanged; the solved pivot blocks go to the second half of that
-// workspace (Y, another N x nrhs), where other tasks read them.
+// levels are unchanged; the solved pivot blocks go to the launch's scratch (Y,
+// 64 rows per pivot block and nrhs columns a front), where other tasks read them.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -87,24 +87,35 @@ __global__ void __launch_bounds__(SB) k_diag_inv(const int* __restrict__ flist,
   }
 }
 
-// Ready flags of the solved pivot blocks: written once per launch (after the
-// block's values are visible device-wide), read by spinning thread 0s.  A
-// wait gives up after the error word's poll limit (default kFlowSpin),
-// records error code 3 and lets the CTA go on, so the launch always ends.
+// Hand-off of the solved pivot blocks.  A launch starts with its scratch set to
+// all ones: a block's flag is negative until its values are visible
+// device-wide, and a value holds the all-ones NaN until it is written.  The task
+// that a block is the last dependency of (the next link of the chain) polls the
+// values themselves, which saves the writer's fence, the flag and a second
+// trip through L2; every other task waits for the flag, the less often the
+// farther it is from the front's chain, so that the hundreds of waiting CTAs do
+// not queue at the flag's L2 slice.  A wait gives up after the error word's poll
+// limit (default kFlowSpin), records error code 3 and lets the CTA go on, so the
+// launch always ends.
 constexpr unsigned kFlowSpin = 1u << 25;
 
-__device__ __forceinline__ void flow_wait(const int* flag, DevError* err) {
+// One poll of a bounded wait has failed: true to give up.
+__device__ __forceinline__ bool flow_give_up(unsigned& it, unsigned lim, DevError* err) {
+  if (++it > lim) {
+    if (err) atomicCAS(&err->code, 0, 3);
+    return true;
+  }
+  return (it & 1023u) == 0 && err && *(volatile int*)&err->code == 3;   // another CTA gave up
+}
+
+// dist: blocks between this task's chain and the flag's.
+__device__ __forceinline__ void flow_wait(const int* flag, DevError* err, int dist = 0) {
   const volatile int* f = flag;
-  volatile int* code = err ? &err->code : nullptr;
   const unsigned lim = wait_limit(err, kFlowSpin);
   unsigned it = 0;
-  while (*f == 0) {
-    if (++it > lim) {
-      if (err) atomicCAS(&err->code, 0, 3);
-      break;
-    }
-    if ((it & 1023u) == 0 && code && *code == 3) break;   // another CTA gave up
-    __nanosleep(32);
+  while (*f < 0) {
+    if (flow_give_up(it, lim, err)) break;
+    __nanosleep(32 + 32 * min(dist, 32));
   }
   __threadfence();
 }
@@ -112,6 +123,27 @@ __device__ __forceinline__ void flow_wait(const int* flag, DevError* err) {
 __device__ __forceinline__ void flow_publish(int* flag) {
   __threadfence();
   atomicExch(flag, 1);
+}
+
+// The value at p once it is written.
+__device__ __forceinline__ bool unwritten(float v) { return __float_as_int(v) == -1; }
+__device__ __forceinline__ bool unwritten(double v) { return __double_as_longlong(v) == -1ll; }
+template <class T>
+__device__ __forceinline__ T flow_value(const T* p, DevError* err) {
+  const volatile T* q = p;
+  T v = *q;
+  if (unwritten(v)) {
+    const unsigned lim = wait_limit(err, kFlowSpin);
+    unsigned it = 0;
+    while (unwritten(v = *q))
+      if (flow_give_up(it, lim, err)) return T(0);
+  }
+  return v;
+}
+// A value to hand off: never the unwritten pattern (a NaN stays a NaN).
+__device__ __forceinline__ float written(float v) { return unwritten(v) ? __int_as_float(0x7fffffff) : v; }
+__device__ __forceinline__ double written(double v) {
+  return unwritten(v) ? __longlong_as_double(0x7fffffffffffffffll) : v;
 }
 
 template <class T>
@@ -145,7 +177,7 @@ __global__ void __launch_bounds__(SCT) k_solve_flow_fwd(const int* __restrict__ 
                                                         const int64_t* __restrict__ dinv_off,
                                                         const int2* __restrict__ tasks, int ntasks,
                                                         const int* __restrict__ flagoff, int* flags,
-                                                        DevError* err) {
+                                                        T* Yb, DevError* err) {
   constexpr int CH = 4;                       // column blocks per shared-memory round
   __shared__ T ys[CH * SB][NR + 1];           // solved blocks
   __shared__ T ws[SB][NR + 1];                // b_R - acc of the block
@@ -156,7 +188,8 @@ __global__ void __launch_bounds__(SCT) k_solve_flow_fwd(const int* __restrict__ 
     const FrontDev d = fr[f];
     const T* A = F + d.off;
     T* W = Wb + woff[f] * nrhs;
-    T* Y = W + (int64_t)d.N * nrhs;
+    const int ldy = cdiv(d.n, SB) * SB;
+    T* Y = Yb + (int64_t)flagoff[i] * SB * nrhs;
     const int* dl = dofs + d.dof_off;
     const int* fl = flags + flagoff[i];
     const int nb = cdiv(d.n, SB);
@@ -182,12 +215,12 @@ __global__ void __launch_bounds__(SCT) k_solve_flow_fwd(const int* __restrict__ 
       const int jc = min(CH, jmax - 1 - j0);
       __syncthreads();                        // ys of the previous round is consumed
       if (tid == 0)
-        for (int jj = 0; jj < jc; jj++) flow_wait(fl + j0 + jj, err);
+        for (int jj = 0; jj < jc; jj++) flow_wait(fl + j0 + jj, err, jmax - 1 - j0 - jj);
       __syncthreads();
       for (int idx = tid; idx < jc * SB * nrhs; idx += SCT) {
         const int r = idx % (jc * SB), c = idx / (jc * SB);
         const int col = j0 * SB + r;
-        ys[r][c] = col < d.n ? ldcg(Y + col + (int64_t)c * d.N) : T(0);
+        ys[r][c] = col < d.n ? ldcg(Y + col + (int64_t)c * ldy) : T(0);
       }
       __syncthreads();
       if (rl2 < rows) {
@@ -228,12 +261,10 @@ __global__ void __launch_bounds__(SCT) k_solve_flow_fwd(const int* __restrict__ 
     }
     if (jmax > 0) {
       __syncthreads();                        // ys of the previous round is consumed
-      if (tid == 0) flow_wait(fl + jmax - 1, err);
-      __syncthreads();
       for (int idx = tid; idx < SB * nrhs; idx += SCT) {
         const int r = idx % SB, c = idx / SB;
         const int col = (jmax - 1) * SB + r;
-        ys[r][c] = col < d.n ? ldcg(Y + col + (int64_t)c * d.N) : T(0);
+        ys[r][c] = col < d.n ? flow_value(Y + col + (int64_t)c * ldy, err) : T(0);
       }
       __syncthreads();
 #pragma unroll
@@ -275,7 +306,7 @@ __global__ void __launch_bounds__(SCT) k_solve_flow_fwd(const int* __restrict__ 
 #pragma unroll
       for (int c = 0; c < NR; c++)
         if (c < nrhs) {
-          Y[row0 + rl + (int64_t)c * d.N] = y[c];
+          Y[row0 + rl + (int64_t)c * ldy] = written(y[c]);
           X[dl[row0 + rl] + (int64_t)c * ldx] = y[c];
         }
     __syncthreads();
@@ -303,7 +334,7 @@ __global__ void __launch_bounds__(SCT) k_solve_flow_bwd(const int* __restrict__ 
                                                         const int64_t* __restrict__ dinv_off,
                                                         const int2* __restrict__ tasks, int ntasks,
                                                         const int* __restrict__ flagoff, int* flags,
-                                                        DevError* err) {
+                                                        T* Yb, DevError* err) {
   constexpr int BR = 4;                       // boundary row blocks per shared-memory round
   // Up to four right-hand sides the rows below go warp by column: warp wp
   // takes columns 8 wp .. 8 wp + 7 of the block, its lanes 32 consecutive rows
@@ -320,7 +351,8 @@ __global__ void __launch_bounds__(SCT) k_solve_flow_bwd(const int* __restrict__ 
     const FrontDev d = fr[f];
     const T* A = F + d.off;
     T* W = Wb + woff[f] * nrhs;
-    T* Y = W + (int64_t)d.N * nrhs;
+    const int ldy = cdiv(d.n, SB) * SB;
+    T* Y = Yb + (int64_t)flagoff[i] * SB * nrhs;
     const int* dl = dofs + d.dof_off;
     const int* fl = flags + flagoff[i];
     const int nb = cdiv(d.n, SB), col0 = j * SB, kbj = min(SB, d.n - col0);
@@ -378,11 +410,11 @@ __global__ void __launch_bounds__(SCT) k_solve_flow_bwd(const int* __restrict__ 
     for (int R = nb - 1; R > j + 1; R--) {              // solved pivot blocks below but the nearest
       const int r0 = R * SB, nr = min(SB, d.n - r0);
       __syncthreads();
-      if (tid == 0) flow_wait(fl + R, err);
+      if (tid == 0) flow_wait(fl + R, err, R - j - 1);
       __syncthreads();
       for (int idx = tid; idx < SB * nrhs; idx += SCT) {
         const int r = idx % SB, c = idx / SB;
-        xs[r][c] = r < nr ? ldcg(Y + r0 + r + (int64_t)c * d.N) : T(0);
+        xs[r][c] = r < nr ? ldcg(Y + r0 + r + (int64_t)c * ldy) : T(0);
       }
       __syncthreads();
       chunk(r0, nr, 0);
@@ -418,11 +450,9 @@ __global__ void __launch_bounds__(SCT) k_solve_flow_bwd(const int* __restrict__ 
     }
     if (nn > 0) {
       __syncthreads();                        // xs of the previous round is consumed
-      if (tid == 0) flow_wait(fl + j + 1, err);
-      __syncthreads();
       for (int idx = tid; idx < SB * nrhs; idx += SCT) {
         const int r = idx % SB, c = idx / SB;
-        xs[r][c] = r < nn ? ldcg(Y + rn + r + (int64_t)c * d.N) : T(0);
+        xs[r][c] = r < nn ? flow_value(Y + rn + r + (int64_t)c * ldy, err) : T(0);
       }
       __syncthreads();
 #pragma unroll
@@ -457,7 +487,7 @@ __global__ void __launch_bounds__(SCT) k_solve_flow_bwd(const int* __restrict__ 
 #pragma unroll
       for (int c = 0; c < NR; c++)
         if (c < nrhs) {
-          Y[col0 + cl + (int64_t)c * d.N] = x[c];
+          Y[col0 + cl + (int64_t)c * ldy] = written(x[c]);
           X[dl[col0 + cl] + (int64_t)c * ldx] = x[c];
         }
     __syncthreads();
@@ -527,7 +557,7 @@ __global__ void __launch_bounds__(SCT, 2)
                  int nrhs, double* Wb, const int64_t* __restrict__ woff,
                  const double* __restrict__ Dv, const int64_t* __restrict__ dinv_off,
                  const int2* __restrict__ tasks, int ntasks, const int* __restrict__ flagoff,
-                 int* flags, DevError* err) {
+                 int* flags, double* Yb, DevError* err) {
   __shared__ double xs[2][SB * MS * NT];
   const int tid = threadIdx.x, lane = tid & 31, w8 = 8 * (tid >> 5), rr = lane >> 2, cc = lane & 3;
   for (int t = blockIdx.x; t < ntasks; t += gridDim.x) {
@@ -535,7 +565,8 @@ __global__ void __launch_bounds__(SCT, 2)
     const int i = tk.x, R = tk.y, f = flist[i];
     const FrontDev d = fr[f];
     double* W = Wb + woff[f] * nrhs;
-    double* Y = W + (int64_t)d.N * nrhs;
+    const int ldy = cdiv(d.n, SB) * SB;
+    double* Y = Yb + (int64_t)flagoff[i] * SB * nrhs;
     const int* dl = dofs + d.dof_off;
     const int* fl = flags + flagoff[i];
     const int nb = cdiv(d.n, SB);
@@ -560,13 +591,13 @@ __global__ void __launch_bounds__(SCT, 2)
     };
     auto solved = [&](int j) {
       return [&, j](int r, int c) {
-        return j * SB + r < d.n ? ldcg(Y + j * SB + r + (int64_t)c * d.N) : 0.0;
+        return j * SB + r < d.n ? ldcg(Y + j * SB + r + (int64_t)c * ldy) : 0.0;
       };
     };
     double a[16], an[16];
     if (jmax > 0) load(a, 0);
     for (int j = 0; j < jmax - 1; j++) {
-      if (tid == 0) flow_wait(fl + j, err);
+      if (tid == 0) flow_wait(fl + j, err, jmax - 1 - j);
       __syncthreads();
       stage_rhs<NT>(xs[j & 1], SB, nrhs, solved(j));
       load(an, j + 1);                          // the next block in flight
@@ -591,9 +622,10 @@ __global__ void __launch_bounds__(SCT, 2)
     }
     if (jmax > 0) {
       const int j = jmax - 1;
-      if (tid == 0) flow_wait(fl + j, err);
-      __syncthreads();
-      stage_rhs<NT>(xs[j & 1], SB, nrhs, solved(j));
+      __syncthreads();                          // xs of the round before the last is consumed
+      stage_rhs<NT>(xs[j & 1], SB, nrhs, [&](int r, int c) {
+        return j * SB + r < d.n ? flow_value(Y + j * SB + r + (int64_t)c * ldy, err) : 0.0;
+      });
       __syncthreads();
       mma_block<NT>(acc, a, xs[j & 1], rr, cc);
     }
@@ -627,7 +659,7 @@ __global__ void __launch_bounds__(SCT, 2)
         const int c = 8 * q + 2 * cc + e;
         const double y = mma_sum(acc[q], e);
         if (live && c < nrhs) {
-          Y[row0 + w8 + rr + (int64_t)c * d.N] = y;
+          Y[row0 + w8 + rr + (int64_t)c * ldy] = written(y);
           X[dl[row0 + w8 + rr] + (int64_t)c * ldx] = y;
         }
       }
@@ -648,14 +680,15 @@ __global__ void __launch_bounds__(SCT, 2)
                  int nrhs, double* Wb, const int64_t* __restrict__ woff,
                  const double* __restrict__ Dv, const int64_t* __restrict__ dinv_off,
                  const int2* __restrict__ tasks, int ntasks, const int* __restrict__ flagoff,
-                 int* flags, DevError* err) {
+                 int* flags, double* Yb, DevError* err) {
   __shared__ double xs[2][SB * MS * NT];
   const int tid = threadIdx.x, lane = tid & 31, w8 = 8 * (tid >> 5), rr = lane >> 2, cc = lane & 3;
   for (int t = blockIdx.x; t < ntasks; t += gridDim.x) {
     const int2 tk = tasks[t];
     const int i = tk.x, j = tk.y, f = flist[i];
     const FrontDev d = fr[f];
-    double* Y = Wb + woff[f] * nrhs + (int64_t)d.N * nrhs;
+    const int ldy = cdiv(d.n, SB) * SB;
+    double* Y = Yb + (int64_t)flagoff[i] * SB * nrhs;
     const int* dl = dofs + d.dof_off;
     const int* fl = flags + flagoff[i];
     const int nb = cdiv(d.n, SB), nbr = cdiv(d.N, SB), col0 = j * SB, kbj = min(SB, d.n - col0);
@@ -683,13 +716,15 @@ __global__ void __launch_bounds__(SCT, 2)
           }
       }
     };
-    auto stage = [&](double* x, int R) {        // x(row, rhs) in the fragments' row order
+    auto stage = [&](double* x, int R, bool last) {   // x(row, rhs) in the fragments' row order
       const int r0 = R * SB, lo = R == j ? d.n : r0;
       for (int idx = tid; idx < SB * 8 * NT; idx += SCT) {
         const int r = idx & (SB - 1), c = idx / SB, g = r0 + r;
         double v = 0.0;
         if (g >= lo && g < d.N && c < nrhs)
-          v = g < d.n ? ldcg(Y + g + (int64_t)c * d.N) : X[dl[g] + (int64_t)c * ldx];
+          v = g >= d.n ? X[dl[g] + (int64_t)c * ldx]
+              : last   ? flow_value(Y + g + (int64_t)c * ldy, err)
+                       : ldcg(Y + g + (int64_t)c * ldy);
         const int k = (r & ~7) + 4 * (r & 1) + ((r & 7) >> 1);
         x[(c >> 3) * SB * MS + k * MS + (c & 7)] = v;
       }
@@ -700,10 +735,10 @@ __global__ void __launch_bounds__(SCT, 2)
     if (Rlast < nbr) load(a, nbr - 1);
     for (int R = nbr - 1; R > Rlast; R--) {
       if (R < nb) {
-        if (tid == 0) flow_wait(fl + R, err);
+        if (tid == 0) flow_wait(fl + R, err, R - j - 1);
         __syncthreads();
       }
-      stage(xs[R & 1], R);
+      stage(xs[R & 1], R, false);
       load(an, R - 1);
       __syncthreads();
       mma_block<NT>(acc, a, xs[R & 1], rr, cc);
@@ -723,11 +758,7 @@ __global__ void __launch_bounds__(SCT, 2)
         b[q][e] = live && c < nrhs ? X[dl[col0 + w8 + rr] + (int64_t)c * ldx] : 0.0;
       }
     if (Rlast < nbr) {
-      if (Rlast < nb && Rlast > j) {
-        if (tid == 0) flow_wait(fl + Rlast, err);
-        __syncthreads();
-      }
-      stage(xs[Rlast & 1], Rlast);
+      stage(xs[Rlast & 1], Rlast, true);
       __syncthreads();
       mma_block<NT>(acc, a, xs[Rlast & 1], rr, cc);
     }
@@ -749,7 +780,7 @@ __global__ void __launch_bounds__(SCT, 2)
         const int c = 8 * q + 2 * cc + e;
         const double x = mma_sum(acc[q], e);
         if (live && c < nrhs) {
-          Y[col0 + w8 + rr + (int64_t)c * d.N] = x;
+          Y[col0 + w8 + rr + (int64_t)c * ldy] = written(x);
           X[dl[col0 + w8 + rr] + (int64_t)c * ldx] = x;
         }
       }
@@ -771,6 +802,8 @@ int flowGrid(const void* kern) {
   return sms * std::max(1, per);
 }
 
+size_t flag_bytes(int nflags) { return ((size_t)std::max(1, nflags) * sizeof(int) + 15) & ~(size_t)15; }
+
 // Kernels of a direction and bound of the right-hand-side count: the scalar
 // form in FP32, the tensor-core form in FP64.
 template <class T, int NR>
@@ -790,7 +823,10 @@ cudaError_t launchFlowSolve(bool fwd, const int* flist, const FrontDev* fr, cons
                             const int64_t* woff, const T* Dv, const int64_t* dinv_off,
                             const int2* tasks, int ntasks, const int* flagoff, int* flags,
                             int nflags, DevError* err, cudaStream_t st) {
-  cudaError_t me = cudaMemsetAsync(flags, 0, sizeof(int) * (size_t)std::max(1, nflags), st);
+  // flags and, from a 16-byte boundary behind them, the solved blocks
+  const size_t fb = flag_bytes(nflags);
+  T* Y = reinterpret_cast<T*>(reinterpret_cast<unsigned char*>(flags) + fb);
+  cudaError_t me = cudaMemsetAsync(flags, 0xff, fb + (size_t)nflags * SB * nrhs * sizeof(T), st);
   if (me != cudaSuccess) return me;
   using K = FlowKernels<T, NR>;
   static const int gf = flowGrid(K::fwd());   // thread-safe one-time set-up
@@ -799,7 +835,7 @@ cudaError_t launchFlowSolve(bool fwd, const int* flist, const FrontDev* fr, cons
   void* args[] = {(void*)&flist, (void*)&fr,    (void*)&F,      (void*)&dofs,    (void*)&X,
                   (void*)&ldx,   (void*)&nrhs,  (void*)&W,      (void*)&woff,    (void*)&Dv,
                   (void*)&dinv_off, (void*)&tasks, (void*)&ntasks, (void*)&flagoff, (void*)&flags,
-                  (void*)&err};
+                  (void*)&Y,     (void*)&err};
   g_launches++;
   return cudaLaunchCooperativeKernel(fwd ? K::fwd() : K::bwd(), dim3(grid), dim3(SCT), args, 0, st);
 }
@@ -807,6 +843,10 @@ cudaError_t launchFlowSolve(bool fwd, const int* flist, const FrontDev* fr, cons
 }  // namespace
 
 int solve_coop_max_fronts() { return kMaxSolveCoopFronts; }
+
+size_t flow_scratch_bytes(int nflags, int elem_bytes) {
+  return flag_bytes(nflags) + (size_t)nflags * SB * 16 * elem_bytes;
+}
 
 void flow_tasks(const std::vector<int>& n, const std::vector<int>& N, std::vector<int>& fwd,
                 std::vector<int>& bwd, std::vector<int>& flagoff) {

@@ -1944,7 +1944,8 @@ int createFrom(std::unique_ptr<Schedule> sched, int n, const int* row_ptr, const
       if (!tab.empty())
         ck(cudaMemcpy(H.d_flow, tab.data(), tab.size() * sizeof(int), cudaMemcpyHostToDevice),
            "upload sweep task lists");
-      H.d_flags = dalloc<int>(std::max(H.maxFlags, 1), "alloc sweep ready flags");
+      H.d_flags = dalloc<int>(mfgpu::flow_scratch_bytes(H.maxFlags, (int)H.esz) / sizeof(int),
+                              "alloc sweep ready flags");
       H.d_dinv_off = dalloc<int64_t>(doff.size(), "alloc block inverse offsets");
       ck(cudaMemcpy(H.d_dinv_off, doff.data(), doff.size() * sizeof(int64_t),
                     cudaMemcpyHostToDevice), "upload block inverse offsets");
@@ -3142,7 +3143,8 @@ std::unique_ptr<mfgpu_handle> makeView(mfgpu_handle& B) {
   H.flow = B.flow;
   H.d_flow = B.d_flow;
   H.maxFlags = B.maxFlags;
-  H.d_flags = dalloc<int>(std::max(B.maxFlags, 1), "alloc sweep ready flags");
+  H.d_flags = dalloc<int>(mfgpu::flow_scratch_bytes(B.maxFlags, (int)B.esz) / sizeof(int),
+                          "alloc sweep ready flags");
   H.d_Dinv = dalloc<unsigned char>(std::max<int64_t>(B.dinvElems, 1) * H.esz, "alloc block inverses");
   if (H.mixed) {
     H.d_sc = dalloc<double>(80 * (size_t)H.nseg, "alloc refinement scalars");
