@@ -216,7 +216,8 @@ cudaError_t launch_trail_tc(const int* flist, int nf, int64_t ntiles, const Fron
 // (front slot, block) pairs, forward R-major and backward by distance from
 // each front's last block, and the per-front offsets of the ready flags
 // (flagoff[nf] = flags needed); `flags`: flow_scratch_bytes(flags, element
-// bytes) of scratch for the flags and the solved blocks, reset by every launch.
+// bytes) of scratch for the flags and the solved blocks, reset by every launch;
+// chain: a single front, bound by the chain of its blocks.
 int solve_coop_max_fronts();
 size_t flow_scratch_bytes(int nflags, int elem_bytes);
 void flow_tasks(const std::vector<int>& n, const std::vector<int>& N, std::vector<int>& fwd,
@@ -228,7 +229,7 @@ cudaError_t launch_solve_flow(bool forward, const int* flist, const FrontDev* fr
                               const int* dofs, T* X, int64_t ldx, int nrhs, T* W,
                               const int64_t* woff, const T* Dv, const int64_t* dinv_off,
                               const int* tasks, int ntasks, const int* flagoff, int* flags,
-                              int nflags, DevError* err, cudaStream_t st);
+                              int nflags, bool chain, DevError* err, cudaStream_t st);
 constexpr int kDinvBlock = 64;   // diagonal-block size of the cooperative sweeps
 template <class T>
 void launch_diag_inv(const int* flist, int nf, int maxn, const FrontDev* fr, const T* F, T* Dv,

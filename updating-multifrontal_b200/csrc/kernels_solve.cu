@@ -88,15 +88,20 @@ __global__ void __launch_bounds__(SB) k_diag_inv(const int* __restrict__ flist,
 }
 
 // Hand-off of the solved pivot blocks.  A launch starts with its scratch set to
-// all ones: a block's flag is negative until its values are visible
-// device-wide, and a value holds the all-ones NaN until it is written.  The task
-// that a block is the last dependency of (the next link of the chain) polls the
-// values themselves, which saves the writer's fence, the flag and a second
-// trip through L2; every other task waits for the flag, the less often the
-// farther it is from the front's chain, so that the hundreds of waiting CTAs do
-// not queue at the flag's L2 slice.  A wait gives up after the error word's poll
-// limit (default kFlowSpin), records error code 3 and lets the CTA go on, so the
-// launch always ends.
+// all ones: a block's flag is negative until its values are visible device-wide,
+// and a value holds the all-ones NaN until it is written.  The task of the next
+// link of the chain polls the values themselves, with its L in registers, which
+// saves the writer's fence, the flag and a second trip through L2; every other
+// task waits for the flag, the less often the farther it is from the front's
+// chain, so that the hundreds of waiting CTAs do not queue at the flag's L2
+// slice.  In a level of one front, where nothing but its chain bounds the sweep,
+// that goes for the next kChainTail links: a task takes the block before its last
+// dependency while that one is being solved, so that block must not lag either
+// (3D 63^3 root in FP32, three refinements' sweeps, 3.49 -> 2.65 ms; levels of
+// several fronts lose a tenth to the registers and stay with one).  A wait
+// gives up after the error word's poll limit (default kFlowSpin), records error
+// code 3 and lets the CTA go on, so the launch always ends.
+constexpr int kChainTail = 3;
 constexpr unsigned kFlowSpin = 1u << 25;
 
 // One poll of a bounded wait has failed: true to give up.
@@ -166,7 +171,7 @@ __device__ __forceinline__ T ldcg(const T* p) {
 // column offset still cover whole 32-byte sectors.  A task waits only on
 // tasks listed before it, and a cooperative launch keeps every CTA resident,
 // so the sweep cannot stall.
-template <class T, int NR>
+template <class T, int NR, int TAIL>
 __global__ void __launch_bounds__(SCT) k_solve_flow_fwd(const int* __restrict__ flist,
                                                         const FrontDev* __restrict__ fr,
                                                         const T* __restrict__ F,
@@ -202,17 +207,18 @@ __global__ void __launch_bounds__(SCT) k_solve_flow_fwd(const int* __restrict__ 
     T acc[NR];
 #pragma unroll
     for (int c = 0; c < NR; c++) acc[c] = T(0);
-    // every block but the last, CH at a time as their flags come up.  These
+    // every block but the last TAIL, CH at a time as their flags come up.  These
     // bulk loads go by (row tid & 63, column group tid >> 6): a warp reads 32
     // consecutive rows of a column (coalesced); the sums are handed to the
     // (row, quarter) lanes once, after the loop.
+    const int jbulk = max(0, jmax - TAIL);
     const int rl2 = tid & (SB - 1), g2 = tid >> 6;
     const T* Ar2 = A + row0 + rl2;
     T acc2[NR];
 #pragma unroll
     for (int c = 0; c < NR; c++) acc2[c] = T(0);
-    for (int j0 = 0; j0 < jmax - 1; j0 += CH) {
-      const int jc = min(CH, jmax - 1 - j0);
+    for (int j0 = 0; j0 < jbulk; j0 += CH) {
+      const int jc = min(CH, jbulk - j0);
       __syncthreads();                        // ys of the previous round is consumed
       if (tid == 0)
         for (int jj = 0; jj < jc; jj++) flow_wait(fl + j0 + jj, err, jmax - 1 - j0 - jj);
@@ -236,21 +242,16 @@ __global__ void __launch_bounds__(SCT) k_solve_flow_fwd(const int* __restrict__ 
         }
       }
     }
-    if (jmax > 1) {                           // hand the sums to the (row, quarter) lanes
-      __syncthreads();
-#pragma unroll
-      for (int c = 0; c < NR; c++) ys[g2 * SB + rl2][c] = acc2[c];
-      __syncthreads();
-#pragma unroll
-      for (int c = 0; c < NR; c++) acc[c] = ys[g * SB + rl][c];
-    }
-    // before the last wait: that block's L values, this row's quarter of
+    // before the last waits: those blocks' L values, this row's quarter of
     // Dinv_R (lower triangular, column-major) and the right-hand side
-    T ll[16], dv[16], w[NR];
-    const int cl = (jmax - 1) * SB + 16 * g;
+    T ll[TAIL][16], dv[16], w[NR];
 #pragma unroll
-    for (int q = 0; q < 16; q++)
-      ll[q] = (jmax > 0 && live && cl + q < d.n) ? Ar[(int64_t)(cl + q) * d.ld] : T(0);
+    for (int u = 0; u < TAIL; u++)
+#pragma unroll
+      for (int q = 0; q < 16; q++) {
+        const int c = (jbulk + u) * SB + 16 * g + q;
+        ll[u][q] = (jbulk + u < jmax && live && c < d.n) ? Ar[(int64_t)c * d.ld] : T(0);
+      }
     if (piv) {
       const T* D = Dv + dinv_off[f] + (int64_t)R * 2 * SB * SB;
 #pragma unroll
@@ -259,18 +260,30 @@ __global__ void __launch_bounds__(SCT) k_solve_flow_fwd(const int* __restrict__ 
       for (int c = 0; c < NR; c++)
         w[c] = (live && g == 0 && c < nrhs) ? X[dl[row0 + rl] + (int64_t)c * ldx] : T(0);
     }
-    if (jmax > 0) {
-      __syncthreads();                        // ys of the previous round is consumed
-      for (int idx = tid; idx < SB * nrhs; idx += SCT) {
-        const int r = idx % SB, c = idx / SB;
-        const int col = (jmax - 1) * SB + r;
-        ys[r][c] = col < d.n ? flow_value(Y + col + (int64_t)c * ldy, err) : T(0);
-      }
+    if (jbulk > 0) {                          // hand the sums to the (row, quarter) lanes
       __syncthreads();
 #pragma unroll
-      for (int q = 0; q < 16; q++)
+      for (int c = 0; c < NR; c++) ys[g2 * SB + rl2][c] = acc2[c];
+      __syncthreads();
 #pragma unroll
-        for (int c = 0; c < NR; c++) acc[c] = fma(ll[q], ys[16 * g + q][c], acc[c]);
+      for (int c = 0; c < NR; c++) acc[c] = ys[g * SB + rl][c];
+    }
+    if (jmax > 0) __syncthreads();            // ys of the previous round is consumed
+    // the last blocks, each in its own part of ys, as their values come up
+#pragma unroll
+    for (int u = 0; u < TAIL; u++) {
+      if (jbulk + u < jmax) {
+        for (int idx = tid; idx < SB * nrhs; idx += SCT) {
+          const int r = idx % SB, c = idx / SB;
+          const int col = (jbulk + u) * SB + r;
+          ys[u * SB + r][c] = col < d.n ? flow_value(Y + col + (int64_t)c * ldy, err) : T(0);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 16; q++)
+#pragma unroll
+          for (int c = 0; c < NR; c++) acc[c] = fma(ll[u][q], ys[u * SB + 16 * g + q][c], acc[c]);
+      }
     }
     // sum the four quarters of the row
 #pragma unroll
@@ -323,7 +336,7 @@ __global__ void __launch_bounds__(SCT) k_solve_flow_fwd(const int* __restrict__ 
 // quarter of Dinv_j^T and y_j in registers before the wait); then
 // x_j = Dinv_j^T (y_j - r) to X and Y and the flag.  The four lanes of a
 // column (tid & 3) split the rows.
-template <class T, int NR>
+template <class T, int NR, int TAIL>
 __global__ void __launch_bounds__(SCT) k_solve_flow_bwd(const int* __restrict__ flist,
                                                         const FrontDev* __restrict__ fr,
                                                         const T* __restrict__ F,
@@ -407,7 +420,7 @@ __global__ void __launch_bounds__(SCT) k_solve_flow_bwd(const int* __restrict__ 
       for (int s = 0; s < BR; s++)
         if (s * SB < nr) chunk(r0 + s * SB, min(SB, nr - s * SB), s * SB);
     }
-    for (int R = nb - 1; R > j + 1; R--) {              // solved pivot blocks below but the nearest
+    for (int R = nb - 1; R > j + TAIL; R--) {           // solved pivot blocks below but the nearest
       const int r0 = R * SB, nr = min(SB, d.n - r0);
       __syncthreads();
       if (tid == 0) flow_wait(fl + R, err, R - j - 1);
@@ -433,13 +446,16 @@ __global__ void __launch_bounds__(SCT) k_solve_flow_bwd(const int* __restrict__ 
 #pragma unroll
       for (int c = 0; c < NR; c++) acc[c] = (q == 0 && live) ? red[cl][c] : T(0);
     }
-    // before the last wait: block j + 1's L values, this column's quarter of
-    // Dinv_j^T (upper triangular, column-major) and y_j
-    const int rn = (j + 1) * SB, nn = j + 1 < nb ? min(SB, d.n - rn) : 0;
-    T ln[16], dt[16], v[NR];
+    // before the last waits: the L values of blocks j + TAIL .. j + 1, this
+    // column's quarter of Dinv_j^T (upper triangular, column-major) and y_j
+    T ln[TAIL][16], dt[16], v[NR];
 #pragma unroll
-    for (int rr = 0; rr < 16; rr++)
-      ln[rr] = (live && 16 * q + rr < nn) ? Lc[rn + 16 * q + rr] : T(0);
+    for (int u = 0; u < TAIL; u++)
+#pragma unroll
+      for (int rr = 0; rr < 16; rr++) {
+        const int r = (j + TAIL - u) * SB + 16 * q + rr;
+        ln[u][rr] = (live && r < d.n) ? Lc[r] : T(0);
+      }
     {
       const T* D = Dv + dinv_off[f] + (int64_t)j * 2 * SB * SB + SB * SB;
 #pragma unroll
@@ -448,17 +464,23 @@ __global__ void __launch_bounds__(SCT) k_solve_flow_bwd(const int* __restrict__ 
       for (int c = 0; c < NR; c++)
         v[c] = (live && q == 0 && c < nrhs) ? X[dl[col0 + cl] + (int64_t)c * ldx] : T(0);
     }
-    if (nn > 0) {
-      __syncthreads();                        // xs of the previous round is consumed
-      for (int idx = tid; idx < SB * nrhs; idx += SCT) {
-        const int r = idx % SB, c = idx / SB;
-        xs[r][c] = r < nn ? flow_value(Y + rn + r + (int64_t)c * ldy, err) : T(0);
+    __syncthreads();                          // xs of the previous round is consumed
+    // the nearest blocks, each in its own part of xs, as their values come up
+#pragma unroll
+    for (int u = 0; u < TAIL; u++) {
+      const int rn = (j + TAIL - u) * SB;
+      if (rn < d.n) {
+        for (int idx = tid; idx < SB * nrhs; idx += SCT) {
+          const int r = idx % SB, c = idx / SB;
+          xs[u * SB + r][c] = rn + r < d.n ? flow_value(Y + rn + r + (int64_t)c * ldy, err) : T(0);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int rr = 0; rr < 16; rr++)
+#pragma unroll
+          for (int c = 0; c < NR; c++)
+            acc[c] = fma(ln[u][rr], xs[u * SB + 16 * q + rr][c], acc[c]);
       }
-      __syncthreads();
-#pragma unroll
-      for (int rr = 0; rr < 16; rr++)
-#pragma unroll
-        for (int c = 0; c < NR; c++) acc[c] = fma(ln[rr], xs[16 * q + rr][c], acc[c]);
     }
 #pragma unroll
     for (int c = 0; c < NR; c++) {
@@ -550,7 +572,7 @@ __device__ __forceinline__ void stage_rhs(double* xs, int nr, int nrhs, Get&& ge
   }
 }
 
-template <int NT>
+template <int NT, int NEAR>
 __global__ void __launch_bounds__(SCT, 2)
     k_flow_fwd64(const int* __restrict__ flist, const FrontDev* __restrict__ fr,
                  const double* __restrict__ F, const int* __restrict__ dofs, double* X, int64_t ldx,
@@ -594,13 +616,23 @@ __global__ void __launch_bounds__(SCT, 2)
         return j * SB + r < d.n ? ldcg(Y + j * SB + r + (int64_t)c * ldy) : 0.0;
       };
     };
+    auto value = [&](int j) {
+      return [&, j](int r, int c) {
+        return j * SB + r < d.n ? flow_value(Y + j * SB + r + (int64_t)c * ldy, err) : 0.0;
+      };
+    };
     double a[16], an[16];
     if (jmax > 0) load(a, 0);
     for (int j = 0; j < jmax - 1; j++) {
-      if (tid == 0) flow_wait(fl + j, err, jmax - 1 - j);
-      __syncthreads();
-      stage_rhs<NT>(xs[j & 1], SB, nrhs, solved(j));
-      load(an, j + 1);                          // the next block in flight
+      if (NEAR > 1 && jmax - 1 - j < NEAR) {
+        load(an, j + 1);                        // the next block in flight
+        stage_rhs<NT>(xs[j & 1], SB, nrhs, value(j));
+      } else {
+        if (tid == 0) flow_wait(fl + j, err, jmax - 1 - j);
+        __syncthreads();
+        stage_rhs<NT>(xs[j & 1], SB, nrhs, solved(j));
+        load(an, j + 1);
+      }
       __syncthreads();
       mma_block<NT>(acc, a, xs[j & 1], rr, cc);
 #pragma unroll
@@ -623,9 +655,7 @@ __global__ void __launch_bounds__(SCT, 2)
     if (jmax > 0) {
       const int j = jmax - 1;
       __syncthreads();                          // xs of the round before the last is consumed
-      stage_rhs<NT>(xs[j & 1], SB, nrhs, [&](int r, int c) {
-        return j * SB + r < d.n ? flow_value(Y + j * SB + r + (int64_t)c * ldy, err) : 0.0;
-      });
+      stage_rhs<NT>(xs[j & 1], SB, nrhs, value(j));
       __syncthreads();
       mma_block<NT>(acc, a, xs[j & 1], rr, cc);
     }
@@ -673,7 +703,7 @@ __global__ void __launch_bounds__(SCT, 2)
 // steps of four rows 8 s + {0, 2, 4, 6} and {1, 3, 5, 7}).  Blocks from the last
 // one up: boundary rows from X, pivot rows from Y as their flags come up; the
 // block holding the last pivots may hold both.
-template <int NT>
+template <int NT, int NEAR>
 __global__ void __launch_bounds__(SCT, 2)
     k_flow_bwd64(const int* __restrict__ flist, const FrontDev* __restrict__ fr,
                  const double* __restrict__ F, const int* __restrict__ dofs, double* X, int64_t ldx,
@@ -716,14 +746,14 @@ __global__ void __launch_bounds__(SCT, 2)
           }
       }
     };
-    auto stage = [&](double* x, int R, bool last) {   // x(row, rhs) in the fragments' row order
+    auto stage = [&](double* x, int R, bool near) {   // x(row, rhs) in the fragments' row order
       const int r0 = R * SB, lo = R == j ? d.n : r0;
       for (int idx = tid; idx < SB * 8 * NT; idx += SCT) {
         const int r = idx & (SB - 1), c = idx / SB, g = r0 + r;
         double v = 0.0;
         if (g >= lo && g < d.N && c < nrhs)
           v = g >= d.n ? X[dl[g] + (int64_t)c * ldx]
-              : last   ? flow_value(Y + g + (int64_t)c * ldy, err)
+              : near   ? flow_value(Y + g + (int64_t)c * ldy, err)
                        : ldcg(Y + g + (int64_t)c * ldy);
         const int k = (r & ~7) + 4 * (r & 1) + ((r & 7) >> 1);
         x[(c >> 3) * SB * MS + k * MS + (c & 7)] = v;
@@ -734,12 +764,17 @@ __global__ void __launch_bounds__(SCT, 2)
     double a[16], an[16];
     if (Rlast < nbr) load(a, nbr - 1);
     for (int R = nbr - 1; R > Rlast; R--) {
-      if (R < nb) {
-        if (tid == 0) flow_wait(fl + R, err, R - j - 1);
-        __syncthreads();
+      if (NEAR > 1 && R - j <= NEAR) {
+        load(an, R - 1);                        // the next block in flight
+        stage(xs[R & 1], R, true);
+      } else {
+        if (R < nb) {
+          if (tid == 0) flow_wait(fl + R, err, R - j - 1);
+          __syncthreads();
+        }
+        stage(xs[R & 1], R, false);
+        load(an, R - 1);
       }
-      stage(xs[R & 1], R, false);
-      load(an, R - 1);
       __syncthreads();
       mma_block<NT>(acc, a, xs[R & 1], rr, cc);
 #pragma unroll
@@ -806,18 +841,18 @@ size_t flag_bytes(int nflags) { return ((size_t)std::max(1, nflags) * sizeof(int
 
 // Kernels of a direction and bound of the right-hand-side count: the scalar
 // form in FP32, the tensor-core form in FP64.
-template <class T, int NR>
+template <class T, int NR, int TAIL>
 struct FlowKernels {
-  static const void* fwd() { return (const void*)k_solve_flow_fwd<T, NR>; }
-  static const void* bwd() { return (const void*)k_solve_flow_bwd<T, NR>; }
+  static const void* fwd() { return (const void*)k_solve_flow_fwd<T, NR, TAIL>; }
+  static const void* bwd() { return (const void*)k_solve_flow_bwd<T, NR, TAIL>; }
 };
-template <int NR>
-struct FlowKernels<double, NR> {
-  static const void* fwd() { return (const void*)k_flow_fwd64<NR / 8>; }
-  static const void* bwd() { return (const void*)k_flow_bwd64<NR / 8>; }
+template <int NR, int TAIL>
+struct FlowKernels<double, NR, TAIL> {
+  static const void* fwd() { return (const void*)k_flow_fwd64<NR / 8, TAIL>; }
+  static const void* bwd() { return (const void*)k_flow_bwd64<NR / 8, TAIL>; }
 };
 
-template <class T, int NR>
+template <class T, int NR, int TAIL>
 cudaError_t launchFlowSolve(bool fwd, const int* flist, const FrontDev* fr, const T* F,
                             const int* dofs, T* X, int64_t ldx, int nrhs, T* W,
                             const int64_t* woff, const T* Dv, const int64_t* dinv_off,
@@ -828,7 +863,7 @@ cudaError_t launchFlowSolve(bool fwd, const int* flist, const FrontDev* fr, cons
   T* Y = reinterpret_cast<T*>(reinterpret_cast<unsigned char*>(flags) + fb);
   cudaError_t me = cudaMemsetAsync(flags, 0xff, fb + (size_t)nflags * SB * nrhs * sizeof(T), st);
   if (me != cudaSuccess) return me;
-  using K = FlowKernels<T, NR>;
+  using K = FlowKernels<T, NR, TAIL>;
   static const int gf = flowGrid(K::fwd());   // thread-safe one-time set-up
   static const int gb = flowGrid(K::bwd());
   const int grid = std::max(1, std::min(fwd ? gf : gb, ntasks));
@@ -876,19 +911,26 @@ cudaError_t launch_solve_flow(bool forward, const int* flist, const FrontDev* fr
                               const int* dofs, T* X, int64_t ldx, int nrhs, T* W,
                               const int64_t* woff, const T* Dv, const int64_t* dinv_off,
                               const int* tasks, int ntasks, const int* flagoff, int* flags,
-                              int nflags, DevError* err, cudaStream_t st) {
+                              int nflags, bool chain, DevError* err, cudaStream_t st) {
   if (ntasks <= 0) return cudaSuccess;
   if (nrhs > 16) return cudaErrorInvalidValue;
   const int2* tk = reinterpret_cast<const int2*>(tasks);
-#define MFGPU_FLOW(NRV)                                                                           \
-  return launchFlowSolve<T, NRV>(forward, flist, fr, F, dofs, X, ldx, nrhs, W, woff, Dv, dinv_off, \
-                                 tk, ntasks, flagoff, flags, nflags, err, st)
+#define MFGPU_FLOW(NRV, TAIL)                                                                     \
+  return launchFlowSolve<T, NRV, TAIL>(forward, flist, fr, F, dofs, X, ldx, nrhs, W, woff, Dv,      \
+                                       dinv_off, tk, ntasks, flagoff, flags, nflags, err, st)
   if constexpr (sizeof(T) == sizeof(float)) {
-    if (nrhs == 1) MFGPU_FLOW(1);
-    if (nrhs <= 4) MFGPU_FLOW(4);
+    if (nrhs == 1 && chain) MFGPU_FLOW(1, kChainTail);
+    if (nrhs == 1) MFGPU_FLOW(1, 1);
+    if (nrhs <= 4 && chain) MFGPU_FLOW(4, kChainTail);
+    if (nrhs <= 4) MFGPU_FLOW(4, 1);
+    if (nrhs <= 8) MFGPU_FLOW(8, 1);
+    MFGPU_FLOW(16, 1);
+  } else {
+    if (nrhs <= 8 && chain) MFGPU_FLOW(8, kChainTail);
+    if (nrhs <= 8) MFGPU_FLOW(8, 1);
+    if (chain) MFGPU_FLOW(16, kChainTail);
+    MFGPU_FLOW(16, 1);
   }
-  if (nrhs <= 8) MFGPU_FLOW(8);
-  MFGPU_FLOW(16);
 #undef MFGPU_FLOW
 }
 
@@ -908,13 +950,13 @@ void launch_diag_inv(const int* flist, int nf, int maxn, const FrontDev* fr, con
 template cudaError_t launch_solve_flow<double>(bool, const int*, const FrontDev*, const double*,
                                                const int*, double*, int64_t, int, double*,
                                                const int64_t*, const double*, const int64_t*,
-                                               const int*, int, const int*, int*, int, DevError*,
-                                               cudaStream_t);
+                                               const int*, int, const int*, int*, int, bool,
+                                               DevError*, cudaStream_t);
 template cudaError_t launch_solve_flow<float>(bool, const int*, const FrontDev*, const float*,
                                               const int*, float*, int64_t, int, float*,
                                               const int64_t*, const float*, const int64_t*,
-                                              const int*, int, const int*, int*, int, DevError*,
-                                              cudaStream_t);
+                                              const int*, int, const int*, int*, int, bool,
+                                              DevError*, cudaStream_t);
 template void launch_diag_inv<double>(const int*, int, int, const FrontDev*, const double*, double*,
                                       const int64_t*, cudaStream_t);
 template void launch_diag_inv<float>(const int*, int, int, const FrontDev*, const float*, float*,

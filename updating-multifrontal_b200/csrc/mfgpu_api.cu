@@ -1398,7 +1398,8 @@ struct mfgpu_handle {
       ck(mfgpu::launch_solve_flow<T>(forward, big, d_fr, F, d_dofs, X, ldx, nrhs, W, d_woff,
                                      (const T*)d_Dinv, d_dinv_off,
                                      d_flow + (forward ? q.fwd : q.bwd), forward ? q.nfwd : q.nbwd,
-                                     d_flow + q.flagoff, d_flags, q.nflags, d_err, stream),
+                                     d_flow + q.flagoff, d_flags, q.nflags,
+                                     (q.list < 0 ? nf : nf - q.nrest) == 1, d_err, stream),
          forward ? "launch cooperative forward sweep (k_solve_flow_fwd)"
                  : "launch cooperative backward sweep (k_solve_flow_bwd)");
       if (q.list < 0) return;
