@@ -44,7 +44,7 @@ namespace {
 
 constexpr int SB = 64;          // diagonal block of the substitution
 constexpr int SCT = 256;        // threads per CTA
-constexpr int kMaxSolveCoopFronts = 256;
+constexpr int kMaxSolveCoopFronts = 1024;
 
 __host__ __device__ __forceinline__ int cdiv(int a, int b) { return (a + b - 1) / b; }
 

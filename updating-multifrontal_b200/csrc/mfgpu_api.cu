@@ -382,6 +382,7 @@ struct mfgpu_handle {
     int nfwd = 0, nbwd = 0, nflags = 0;
     int64_t list = -1, rest = -1;   // -1: every front of the level
     int nrest = 0, restMaxN = 0;
+    int minRhs = 1;                 // fewest right-hand sides for the flow sweeps
   };
   std::vector<FlowLevel> flow;
   int* d_flow = nullptr;       // shared with serving-loop views
@@ -1356,23 +1357,36 @@ struct mfgpu_handle {
   // Forward / backward sweeps of the factorization in precision T, in place on
   // X (n x nrhs, ld ldx, nrhs <= 16) with per-front workspace W
   // (src/DE/mf2d.cpp:976-1054).
-  bool coopSweep(int ell) const {
-    return solveCoopMinN > 0 && lvMaxN[ell] >= solveCoopMinN &&
-           S->lv[ell].nbox <= mfgpu::solve_coop_max_fronts();
+  // Levels whose sweeps are ordered by flags over all SMs, by their largest front
+  // (M = solveCoopMinN rows) and count; the least number of right-hand sides, or 0.
+  //   M rows, up to 256 fronts: the level is bound by its fronts' chains;
+  //   M / 4 rows, fewer fronts than SMs: one CTA a front leaves SMs idle (64
+  //     fronts of 761 x 253, FP64, 4 right-hand sides: 175 us against 77; the 24
+  //     roots of a batch, up to 509: 142 against 58);
+  //   FP64, M / 2 rows, up to 1024 fronts, more than four right-hand sides: the
+  //     tensor cores take them eight at a time (512 fronts of 637 x 343, 16:
+  //     1830 us against 748; with one, 314 against 407).
+  int flowMinRhs(int ell) const {
+    const int N = lvMaxN[ell], nf = S->lv[ell].nbox, M = solveCoopMinN;
+    if (M <= 0) return 0;
+    if (N >= M && nf <= 256) return 1;
+    if (N >= M / 4 && nf < 148) return 1;
+    if (!mixed && N >= M / 2 && nf <= mfgpu::solve_coop_max_fronts()) return 5;
+    return 0;
   }
-  // The large fronts of a level too numerous for coopSweep (ragged grids leave
+  // The large fronts of a level too numerous for that (ragged grids leave
   // their remainder to the last boxes, so leaf levels of thousands of small
   // fronts hold a few large ones); empty when they are too many as well.
   // One CTA's sweep of such a front holds up the level: 2D 700 x 333 mixed (4096
   // leaves, one of 1348 x 1260), factor + solve 6.38 -> 5.66 ms.
   std::vector<int> largeFronts(int ell) const {
     std::vector<int> big;
-    if (solveCoopMinN <= 0 || lvMaxN[ell] < solveCoopMinN || coopSweep(ell) ||
+    if (solveCoopMinN <= 0 || lvMaxN[ell] < solveCoopMinN || flowMinRhs(ell) == 1 ||
         S->lv[ell].nbox > 32768)   // (a launch of k_diag_inv covers a level's fronts)
       return big;
     for (int b = 0; b < S->lv[ell].nbox; b++)
       if (S->fronts[S->lv[ell].front0 + b].N >= solveCoopMinN) big.push_back(S->lv[ell].front0 + b);
-    if ((int)big.size() > mfgpu::solve_coop_max_fronts()) big.clear();
+    if (big.size() > 256) big.clear();
     return big;
   }
   bool hasFlow(int ell) const { return ell < (int)flow.size() && flow[ell].nfwd > 0; }
@@ -1392,7 +1406,7 @@ struct mfgpu_handle {
       return;
     }
     int maxN = lvMaxN[ell];
-    if (hasFlow(ell)) {
+    if (hasFlow(ell) && nrhs >= flow[ell].minRhs) {
       const FlowLevel& q = flow[ell];
       const int* big = q.list < 0 ? fl : d_flow + q.list;
       ck(mfgpu::launch_solve_flow<T>(forward, big, d_fr, F, d_dofs, X, ldx, nrhs, W, d_woff,
@@ -1435,7 +1449,7 @@ struct mfgpu_handle {
       ck(cudaGetLastError(), "launch separator gather (k_sep_gather)");
     }
     vmark(true, 0);
-    if (lu || coopSweep(0) || s.lv[0].nbox > 1) {   // several roots (a batch), LU: generic sweeps
+    if (lu || hasFlow(0) || s.lv[0].nbox > 1) {   // several roots (a batch), LU: generic sweeps
       sweepLevel<T>(true, 0, X, ldx, nrhs, W);
       sweepLevel<T>(false, 0, X, ldx, nrhs, W);
     } else {
@@ -1892,7 +1906,7 @@ int createFrom(std::unique_ptr<Schedule> sched, int n, const int* row_ptr, const
       for (int ell = 0; ell < s.levels; ell++) {
         big[ell] = H.largeFronts(ell);
         for (int f : big[ell]) flowFront[f] = 1;
-        for (int b = 0; b < s.lv[ell].nbox && H.coopSweep(ell); b++)
+        for (int b = 0; b < s.lv[ell].nbox && big[ell].empty() && H.flowMinRhs(ell); b++)
           flowFront[s.lv[ell].front0 + b] = 1;
       }
       for (size_t i = 0; i < s.fronts.size(); i++)
@@ -1907,7 +1921,7 @@ int createFrom(std::unique_ptr<Schedule> sched, int n, const int* row_ptr, const
       std::vector<int> tab;
       H.flow.assign(s.levels, mfgpu_handle::FlowLevel());
       for (int ell = 0; ell < s.levels; ell++) {
-        if (!H.coopSweep(ell) && big[ell].empty()) continue;
+        if (!H.flowMinRhs(ell) && big[ell].empty()) continue;
         std::vector<int> nn, NN, fw, bw, fo, rest;
         mfgpu_handle::FlowLevel& q = H.flow[ell];
         for (int b = 0; b < s.lv[ell].nbox; b++) {
@@ -1921,6 +1935,7 @@ int createFrom(std::unique_ptr<Schedule> sched, int n, const int* row_ptr, const
           }
         }
         mfgpu::flow_tasks(nn, NN, fw, bw, fo);
+        q.minRhs = big[ell].empty() ? H.flowMinRhs(ell) : 1;
         if (!big[ell].empty()) {
           q.list = (int64_t)tab.size();
           tab.insert(tab.end(), big[ell].begin(), big[ell].end());
