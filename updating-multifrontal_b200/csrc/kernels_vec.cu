@@ -183,8 +183,9 @@ __global__ void k_pcg_p(double* __restrict__ p, const double* __restrict__ z, in
   if (i >= n) return;
   const int g = seg_of(seg_row, nseg, i) + nseg * c;
   if (!active[g]) return;
-  const double b = first ? 0.0 : rz_new[g] / rz_old[g];
-  p[i + c * ld] = fma(b, p[i + c * ld], z[i + c * ld]);
+  const double zi = z[i + c * ld];
+  // (the first iteration's p is fresh memory, which may hold NaNs: 0 * p is no zero)
+  p[i + c * ld] = first ? zi : fma(rz_new[g] / rz_old[g], p[i + c * ld], zi);
 }
 
 inline dim3 vgrid(int n, int nrhs) { return dim3((n + VT - 1) / VT, nrhs); }
