@@ -110,29 +110,22 @@ struct Plan {
   int maxRows = 0;                // most block rows of any tile launch
   int nfronts = 0;
   double flops = 0;
-  // device copies
+  // device copies, all in one buffer (one allocation, one copy per upload: a
+  // localized update uploads its plan on every call)
   Task* d_tasks = nullptr;
   int2* d_tiles = nullptr;
   int* d_ids = nullptr;
   int* d_cpref = nullptr;
   int* d_ttask = nullptr;
   int* d_trow = nullptr;
-  size_t cap_tasks = 0, cap_tiles = 0, cap_ids = 0, cap_cpref = 0, cap_ttask = 0, cap_trow = 0;
+  unsigned char* d_buf = nullptr;
+  size_t cap = 0;
+  std::vector<unsigned char> h_buf;
 
   void release() {
-    cudaFree(d_tasks);
-    cudaFree(d_tiles);
-    cudaFree(d_ids);
-    cudaFree(d_cpref);
-    cudaFree(d_ttask);
-    cudaFree(d_trow);
-    d_tasks = nullptr;
-    d_tiles = nullptr;
-    d_ids = nullptr;
-    d_cpref = nullptr;
-    d_ttask = nullptr;
-    d_trow = nullptr;
-    cap_tasks = cap_tiles = cap_ids = cap_cpref = cap_ttask = cap_trow = 0;
+    cudaFree(d_buf);
+    d_buf = nullptr;
+    cap = 0;
   }
 
   void clear(int levels) {
@@ -218,43 +211,40 @@ struct Plan {
   }
 
   void upload(cudaStream_t st) {
-    auto grow = [](auto*& p, size_t& cap, size_t need, const char* what) {
-      if (need <= cap) return;
-      cudaFree(p);
-      p = nullptr;
-      using T = std::remove_reference_t<decltype(*p)>;
-      size_t c = std::max(need, cap * 2);
-      p = dalloc<T>(c, what);
-      cap = c;
+    size_t need = 0;
+    auto place = [&](const auto& v) {   // 16-byte aligned offset of v's copy
+      const size_t at = need;
+      need = (need + v.size() * sizeof(v[0]) + 15) & ~(size_t)15;
+      return at;
     };
-    grow(d_tasks, cap_tasks, tasks.size(), "alloc plan tasks");
-    grow(d_tiles, cap_tiles, tiles.size(), "alloc plan tiles");
-    grow(d_ids, cap_ids, ids.size(), "alloc plan ids");
-    grow(d_cpref, cap_cpref, cpref.size(), "alloc plan phase prefixes");
-    grow(d_ttask, cap_ttask, ttask.size(), "alloc plan tile tasks");
-    grow(d_trow, cap_trow, trow.size(), "alloc plan block rows");
-    if (!tasks.empty())
-      ck(cudaMemcpyAsync(d_tasks, tasks.data(), tasks.size() * sizeof(Task), cudaMemcpyHostToDevice, st),
-         "upload tasks");
-    if (!tiles.empty())
-      ck(cudaMemcpyAsync(d_tiles, tiles.data(), tiles.size() * sizeof(int2), cudaMemcpyHostToDevice,
-                         st),
-         "upload tiles");
-    if (!ids.empty())
-      ck(cudaMemcpyAsync(d_ids, ids.data(), ids.size() * sizeof(int), cudaMemcpyHostToDevice, st),
-         "upload ids");
-    if (!cpref.empty())
-      ck(cudaMemcpyAsync(d_cpref, cpref.data(), cpref.size() * sizeof(int), cudaMemcpyHostToDevice,
-                         st),
-         "upload phase prefixes");
-    if (!ttask.empty())
-      ck(cudaMemcpyAsync(d_ttask, ttask.data(), ttask.size() * sizeof(int), cudaMemcpyHostToDevice,
-                         st),
-         "upload tile tasks");
-    if (!trow.empty())
-      ck(cudaMemcpyAsync(d_trow, trow.data(), trow.size() * sizeof(int), cudaMemcpyHostToDevice, st),
-         "upload block rows");
-    // host vectors must outlive the async copies
+    const size_t o[6] = {place(tasks), place(tiles), place(ids), place(cpref), place(ttask), place(trow)};
+    h_buf.resize(need);
+    auto put = [&](size_t at, const auto& v) {
+      if (!v.empty()) std::memcpy(h_buf.data() + at, v.data(), v.size() * sizeof(v[0]));
+    };
+    put(o[0], tasks);
+    put(o[1], tiles);
+    put(o[2], ids);
+    put(o[3], cpref);
+    put(o[4], ttask);
+    put(o[5], trow);
+    if (need > cap) {
+      cudaFree(d_buf);
+      d_buf = nullptr;
+      const size_t c = std::max(need, cap * 2);
+      cap = 0;
+      d_buf = dalloc<unsigned char>(c, "alloc plan");
+      cap = c;
+    }
+    if (need > 0)
+      ck(cudaMemcpyAsync(d_buf, h_buf.data(), need, cudaMemcpyHostToDevice, st), "upload plan");
+    d_tasks = reinterpret_cast<Task*>(d_buf + o[0]);
+    d_tiles = reinterpret_cast<int2*>(d_buf + o[1]);
+    d_ids = reinterpret_cast<int*>(d_buf + o[2]);
+    d_cpref = reinterpret_cast<int*>(d_buf + o[3]);
+    d_ttask = reinterpret_cast<int*>(d_buf + o[4]);
+    d_trow = reinterpret_cast<int*>(d_buf + o[5]);
+    // the host buffer must outlive the async copy
     ck(cudaStreamSynchronize(st), "plan upload");
   }
 };
