@@ -12,7 +12,7 @@ log-uniform in [0.1, 100] from a fixed seed, leaf parameter 4 (leaf boxes of
   3. a solve with the updated factorization,
 in mixed precision: FP32 factorization of the diagonally scaled matrix with
 the Schur-complement updates of the large-front levels on the tensor cores
-(three-term TF32 products), then conjugate gradients in FP64 preconditioned by
+(three-term FP16 products), then conjugate gradients in FP64 preconditioned by
 it until ||b - A x|| / ||b|| <= 1e-10.  `value` is the algorithmic TFLOP/s of
 that step: Cholesky-form flops sum(n^3/3 + n^2 m + n m^2) over the factored
 fronts, the same over the fronts the update refactors, and 2(n^2 + 2nm) per
@@ -274,7 +274,7 @@ def pct(v, q):
 
 def dtype_of(precision):
     return "f64" if precision == "fp64" else \
-        "f32 factor (tf32x3 tensor-core Schur updates) + f64 residual/refinement"
+        "f32 factor (three-term fp16 tensor-core Schur updates) + f64 residual/refinement"
 
 
 def config_of(w, args, precision):
@@ -874,7 +874,7 @@ def main():
 
 
 # profiling class -> the kernel it times
-KERNEL_OF = {"front": "k_front_small", "coop": "k_level_coop", "tc": "k_trail_tc",
+KERNEL_OF = {"front": "k_front_small", "coop": "k_front_tiles", "tc": "k_trail_tc",
              "assemble": "k_tasks", "solve": "k_solve_*", "apply": "k_apply_*",
              "potrf": "k_potrf", "trsm": "k_trsm", "syrk": "k_syrk"}
 
@@ -886,14 +886,16 @@ def roofline(torch, dom, P, peaks, peak_src, args):
               "traffic": traffic_for(kern, args.workload, args.precision)}
     ach = P["flops"] / (P["ms"] * 1e-3) / 1e12
     if dom == "tc":
-        split = {"1": 1, "tf32": 1, "bf16": 1}.get(os.environ.get("MFGPU_TC_SPLIT", "3"), 3)
-        pk = float(peaks["bf16_tflops"]) / 2.0
+        mode = os.environ.get("MFGPU_TC_SPLIT", "3")
+        split, tf32 = (1, mode in ("1", "tf32")) if mode in ("1", "tf32", "bf16") else (3, False)
+        pk = float(peaks["bf16_tflops"]) / (2.0 if tf32 else 1.0)
         return dict(common, bound="tensor", achieved=ach, peak=pk, unit="TFLOP/s", frac=ach / pk,
                     achieved_executed=ach * split,
-                    peak_source=f"{peak_src} bf16_tflops / 2 (MEASURED_PEAKS.json, else the "
-                                "pool's fallback): the dense TF32 rate is half the BF16 rate; "
-                                "achieved counts the algorithmic flops once, the kernel executes "
-                                f"{split} TF32 products per flop")
+                    peak_source=f"{peak_src} bf16_tflops{' / 2 (TF32)' if tf32 else ''} "
+                                "(MEASURED_PEAKS.json, else the pool's fallback); achieved counts "
+                                "the algorithmic flops once, the kernel executes "
+                                f"{split} 16-bit products per flop" if not tf32 else
+                                f"{peak_src} bf16_tflops / 2: the dense TF32 rate")
     if dom in ("potrf", "trsm", "syrk", "front", "coop"):
         dt, nm = (torch.float32, "SGEMM (float32") if args.precision == "mixed" else \
             (torch.float64, "DGEMM (float64")

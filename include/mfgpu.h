@@ -239,8 +239,8 @@ int mfgpu_graphs(const mfgpu_handle* h, int* factor_graph, int* sweep_graphs);
 
 /* Failure handling (no reference counterpart: the reference has no device
  * waits, and its LAPACK failures abort through assert, include/LinAlg/dense.hpp:187).
- * Every device wait of this library is bounded: the grid barriers of the
- * cooperative kernels give up after 2^25 polls, the tensor-core pipeline's
+ * Every device wait of this library is bounded: the grid barriers, ready words
+ * and flags of the kernels give up after 2^25 polls, the tensor-core pipeline's
  * mbarrier waits after 2^24; a wait that gives up makes the call return
  * MFGPU_ERR_TIMEOUT, and the handle stays usable (the next call starts from a
  * clean error word and barrier counter; refactor before solving again if the
@@ -258,7 +258,7 @@ void mfgpu_inject_alloc_failure(long long after);
 /* Factor serialisation (no counterpart in the reference, whose factorization
  * lives in process memory only; use: restart a serving loop without
  * refactoring its base).  mfgpu_save writes a factored handle's state - front
- * and separator arenas, CSR values, the mixed path's scaling, the cooperative
+ * and separator arenas, CSR values, the mixed path's scaling, the flag-ordered
  * sweeps' block inverses - to `path` with a header describing the problem and
  * a checksum of the payload.  mfgpu_load restores it into a handle created
  * for the same problem (same schedule sizes, precision and sparsity pattern);
@@ -273,7 +273,7 @@ int mfgpu_load(mfgpu_handle* h, const char* path);
 /* Autotuner (no counterpart in the reference): a full factorization, like
  * mfgpu_factor, that also picks each tree level's kernel by timing.  For every
  * level with more than one eligible kernel - one CTA per front
- * (MFGPU_LEVEL_FUSED), the cooperative level kernel (MFGPU_LEVEL_COOP),
+ * (MFGPU_LEVEL_FUSED), tiles over all SMs (MFGPU_LEVEL_COOP),
  * panel-by-panel launches without grid barriers (MFGPU_LEVEL_PANEL), the
  * tensor-core update (MFGPU_LEVEL_TC, mixed precision) - each candidate runs
  * `reps` times on freshly assembled fronts and the fastest is kept; later
@@ -299,7 +299,7 @@ enum mfgpu_kernel_class {
   MFGPU_KC_APPLY = 5,     /* factored-operator application                   */
   MFGPU_KC_FRONT = 6,     /* fused partial factorization, one CTA per front  */
   MFGPU_KC_COOP = 7,      /* per-level partial factorization on CUDA cores:
-                             cooperative kernel, panel kernels, and the
+                             tiles, panel kernels, and the
                              tensor-core levels' sub-panels                   */
   MFGPU_KC_TC = 8,        /* tensor-core trailing updates (mixed path)       */
   MFGPU_KC_COUNT = 9

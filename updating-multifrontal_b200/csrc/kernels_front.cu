@@ -1,9 +1,9 @@
 // Front kernels for both precisions (T = double for the FP64 path, T = float
 // for the mixed-precision factorization): front / separator assembly from
-// task tables, partial Cholesky of every front of a level (fused per front, or
-// one cooperative launch per level), and the solve / apply sweeps.  FP64 tiles
-// use the FP64 tensor cores (mma.sync m8n8k4); FP32 tiles use CUDA-core FMAs
-// with the same fragment layout.
+// task tables, partial Cholesky of every front of a level fused per front (or in
+// one cooperative launch, FP32 sub-panels only), the separator gather of the
+// sweeps and the apply of LU fronts.  FP64 tiles use the FP64 tensor cores
+// (mma.sync m8n8k4); FP32 tiles use CUDA-core FMAs with the same fragment layout.
 //
 // Fronts are column-major with leading dimension ld; only the lower triangle
 // is read or written.  After the partial factorization of a front with n

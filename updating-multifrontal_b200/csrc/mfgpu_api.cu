@@ -1133,7 +1133,7 @@ struct mfgpu_handle {
   // sub-panel of w = L.coopOuter columns at a time, the tensor cores updating
   // the panel's remaining columns after each; w = 512: no sub-panels.)  Tiles
   // against sub-panels of 128 columns (a diagonal-block, a panel-solve, a pack
-  // and an update launch each): PNPN.  Profile attribution: the tensor-core
+  // and an update launch each): 3D 95^3 step 163 -> 144 ms.  Profile attribution: the tensor-core
   // updates' algorithmic flops go to MFGPU_KC_TC, the rest of the level's flops
   // to MFGPU_KC_COOP.
   void runTensorLevel(const Plan& P, const Plan::Level& L, double level_flops, int ell) {
