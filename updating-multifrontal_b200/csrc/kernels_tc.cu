@@ -36,9 +36,20 @@
 //             SPLIT = 2:  acc += a b^T in BF16 (kind::f16, K = 16)
 //         and hands stages back to the producer with tcgen05.commit;
 //       - eight epilogue warps (two per accumulator lane quarter, 128 columns
-//         each, 32 at a time) read the accumulator with tcgen05.ld and
-//         subtract it from C in place; the first 32 values of C are loaded
-//         before the accumulator is ready.
+//         each, 16 at a time) read the accumulator with tcgen05.ld and
+//         subtract it from C in place; the first 16 values of C are loaded
+//         before the accumulator is ready, each later 16 while the ones before
+//         them are subtracted and stored.
+// What bounds it is the epilogue, C read and written once per 512 columns of
+// products: with C neither read nor written the products alone run at 1,658
+// TFLOP/s executed (a front of N = 27,000, the full FP16 rate), without its
+// loads at 1,449, without its stores at 1,195.  Hence the loads always in flight
+// (one front, w = 512): 32 loaded, then 32 stored, 1,050 TFLOP/s; two buffers of
+// 16 1,270 (N = 12,000: 1,068 -> 1,239); three of 16 988 and two of 32 589, which
+// spill (168 registers a thread with ten warps); L2 prefetches of the next tile
+// with 32 in turn 1,149; red.global.add in place of loads and stores 1,159.  A
+// CTA pair sharing B (cta_group::2, 256 x 256 tiles) reads a third less, but
+// both CTAs' epilogues then gate one accumulator: 776.
 // A 256-column tile reads 25% fewer operand bytes per product than a 128 x 128
 // one, and 48 KB stages keep three in flight.  MN-major TF32 operands would let
 // the tensor core read the column-major front directly, but they read back as
@@ -86,6 +97,7 @@ constexpr int NACC = 2;                    // tensor-memory accumulators
 constexpr int MMA_WARP = 1;                // warp 0 produces, warp 1 issues the MMAs
 constexpr int EPI_WARP0 = 2;               // warps 2..9 run the epilogue
 constexpr int NEPI = 8;
+constexpr int CW = 16;                     // columns of C per epilogue step
 constexpr int TCT = (EPI_WARP0 + NEPI) * 32;   // 320 threads
 constexpr int IMG = TM * TK * 4;           // one image of 128 rows x 64 bytes, 8 KB
 constexpr int STAGE_BYTES = 6 * IMG;       // a_hi, a_lo, b_hi (2 blocks), b_lo (2 blocks)
@@ -589,7 +601,7 @@ __global__ void __launch_bounds__(TCT, 1) k_trail_tc(const int* __restrict__ fli
   } else {
     // ---- epilogue: C(tile) -= acc; warp w reads accumulator lanes
     // 32 (w % 4) .. +31 (the lane quarter it may access), columns 128 h .. +127,
-    // 32 at a time ----
+    // 16 at a time ----
     const int quarter = warp & 3, half = (warp - EPI_WARP0) >> 2;
     uint32_t tl = 0;
     for (int tile = blockIdx.x; tile < total && !__shfl_sync(0xffffffffu, abort_flag, 0);
@@ -599,9 +611,7 @@ __global__ void __launch_bounds__(TCT, 1) k_trail_tc(const int* __restrict__ fli
       const int row = ti.r0 + quarter * 32 + lane, cb = ti.c0 + half * (TN / 2);
       const bool live = row < ti.N;
       float* p = ti.A + row + (int64_t)cb * ti.ld;
-      // entry j of the row is live when cb + j <= min(row, cmax - 1); the first
-      // 32 values are loaded while the tile's products are still being
-      // accumulated, each later 32 once the previous ones are stored
+      // entry j of the row is live when cb + j <= min(row, cmax - 1)
       const int jmax = live ? min(row, ti.cmax - 1) - cb : -1;
       const uint32_t src = tmem + b * TN + half * (TN / 2) + ((uint32_t)(quarter * 32) << 16);
       // FP16 parts: the accumulator holds r_i r_j times the product
@@ -609,38 +619,34 @@ __global__ void __launch_bounds__(TCT, 1) k_trail_tc(const int* __restrict__ fli
       const float* rs = rscale ? rscale + ti.rs_off : nullptr;
       float ir = 1.0f;
       if (SPLIT == 3) ir = rs ? (live ? 1.0f / rs[dl[row]] : 0.0f) : 1.0f / kPlainScale;
-      bool ok = true;
-#pragma unroll 1
-      for (int h2 = 0; h2 < TN / 64; h2++) {
-        float cv[32], ic = 1.0f;
-        if (SPLIT == 3) {
-          const int col = cb + 32 * h2 + lane;
-          ic = rs ? (col < ti.N ? 1.0f / rs[dl[col]] : 0.0f) : 1.0f / kPlainScale;
+      float ic[TN / 64];   // lane l of ic[e]: column 32 e + l
+#pragma unroll
+      for (int e = 0; e < TN / 64; e++) {
+        const int col = cb + 32 * e + lane;
+        ic[e] = SPLIT != 3 ? 1.0f : rs ? (col < ti.N ? 1.0f / rs[dl[col]] : 0.0f) : 1.0f / kPlainScale;
+      }
+      float cv[2][CW];
+      const float* q = p;
+#pragma unroll
+      for (int j = 0; j < CW; j++, q += ti.ld) cv[0][j] = j <= jmax ? __ldcg(q) : 0.0f;
+      if (!mbar_wait_warp(&acc_full[b], (tl / NACC) & 1, &abort_flag, lim)) break;
+      tc_fence_after();
+#pragma unroll
+      for (int h = 0; h < TN / 2 / CW; h++) {
+        if (h + 1 < TN / 2 / CW) {
+#pragma unroll
+          for (int j = 0; j < CW; j++, q += ti.ld)
+            cv[(h + 1) & 1][j] = CW * (h + 1) + j <= jmax ? __ldcg(q) : 0.0f;
         }
-        const float* q = p + (int64_t)(32 * h2) * ti.ld;
+        uint32_t v[CW];
+        tmem_ld16(src + CW * h, v);
 #pragma unroll
-        for (int j = 0; j < 32; j++, q += ti.ld) cv[j] = 32 * h2 + j <= jmax ? *q : 0.0f;
-        if (h2 == 0) {
-          if (!mbar_wait_warp(&acc_full[b], (tl / NACC) & 1, &abort_flag, lim)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-        }
-        float* wp = p + (int64_t)(32 * h2) * ti.ld;
-#pragma unroll
-        for (int qb = 0; qb < 2; qb++) {
-          uint32_t v[16];
-          tmem_ld16(src + 32 * h2 + 16 * qb, v);
-#pragma unroll
-          for (int j = 0; j < 16; j++, wp += ti.ld) {
-            const float inv = SPLIT == 3 ? ir * __shfl_sync(0xffffffffu, ic, 16 * qb + j) : 1.0f;
-            if (32 * h2 + 16 * qb + j <= jmax)
-              *wp = fmaf(-inv, __uint_as_float(v[j]), cv[16 * qb + j]);
-          }
+        for (int j = 0; j < CW; j++, p += ti.ld) {
+          const int c = CW * h + j;
+          const float inv = SPLIT == 3 ? ir * __shfl_sync(0xffffffffu, ic[c / 32], c % 32) : 1.0f;
+          if (c <= jmax) *p = fmaf(-inv, __uint_as_float(v[j]), cv[h & 1][j]);
         }
       }
-      if (!ok) break;
       tc_fence_before();
       mbar_arrive(&acc_empty[b]);
     }
