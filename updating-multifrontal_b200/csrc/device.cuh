@@ -114,8 +114,7 @@ void launch_tasks(const Task* tasks, const int2* tiles, int64_t ntiles, bool sta
                   T* seps, const int* rp, const int* ci, const double* va, const int* dofs,
                   const double* scale, cudaStream_t st);
 
-// Stepped FP64 path (one launch per panel step and kernel), kept for levels a
-// cooperative launch cannot take.
+// Stepped FP64 path (one launch per panel step and kernel; MFGPU_STEPPED=1).
 void launch_potrf(const int* flist, int nf, const FrontDev* fr, double* F, int k, DevError* err,
                   cudaStream_t st);
 void launch_trsm(const int* flist, int nf, const FrontDev* fr, double* F, int k, int max_rows,
@@ -133,7 +132,6 @@ void launch_front_small(const int* flist, int nf, int maxN, const FrontDev* fr, 
 // Partial factorization of every front in flist by one cooperative persistent
 // launch over all SMs.  `slots` holds coop_slot_elems() elements of scratch;
 // `phase_pref` the per-phase work-item prefixes from coop_phase_prefix.
-bool coop_fits(int nf);
 size_t coop_slot_elems();
 std::vector<int> coop_phase_prefix(const std::vector<int>& n, const std::vector<int>& N, int maxn,
                                    int outer = 0);

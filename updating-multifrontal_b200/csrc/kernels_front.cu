@@ -1029,7 +1029,6 @@ bool small_front_fits(int maxN, int elem_bytes) {
   return (size_t)((maxN + 31) & ~31) * kPS * elem_bytes <= 200 * 1024;
 }
 
-bool coop_fits(int nf) { return nf <= kMaxCoopFronts; }
 size_t coop_slot_elems() { return (size_t)kMaxCoopFronts * kDiagSlot; }
 
 // Work items per phase of k_level_coop for fronts (n_i, N_i), in the kernel's
@@ -1086,7 +1085,7 @@ cudaError_t launch_level_coop(const int* flist, int nf, int maxn, const FrontDev
                               int max_items, int outer) {
   if (nf <= 0) return cudaSuccess;
   if (outer <= 0) outer = kOuter;
-  if (outer % kPanel || K0 % outer) return cudaErrorInvalidValue;
+  if (nf > kMaxCoopFronts || outer % kPanel || K0 % outer) return cudaErrorInvalidValue;
   cudaError_t me = cudaMemsetAsync(gbar, 0, sizeof(unsigned), st);
   if (me != cudaSuccess) return me;
   if (K1 < 0) K1 = maxn;

@@ -438,7 +438,7 @@ struct mfgpu_handle {
   std::vector<int> lvMaxN;   // largest front (n + m) per level
   std::vector<int> lvMaxn;   // largest pivot count per level
   int solveCoopMinN = 1024;  // levels with a front this large use the cooperative sweeps
-  bool stepped = false;      // MFGPU_STEPPED=1: per-step launches instead of the cooperative kernel
+  bool stepped = false;      // MFGPU_STEPPED=1: per-step launches instead of the tile kernel
   // Separator widths 2-3: the operators are nonsymmetric, every front is
   // stored whole and factored by pivoted LU (FP64), pivots in d_ipiv beside
   // each front's pivot DOFs.
@@ -547,7 +547,7 @@ struct mfgpu_handle {
       // tile tasks for every level of the full plan (the autotuner may time any
       // kernel), for the levels whose kernel they are otherwise; phase tables
       // for the tensor-core levels
-      if (fl.empty() || lu || !mfgpu::coop_fits((int)fl.size())) continue;
+      if (fl.empty() || lu) continue;
       std::vector<int> nn, NN;
       for (int f : fl) {
         nn.push_back(s.fronts[f].n);
@@ -731,7 +731,7 @@ struct mfgpu_handle {
     if (L.nf <= 0) return LK_NONE;
     if (lu) return LK_LU;
     if (useFused((int)L.nf, L.maxN)) return LK_FUSED;
-    if (!mfgpu::coop_fits((int)L.nf) || (stepped && !mixed)) return LK_STEPPED;
+    if (stepped && !mixed) return LK_STEPPED;
     if (mixed && tcLevel(L)) return LK_TC;
     if (panelFits(L)) return LK_PANEL;
     return LK_COOP;
@@ -756,7 +756,7 @@ struct mfgpu_handle {
     std::vector<int> c;
     if (L.nf <= 0) return c;
     if (mfgpu::small_front_fits(L.maxN, (int)esz)) c.push_back(LK_FUSED);
-    if (mfgpu::coop_fits((int)L.nf) && !(stepped && !mixed)) {
+    if (!(stepped && !mixed)) {
       c.push_back(LK_COOP);
       if (L.nf <= mfgpu::kMaxPanelFronts) c.push_back(LK_PANEL);
       if (mixed && tcCandidate(L)) c.push_back(LK_TC);
@@ -1104,7 +1104,9 @@ struct mfgpu_handle {
   // more than they spread (256 fronts of 77 x 49: 52 us against 64); the tile
   // kernel (k_front_tiles) otherwise, which also spreads the few large fronts
   // of an uneven level (FP64, one CTA per front against tiles: 256 fronts of
-  // 377 x 125 526 against 380 us, 4096 of 285 x 225 5.09 against 4.47 ms).
+  // 377 x 125 526 against 380 us, 4096 of 285 x 225 5.09 against 4.47 ms; the
+  // tiles take any number of fronts: 40 problems of 255^2, 10,240 such leaves,
+  // factor + solve 21.7 against 18.4 ms, 2D 2047^2, 16,384, a step 51.3 against 47.0).
   bool useFused(int nf, int maxN) const {
     return mfgpu::small_front_fits(maxN, (int)esz) &&
            ((nf >= fusedMinFronts && maxN <= fusedMaxN) || maxN <= 64);
@@ -1201,7 +1203,7 @@ struct mfgpu_handle {
     prof.flops[MFGPU_KC_COOP] += std::max(0.0, level_flops - tc_fl);
   }
 
-  // FP64 per-step launches (MFGPU_STEPPED=1, or levels no cooperative launch takes).
+  // FP64 per-step launches (MFGPU_STEPPED=1).
   void runStepped(const Plan& P, const Plan::Level& L) {
     const Schedule& s = *S;
     double* F = (double*)d_F;
