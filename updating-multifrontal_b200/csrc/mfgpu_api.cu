@@ -2399,7 +2399,8 @@ namespace {
 // 64-bit FNV-1a checksum of the payload (taken 8 bytes at a time).
 struct FacHeader {
   char magic[8];
-  uint32_t version, esz, mixed, pad;
+  uint32_t version, esz, mixed;
+  uint32_t dinv_set;  // checksum of the fronts that have block inverses (0: not recorded)
   int64_t n, nnz, front_elems, sep_elems, dinv_elems, nfronts, nseps;
   uint64_t pattern;   // checksum of row_ptr and col_ind
 };
@@ -2430,6 +2431,9 @@ FacHeader facHeader(const mfgpu_handle* h) {
   f.front_elems = h->S->front_elems;
   f.sep_elems = h->S->sep_elems;
   f.dinv_elems = h->dinvElems;
+  const uint64_t d = fnv64(kFnvBasis, (const unsigned char*)h->h_dinv_off.data(),
+                           h->h_dinv_off.size() * sizeof(int64_t));
+  f.dinv_set = std::max<uint32_t>(1u, (uint32_t)(d ^ (d >> 32)));
   f.nfronts = (int64_t)h->S->fronts.size();
   f.nseps = (int64_t)h->S->seps.size();
   uint64_t c = fnv64(kFnvBasis, (const unsigned char*)h->h_rowptr.data(), h->h_rowptr.size() * 4);
@@ -2517,8 +2521,9 @@ int mfgpu_load(mfgpu_handle* h, const char* path) {
     ck(cudaStreamSynchronize(h->stream), "sync before load");
     h->factored = false;
     // block inverses saved for another set of fronts (other sweep thresholds,
-    // an earlier build) are read over and formed anew
-    const bool same = hd.dinv_elems == me.dinv_elems;
+    // which may give sets of equal size; an earlier build) are read over and
+    // formed anew
+    const bool same = hd.dinv_elems == me.dinv_elems && hd.dinv_set == me.dinv_set;
     auto blocks = facBlocks(h);
     if (!same) {
       for (size_t i = 0; i < blocks.size();)
