@@ -38,7 +38,9 @@ enum mfgpu_status {
   MFGPU_ERR_PIVOT = 6,      /* non-positive pivot: matrix not SPD            */
   MFGPU_ERR_TIMEOUT = 7,    /* a bounded device wait gave up                 */
   MFGPU_ERR_STATE = 8,      /* call out of order (e.g. solve before factor)  */
-  MFGPU_ERR_NOT_CONVERGED = 9 /* mixed precision: refinement did not reach tol */
+  MFGPU_ERR_NOT_CONVERGED = 9 /* mixed precision: refinement did not reach tol for
+                                 some column (NaN or infinity included); the
+                                 output vectors are written all the same       */
 };
 
 enum mfgpu_precision {
@@ -69,6 +71,7 @@ typedef struct mfgpu_stats {
   int fronts;             /* fronts (boxes) refactored by the last factor/update */
   int iterations;         /* refinement iterations of the last mixed solve    */
   double residual;        /* last mixed solve: max_j ||b_j - A x_j|| / ||b_j|| */
+                          /* (NaN when one of them is not a number)           */
 } mfgpu_stats;
 
 void mfgpu_default_options(mfgpu_options* opts);

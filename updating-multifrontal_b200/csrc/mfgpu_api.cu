@@ -15,6 +15,7 @@
 #include <map>
 #include <tuple>
 #include <deque>
+#include <exception>
 #include <functional>
 #include <condition_variable>
 #include <thread>
@@ -1525,7 +1526,8 @@ struct mfgpu_handle {
     int it = 0, restarts = 0;
     bool first = true;
     double worst = 0;
-    // relative residual of every (segment, column); returns how many miss tol
+    // relative residual of every (segment, column); returns how many miss tol and
+    // can be improved (one that is not a number cannot: it ends in `worst`)
     auto check = [&]() {
       dots(d_R, d_R, nc, rr);
       ck(cudaMemcpyAsync(hr.data(), rr, G * sizeof(double), cudaMemcpyDeviceToHost, stream),
@@ -1535,7 +1537,7 @@ struct mfgpu_handle {
       worst = 0;
       for (int g = 0; g < G; g++) {
         const double rel = hb[g] > 0 ? std::sqrt(hr[g] / hb[g]) : std::sqrt(hr[g]);
-        worst = std::max(worst, rel);
+        if (std::isnan(rel) || rel > worst) worst = rel;   // (a NaN stays)
         act[g] = rel > tol;
         nact += act[g];
       }
@@ -1565,8 +1567,8 @@ struct mfgpu_handle {
       it++;
     }
     stats.iterations = std::max(stats.iterations, it);
-    stats.residual = std::max(stats.residual, worst);
-    if (worst > tol) {
+    if (std::isnan(worst) || worst > stats.residual) stats.residual = worst;
+    if (!(worst <= tol)) {
       char buf[160];
       snprintf(buf, sizeof buf,
                "refinement stopped after %d iterations at relative residual %.3e (target %.1e)", it,
@@ -2163,6 +2165,7 @@ static int solveOrApply(mfgpu_handle* h, const double* in, double* out, int nrhs
   if (nrhs == 0) return MFGPU_OK;
   return guarded(h, [&]() {
     const int chunk = 16;
+    std::exception_ptr missed;
     h->stats.iterations = 0;
     h->stats.residual = 0;
     h->clearErr();
@@ -2177,7 +2180,13 @@ static int solveOrApply(mfgpu_handle* h, const double* in, double* out, int nrhs
            "copy rhs in");
       if (!h->prof.verbose) h->prof.begin(apply ? MFGPU_KC_APPLY : MFGPU_KC_SOLVE, h->stream);
       if (apply) h->applyChunk(X, nc);
-      else h->solveChunk(X, nc);
+      else
+        try {
+          h->solveChunk(X, nc);
+        } catch (const CudaError& e) {   // some columns missed tol: the others are still handed out
+          if (e.status != MFGPU_ERR_NOT_CONVERGED) throw;
+          missed = missed ? missed : std::make_exception_ptr(e);
+        }
       if (!h->prof.verbose) h->prof.end(h->stream);
       if (h->prof.on) {
         // L11 (lower) and L21 are read once forward and once backward; the
@@ -2208,6 +2217,7 @@ static int solveOrApply(mfgpu_handle* h, const double* in, double* out, int nrhs
     double fl = 0;
     for (const mfgpu::Front& f : h->S->fronts) fl += 2.0 * ((double)f.n * f.n + 2.0 * f.n * f.m);
     h->stats.flops = fl * nrhs;
+    if (missed) std::rethrow_exception(missed);
   });
 }
 
