@@ -122,6 +122,7 @@ struct Plan {
   unsigned char* d_buf = nullptr;
   size_t cap = 0;
   std::vector<unsigned char> h_buf;
+  static constexpr size_t kOneCopy = (size_t)2 << 20;
 
   void release() {
     cudaFree(d_buf);
@@ -177,6 +178,26 @@ struct Plan {
     tpanel.push_back((int64_t)ttask.size());
   }
 
+  // Tiles of a task (lower: none above the diagonal).
+  static size_t tileCount(const Task& t) {
+    const int E = mfgpu::kTaskTile;
+    const size_t r = (t.rows + E - 1) / E, c = (t.cols + E - 1) / E;
+    return t.lower ? c * r - c * (c - 1) / 2 : c * r;
+  }
+
+  // Room for every task of the schedule and its tiles, so that the tables of a
+  // full plan are not moved while they grow.
+  void reserveAll(const Schedule& s) {
+    size_t nt = 0, ntiles = 0;
+    for (const std::vector<Task>* v : {&s.front_tasks, &s.sep_tasks, &s.sep_add_tasks}) {
+      nt += v->size();
+      const size_t step = v == &s.sep_add_tasks ? 2 : 1;   // (pairs: one list of tiles)
+      for (size_t t = 0; t < v->size(); t += step) ntiles += tileCount((*v)[t]);
+    }
+    tasks.reserve(nt);
+    tiles.reserve(ntiles);
+  }
+
   // A group is built by beginGroup, appendGroup (the tasks of some owners,
   // optionally rewritten by fx), endGroup.  pairs: the owners' tasks come in
   // pairs that one tile executes together, so the second one has no tiles.
@@ -200,9 +221,12 @@ struct Plan {
         if (fx) fx(tasks.back());
         if (pairs && t != a) continue;
         g.staged |= (T.kind == mfgpu::TK_COPY && T.trans) || (wide && T.kind == mfgpu::TK_SPARSE);
-        for (int j = 0; j * E < T.cols; j++)
-          for (int i = T.lower ? j : 0; i * E < T.rows; i++)   // (nothing above the diagonal)
-            tiles.push_back(make_int2(id, i | (j << 16)));
+        const int R = (T.rows + E - 1) / E, C = (T.cols + E - 1) / E;
+        const size_t at = tiles.size();
+        tiles.resize(at + tileCount(T));
+        int2* p = tiles.data() + at;
+        for (int j = 0; j < C; j++)
+          for (int i = T.lower ? j : 0; i < R; i++) *p++ = make_int2(id, i | (j << 16));
       }
     }
   }
@@ -219,16 +243,6 @@ struct Plan {
       return at;
     };
     const size_t o[6] = {place(tasks), place(tiles), place(ids), place(cpref), place(ttask), place(trow)};
-    h_buf.resize(need);
-    auto put = [&](size_t at, const auto& v) {
-      if (!v.empty()) std::memcpy(h_buf.data() + at, v.data(), v.size() * sizeof(v[0]));
-    };
-    put(o[0], tasks);
-    put(o[1], tiles);
-    put(o[2], ids);
-    put(o[3], cpref);
-    put(o[4], ttask);
-    put(o[5], trow);
     if (need > cap) {
       cudaFree(d_buf);
       d_buf = nullptr;
@@ -237,7 +251,23 @@ struct Plan {
       d_buf = dalloc<unsigned char>(c, "alloc plan");
       cap = c;
     }
-    if (need > 0)
+    // small plans (a localized update's) by one copy; large ones without a
+    // second host copy of their tables (3D 95^3: 57 MB, 30 -> 9 ms)
+    const bool one = need <= kOneCopy;
+    if (one) h_buf.resize(need);
+    auto put = [&](size_t at, const auto& v) {
+      if (v.empty()) return;
+      const size_t bytes = v.size() * sizeof(v[0]);
+      if (one) std::memcpy(h_buf.data() + at, v.data(), bytes);
+      else ck(cudaMemcpyAsync(d_buf + at, v.data(), bytes, cudaMemcpyHostToDevice, st), "upload plan");
+    };
+    put(o[0], tasks);
+    put(o[1], tiles);
+    put(o[2], ids);
+    put(o[3], cpref);
+    put(o[4], ttask);
+    put(o[5], trow);
+    if (one && need > 0)
       ck(cudaMemcpyAsync(d_buf, h_buf.data(), need, cudaMemcpyHostToDevice, st), "upload plan");
     d_tasks = reinterpret_cast<Task*>(d_buf + o[0]);
     d_tiles = reinterpret_cast<int2*>(d_buf + o[1]);
@@ -245,7 +275,7 @@ struct Plan {
     d_cpref = reinterpret_cast<int*>(d_buf + o[3]);
     d_ttask = reinterpret_cast<int*>(d_buf + o[4]);
     d_trow = reinterpret_cast<int*>(d_buf + o[5]);
-    // the host buffer must outlive the async copy
+    // the host tables must outlive the async copies
     ck(cudaStreamSynchronize(st), "plan upload");
   }
 };
@@ -357,9 +387,10 @@ struct mfgpu_handle {
   cudaGraphExec_t fullGraph = nullptr;
   std::map<std::tuple<const void*, const void*, int>, cudaGraphExec_t> sweepGraphs;
   std::map<std::tuple<const void*, const void*, int>, int> sweepSeen;
-  void* d_slots = nullptr;     // diagonal-block hand-off slots of the cooperative kernel
+  void* d_slots = nullptr;     // diagonal-block hand-off slots of the cooperative kernel (MFGPU_SUBPANEL=0)
   void* d_tcpack = nullptr;    // tensor-core panel images (mixed path)
-  void* d_pslot = nullptr;     // factored diagonal blocks of the panel-by-panel kernels
+  void* d_pslot = nullptr;     // factored diagonal blocks of the panel-by-panel kernels (MFGPU_PANEL_MAX_N,
+                               // the autotuner)
   size_t tcPackCap = 0;
   int* d_done = nullptr;       // finished block columns per block row + the tile kernel's task counter
   size_t capDone = 0;
@@ -432,7 +463,11 @@ struct mfgpu_handle {
   int nApplyCols = 0, nApplyRows = 0;
   int64_t woffTotal = 0;     // sum over fronts of 2N
   Plan full, upd;
+  Plan tune;                 // the full plan with the tables of every level's candidate kernels,
+                             // from the first mfgpu_autotune on (in a buffer of its own)
   std::vector<int> tuned;    // per level of the full plan: kernel picked by mfgpu_autotune, or -1
+  const Plan& fullPlan() const { return tuned.empty() ? full : tune; }
+  bool isFull(const Plan& P) const { return &P == &full || &P == &tune; }
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   int64_t device_bytes = 0;
   Profiler prof;
@@ -453,6 +488,7 @@ struct mfgpu_handle {
   ~mfgpu_handle() {
     if (stream) cudaStreamSynchronize(stream);
     full.release();
+    tune.release();
     upd.release();
     if (!view) {
       cudaFree(d_F);
@@ -513,6 +549,7 @@ struct mfgpu_handle {
   void buildPlan(Plan& P, const std::vector<char>& dirtyFront) {
     const Schedule& s = *S;
     P.clear(s.levels);
+    if (isFull(P)) P.reserveAll(s);
     for (int ell = s.levels - 1; ell >= 0; ell--) {
       Plan::Level& L = P.lv[ell];
       std::vector<int> fl, sl;
@@ -545,22 +582,23 @@ struct mfgpu_handle {
       P.appendGroup(L.sadd, s.sep_add_tasks, s.sep_task_ptr, sl, true, longRows);
       P.endGroup(L.sadd);
       L.cpref0 = (int64_t)P.cpref.size();
-      // tile tasks for every level of the full plan (the autotuner may time any
-      // kernel), for the levels whose kernel they are otherwise; phase tables
-      // for the tensor-core levels
+      // tile tasks and, for the tensor-core levels, panel tiles or phase tables
+      // of the levels whose kernel they are; in the autotuner's plan of every
+      // level that could take them
       if (fl.empty() || lu) continue;
       std::vector<int> nn, NN;
       for (int f : fl) {
         nn.push_back(s.fronts[f].n);
         NN.push_back(s.fronts[f].N);
       }
-      if (&P == &full || ruleKernel(L) == LK_COOP) P.addTiles(L, nn, NN);
+      const bool all = &P == &tune;
+      if (all || ruleKernel(L) == LK_COOP) P.addTiles(L, nn, NN);
       const bool tc = mixed && tcLevel(L);
-      if ((tc || (mixed && &P == &full && tcCandidate(L))) && subpanel) {
+      if ((tc || (mixed && all && tcCandidate(L))) && subpanel) {
         const int W = mfgpu::tc_outer();
         P.addPanelTiles(L, nn, NN, W);
         if (tc) P.tcPackBytes = std::max(P.tcPackBytes, packBytes(nn, NN, L.maxn, W));
-      } else if (tc || (mixed && &P == &full && tcCandidate(L))) {
+      } else if (tc || (mixed && all && tcCandidate(L))) {
         const int W = mfgpu::tc_outer();
         L.coopOuter = tc && tcSub > 0 && tcSub < W ? tcSub : 0;
         std::vector<int> pp = mfgpu::coop_phase_prefix(nn, NN, L.maxn, L.coopOuter);
@@ -739,7 +777,7 @@ struct mfgpu_handle {
   }
 
   int levelKernel(const Plan& P, const Plan::Level& L, int ell) const {
-    if (&P == &full && ell < (int)tuned.size() && tuned[ell] != LK_NONE && L.nf > 0)
+    if (isFull(P) && ell < (int)tuned.size() && tuned[ell] != LK_NONE && L.nf > 0)
       return tuned[ell];
     return ruleKernel(L);
   }
@@ -860,6 +898,21 @@ struct mfgpu_handle {
     tcPackCap = bytes;
   }
 
+  // Scratch of the kernels that only a switch or the autotuner reaches.
+  void ensureCoopSlots() {
+    if (mixed && !subpanel && !d_slots)
+      d_slots = dalloc<unsigned char>(mfgpu::coop_slot_elems() * esz, "alloc diagonal slots");
+  }
+  void ensurePanelSlots() {
+    if (d_pslot) return;
+    int most = 1;   // fronts of one launch
+    if (view) most = mfgpu::kMaxPanelFronts;   // a batch of requests: several copies of a level
+    else
+      for (int ell = 0; ell < S->levels; ell++) most = std::max(most, S->lv[ell].nbox);
+    d_pslot = dalloc<unsigned char>(mfgpu::panel_slot_bytes(most, (int)esz),
+                                    "alloc panel diagonal slots");
+  }
+
   void ensureDone(const Plan& P) {
     const size_t need = (size_t)P.maxRows + 1;
     if (need <= capDone) return;
@@ -971,13 +1024,13 @@ struct mfgpu_handle {
   void runPlanT(const Plan& P) {
     const Schedule& s = *S;
     size_t pack = P.tcPackBytes;   // tuned tensor-core levels may need more than the rules
-    if (&P == &full)
+    if (isFull(P))
       for (int ell = 0; ell < s.levels && ell < (int)tuned.size(); ell++)
         if (tuned[ell] == LK_TC) pack = std::max(pack, levelPackBytes(P, P.lv[ell]));
     ensurePack(pack);
     ensureDone(P);
     // the full factorization's schedule as one graph, from its second run on
-    if (&P == &full && graphs && !prof.on && fullRuns++ > 0) {
+    if (isFull(P) && graphs && !prof.on && fullRuns++ > 0) {
       if (!fullGraph) fullGraph = capture([&] { enqueuePlanT<T>(P); });
       if (fullGraph) {
         ck(cudaGraphLaunch(fullGraph, stream), "launch factorization graph");
@@ -1051,7 +1104,12 @@ struct mfgpu_handle {
   template <class T>
   void autotuneT(int reps, int* choices) {
     const Schedule& s = *S;
-    const Plan& P = full;
+    if (!tune.d_buf) {
+      buildPlan(tune, std::vector<char>(s.fronts.size(), 1));
+      tune.upload(stream);
+    }
+    ensurePanelSlots();
+    const Plan& P = tune;
     tuned.assign(s.levels, LK_NONE);
     size_t pack = P.tcPackBytes;
     for (int ell = 0; ell < s.levels; ell++)
@@ -1261,7 +1319,7 @@ struct mfgpu_handle {
   void rowScales(const Plan& P) {
     if (!mixed) return;
     bool any = P.tcPackBytes > 0;
-    if (&P == &full)
+    if (isFull(P))
       for (int k : tuned) any |= k == LK_TC;
     if (!any) return;
     mfgpu::launch_row_scale(d_rp, d_ci, d_val, n, nmat, nnz, d_scale, d_rscale, stream);
@@ -1973,13 +2031,8 @@ int createFrom(std::unique_ptr<Schedule> sched, int n, const int* row_ptr, const
     H.d_woff = dalloc<int64_t>(woff.size(), "alloc woff");
     H.d_err = dalloc<DevError>(1, "alloc error word");
     ck(cudaMemset(H.d_err, 0, sizeof(DevError)), "clear error word");
-    H.d_slots = dalloc<unsigned char>(mfgpu::coop_slot_elems() * H.esz, "alloc diagonal slots");
-    {
-      int most = 1;   // fronts of the largest level (panel launches take up to kMaxPanelFronts)
-      for (int ell = 0; ell < s.levels; ell++) most = std::max(most, s.lv[ell].nbox);
-      H.d_pslot = dalloc<unsigned char>(mfgpu::panel_slot_bytes(most, (int)H.esz),
-                                        "alloc panel diagonal slots");
-    }
+    H.ensureCoopSlots();
+    if (H.panelMaxN > 0) H.ensurePanelSlots();
     H.d_gbar = dalloc<unsigned>(1, "alloc grid barrier");
     H.d_all = dalloc<int>(all.size(), "alloc id list");
     if (!H.lu) {
@@ -2031,7 +2084,7 @@ static int factorImpl(mfgpu_handle* h, const double* val, int64_t nnz, bool devi
   return guarded(h, [&]() {
     h->factored = false;
     ck(cudaEventRecord(h->ev0, h->stream), "event");
-    h->factorWith(val, device, h->full, true);
+    h->factorWith(val, device, h->fullPlan(), true);
     ck(cudaEventRecord(h->ev1, h->stream), "event");
     h->checkDevError();
     float ms = 0;
@@ -2108,14 +2161,14 @@ static int updateImpl(mfgpu_handle* h, const double* val, int64_t nnz, const int
     std::vector<char> dirty;
     const size_t ndirty = s.dirty_fronts(mod, nmod, dirty);
     ck(cudaEventRecord(h->ev0, h->stream), "event");
-    const Plan* P = &h->full;
+    const Plan* P = &h->fullPlan();
     if (ndirty < s.fronts.size()) {
       h->buildPlan(h->upd, dirty);
       h->upd.upload(h->stream);
       P = &h->upd;
     }
     h->factored = false;
-    h->factorWith(val, device, *P, P == &h->full);
+    h->factorWith(val, device, *P, h->isFull(*P));
     ck(cudaEventRecord(h->ev1, h->stream), "event");
     h->checkDevError();
     h->factored = true;
@@ -3156,9 +3209,8 @@ std::unique_ptr<mfgpu_handle> makeView(mfgpu_handle& B) {
   H.d_err = dalloc<DevError>(1, "alloc error word");
   ck(cudaMemsetAsync(H.d_err, 0, sizeof(DevError), H.stream), "clear error word");
   H.setLimit(B.waitLimit);   // the base's poll limit
-  H.d_slots = dalloc<unsigned char>(mfgpu::coop_slot_elems() * H.esz, "alloc diagonal slots");
-  H.d_pslot = dalloc<unsigned char>(mfgpu::panel_slot_bytes(mfgpu::kMaxPanelFronts, (int)H.esz),
-                                    "alloc panel diagonal slots");
+  H.ensureCoopSlots();
+  if (H.panelMaxN > 0) H.ensurePanelSlots();
   H.d_gbar = dalloc<unsigned>(1, "alloc grid barrier");
   H.dinvElems = B.dinvElems;
   H.d_dinv_off = B.d_dinv_off;
