@@ -1,10 +1,11 @@
 """GPU: what a handle reserves.  The scratch and the tables of kernels that only
 a switch or the autotuner reaches are made for those alone, and are there when
 they are: in handles, in serving views and after an autotuning factorization."""
+import numpy as np
 import pytest
 import torch
 
-from mfgpu import MF2D, MFGPU_FP64, MFGPU_MIXED, Server, stencil
+from mfgpu import MF2D, MFGPU_FP64, MFGPU_MIXED, Server, Symbolic, stencil
 from problems import patch_update, problem, rel
 
 pytestmark = pytest.mark.gpu
@@ -61,3 +62,23 @@ def test_autotune_again_between_factorizations_and_updates():
         assert rel(F.Solve(b[0]), x2) < 1e-12
         F.Update(A, mod)
         assert rel(F.Solve(b[0]), x) < 1e-12
+
+
+def test_a_solve_reserves_its_vectors_and_workspace_only():
+    """One right-hand side, FP64: the front workspace (2 N per front) and one
+    vector; the second vector is the LU fronts' apply alone."""
+    size = (511, 511)
+    _, A, b = problem(2, size, seed=84)
+    F = MF2D(A, *size, 1, 8)
+    F.Factor()
+    F.Solve(b[0])
+    torch.cuda.synchronize()
+    free0 = torch.cuda.mem_get_info()[0]
+    F.Solve(np.ascontiguousarray(np.tile(b, (16, 1)).T))
+    torch.cuda.synchronize()
+    held = free0 - torch.cuda.mem_get_info()[0]
+    sym = Symbolic(2, size, 1, 8)
+    work = sum(2 * (f["n"] + f["m"]) for f in map(sym.front, range(sym.n_fronts)))
+    # 16 right-hand sides in place of one: 15 more of each, and the allocator's
+    # 2 MiB granules; a second vector would add 15 n doubles, 31 MB
+    assert held <= 8 * 15 * (work + A.n) + (8 << 20), (held, 8 * 15 * work, 8 * 15 * A.n)

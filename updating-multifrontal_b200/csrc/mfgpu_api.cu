@@ -414,7 +414,7 @@ struct mfgpu_handle {
   int64_t* d_dinv_off = nullptr;   // per front: element offset in d_Dinv, -1 outside those levels
   std::vector<int64_t> h_dinv_off; // host copy
   int64_t dinvElems = 0;
-  // solve workspaces (d_Wd / d_Td hold elements of the factor's precision)
+  // solve workspaces (d_Wd holds elements of the factor's precision; d_Td: apply of LU fronts)
   double* d_Wd = nullptr;
   size_t capW = 0;
   double* d_X = nullptr;
@@ -1381,7 +1381,7 @@ struct mfgpu_handle {
   void ensureWork(int nrhs) {
     growBuf(d_Wd, capW, (size_t)woffTotal * nrhs * esz / sizeof(double) + 1, "alloc solve workspace");
     growBuf(d_X, capX, (size_t)n * nrhs, "alloc rhs buffer");
-    growBuf(d_Td, capT, (size_t)n * nrhs * esz / sizeof(double) + 1, "alloc apply buffer");
+    if (lu) growBuf(d_Td, capT, (size_t)n * nrhs, "alloc apply buffer");
     if (mixed) {
       const size_t v = (size_t)n * nrhs;
       growBuf(d_B, capB, v, "alloc refinement buffer");
