@@ -207,8 +207,8 @@ cudaError_t launch_trail_tc(const int* flist, int nf, int64_t ntiles, const Fron
                             DevError* err, cudaStream_t st, const float* rscale = nullptr,
                             const int* dofs = nullptr);
 
-// Cooperative sweeps over all fronts of one level (nrhs <= 16), ordered by
-// ready flags instead of grid barriers: forward = L11 solve and boundary update
+// Sweeps over all fronts of one level (nrhs <= 16) by one cooperative launch,
+// ordered by ready flags instead of grid barriers: forward = L11 solve and boundary update
 // b_bd -= L21 y, backward = L21^T update and L11^T solve, both gathering from
 // and scattering to X themselves.  flow_tasks builds a level's task lists
 // (front slot, block) pairs, forward R-major and backward by distance from
@@ -228,7 +228,7 @@ cudaError_t launch_solve_flow(bool forward, const int* flist, const FrontDev* fr
                               const int64_t* woff, const T* Dv, const int64_t* dinv_off,
                               const int* tasks, int ntasks, const int* flagoff, int* flags,
                               int nflags, bool chain, DevError* err, cudaStream_t st);
-constexpr int kDinvBlock = 64;   // diagonal-block size of the cooperative sweeps
+constexpr int kDinvBlock = 64;   // diagonal-block size of the flag-ordered sweeps
 template <class T>
 void launch_diag_inv(const int* flist, int nf, int maxn, const FrontDev* fr, const T* F, T* Dv,
                      const int64_t* dinv_off, cudaStream_t st);

@@ -459,7 +459,7 @@ __device__ __forceinline__ void row_trsm(double (&x)[kPanel], const double (*L)[
 }
 
 // ---------------------------------------------------------------------------
-// Fused partial factorization, one CTA per front (fronts up to kSmallMaxN).
+// Fused partial factorization, one CTA per front (small_front_fits).
 // The panel of each step is staged in shared memory for the tensor-core update.
 // ---------------------------------------------------------------------------
 template <class T, int NT>
@@ -615,7 +615,8 @@ __global__ void __launch_bounds__(128) k_syrk(const int* __restrict__ flist,
 }
 
 // ---------------------------------------------------------------------------
-// Large fronts: one cooperative persistent launch per level.  Two-level
+// The tensor-core levels' sub-panels under MFGPU_SUBPANEL=0: one cooperative
+// persistent launch.  Two-level
 // blocking: outer panels of `outer` columns (kOuter = 512 unless the caller
 // asks for narrower ones); inside each, 32-column steps
 //   A  triangular solve of the rows below the diagonal block (every work item

@@ -22,7 +22,7 @@
 // On exit rows/cols [0,n) hold L11 (unit lower) and U11 with P A22 = L11 U11,
 // rows [n,N) x cols [0,n) hold L21 = A12 U11^{-1}, rows [0,n) x cols [n,N)
 // hold U12 = L11^{-1} P A21 and the trailing block S + A11.  So XL = L21
-// L11^{-1} P and XR = U11^{-1} U12, and the solve / apply sweeps
+// L11^{-1} P and XR = U11^{-1} U12, and the solve (kernels_sweep.cu) and apply
 // (kernels_front.cu) use the factors directly.  ipiv[j] (front-relative row)
 // is stored beside the front's pivot DOFs.  A zero pivot column (the pivot
 // block is singular) records error code 4.

@@ -1,6 +1,6 @@
-// Cooperative forward / backward sweeps for the levels of large fronts.
+// Flag-ordered forward / backward sweeps for the levels of large fronts.
 //
-// The one-CTA-per-front sweeps (kernels_front.cu) serialise a front's whole
+// The one-CTA-per-front sweeps (kernels_sweep.cu) serialise a front's whole
 // triangular solve on one SM, which leaves a level of a few large fronts (the
 // top of a 3D tree, the root of every problem) far below HBM bandwidth.  These
 // kernels spread every front of a level over all SMs with one persistent
@@ -16,10 +16,10 @@
 //   task per 64-column pivot block accumulates L(rows below, block)^T x over
 //   the boundary rows and the solved blocks after it, then x = L_bb^{-T}(...)
 //   and the flag.
-// The inverses (k_diag_inv, after each factorization of the level) take the
-// sequential substitution out of every block; the chain of dependent blocks
-// costs one flag hand-off and two 64 x 64 products per block, and the rest of
-// the work (every element of L read once) overlaps it.
+// The inverses (left by the tile kernel; k_diag_inv after the other kernels and
+// for loaded factors) take the sequential substitution out of every block; the
+// chain of dependent blocks costs one hand-off and two 64 x 64 products per
+// block, and the rest of the work (every element of L read once) overlaps it.
 //
 // W is the front's right-hand-side block (N x nrhs, ld N) in the same
 // workspace the per-front kernels use, so the separator gathers between
@@ -48,7 +48,7 @@ constexpr int kMaxSolveCoopFronts = 1024;
 
 __host__ __device__ __forceinline__ int cdiv(int a, int b) { return (a + b - 1) / b; }
 
-// Diagonal-block inverses of the cooperative levels' pivot blocks: block b of
+// Diagonal-block inverses of the flag-ordered sweeps' pivot blocks: block b of
 // front f (rows and columns [64 b, 64 b + kb)) gets Dinv = L_bb^{-1} (lower,
 // column-major 64 x 64, zero outside kb x kb) at Dv + dinv_off[f] + b * 8192
 // and its transpose right after it.  Column t of the inverse is computed by
@@ -161,8 +161,8 @@ __device__ __forceinline__ T ldcg(const T* p) {
 // rows from n) are tasks, listed R-major across the fronts; CTAs take them
 // round-robin.  Task (i, R) accumulates L(rows, block j) y_j over the pivot
 // column blocks j before it as their ready flags come up, then a pivot block
-// forms y_R = Dinv_R (b_R - acc), writes it to X and to the front's second
-// workspace half (Y) and raises its flag; a boundary block leaves -acc in W
+// forms y_R = Dinv_R (b_R - acc), writes it to X and to the launch's scratch (Y)
+// and raises its flag; a boundary block leaves -acc in W
 // for the separator gather.  Everything the last dependency does not change -
 // its L block, the block's row of the inverse, the right-hand side - is in
 // registers before the task waits for it, so a step of the chain of dependent

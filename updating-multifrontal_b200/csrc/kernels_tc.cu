@@ -103,7 +103,7 @@ constexpr int IMG = TM * TK * 4;           // one image of 128 rows x 64 bytes, 
 constexpr int STAGE_BYTES = 6 * IMG;       // a_hi, a_lo, b_hi (2 blocks), b_lo (2 blocks)
 constexpr int kTcSmem = NSTAGE * STAGE_BYTES + 1024;   // + alignment slack
 constexpr int kMaxTcFronts = 1024;
-constexpr int kTcOuter = 512;              // outer panel width (the cooperative kernel's)
+constexpr int kTcOuter = 512;              // outer panel width
 constexpr uint32_t kSpinLimit = 1u << 24;
 
 // Image layout (K-major, 64-byte swizzle): element (m, k) of a 128 x 16 image

@@ -395,7 +395,7 @@ struct mfgpu_handle {
   int* d_done = nullptr;       // finished block columns per block row + the tile kernel's task counter
   size_t capDone = 0;
   unsigned* d_gbar = nullptr;  // grid-barrier arrival counter of the cooperative kernels
-  // Cooperative (flag-ordered) sweeps: per level, its forward / backward task
+  // Flag-ordered sweeps: per level, its forward / backward task
   // lists and flag offsets in d_flow; the ready flags of one launch in d_flags.
   // In a level of more fronts than one flow launch takes, its large fronts
   // (`list`, in d_flow) go there and the others (`rest`) to the per-front sweeps.
@@ -410,8 +410,8 @@ struct mfgpu_handle {
   int* d_flow = nullptr;       // shared with serving-loop views
   int* d_flags = nullptr;      // per handle (views have their own)
   int maxFlags = 0;
-  void* d_Dinv = nullptr;      // inverses of the cooperative-sweep levels' 64 x 64 pivot blocks
-  int64_t* d_dinv_off = nullptr;   // per front: element offset in d_Dinv, -1 outside those levels
+  void* d_Dinv = nullptr;      // inverses of the flag-ordered sweeps' 64 x 64 pivot blocks
+  int64_t* d_dinv_off = nullptr;   // per front: element offset in d_Dinv, -1: none
   std::vector<int64_t> h_dinv_off; // host copy
   int64_t dinvElems = 0;
   // solve workspaces (d_Wd holds elements of the factor's precision; d_Td: apply of LU fronts)
@@ -424,7 +424,7 @@ struct mfgpu_handle {
   // mixed precision: scaling and refinement buffers
   bool mixed = false;
   int tcMinN = 4096;               // mixed: smallest level maxN run on the tensor cores (0 = never)
-  int tcSplit = 3;                 // mixed: 3 = three-term TF32 products, 1 = plain TF32, 2 = BF16
+  int tcSplit = 3;                 // mixed: 3 = three-term FP16 products, 1 = plain TF32, 2 = BF16
   int tcSplit3Levels = -1;         // >= 0: tcSplit only on the top levels 0 .. this - 1,
   int tcSplitLow = 1;              //   tcSplitLow (plain TF32 or BF16) below them
   int tcSub = 128;                 // mixed: sub-panel width inside each 512-column outer panel of a
@@ -473,7 +473,7 @@ struct mfgpu_handle {
   Profiler prof;
   std::vector<int> lvMaxN;   // largest front (n + m) per level
   std::vector<int> lvMaxn;   // largest pivot count per level
-  int solveCoopMinN = 1024;  // levels with a front this large use the cooperative sweeps
+  int solveCoopMinN = 1024;  // front rows from which levels use the flag-ordered sweeps (flowMinRhs)
   bool stepped = false;      // MFGPU_STEPPED=1: per-step launches instead of the tile kernel
   // Separator widths 2-3: the operators are nonsymmetric, every front is
   // stored whole and factored by pivoted LU (FP64), pivots in d_ipiv beside
@@ -783,9 +783,7 @@ struct mfgpu_handle {
   }
 
   // Levels of moderate fronts (up to panelMaxN) go panel by panel
-  // (k_diag_factor + k_panel_trsm + k_trail_syrk, no grid barriers); the cooperative kernel's
-  // 512-column outer panels keep the trailing updates of very large fronts
-  // denser.
+  // (k_diag_factor + k_panel_trsm + k_trail_syrk, no grid barriers).
   bool panelFits(const Plan::Level& L) const {
     return panelMaxN > 0 && L.maxN <= panelMaxN && L.nf <= mfgpu::kMaxPanelFronts;
   }
@@ -926,7 +924,7 @@ struct mfgpu_handle {
   }
 
   // Partial factorization of the fronts of level ell with kernel `kind`, and
-  // the block inverses of the cooperative sweeps (which the tile kernel leaves
+  // the block inverses of the flag-ordered sweeps (which the tile kernel leaves
   // itself).
   template <class T>
   void runLevelKernel(const Plan& P, const Plan::Level& L, int ell, int kind) {
@@ -1171,9 +1169,8 @@ struct mfgpu_handle {
            ((nf >= fusedMinFronts && maxN <= fusedMaxN) || maxN <= 64);
   }
 
-  // Mixed path: levels of large fronts run the cooperative kernel one outer
-  // panel at a time (diagonal blocks, panel solves and in-panel updates) and
-  // the trailing update of each panel on the tensor cores.
+  // Mixed path: levels of large fronts are factored one outer panel at a time,
+  // the panel by FP32 tiles and the trailing update on the tensor cores.
   // A level also goes to the tensor cores with fronts of a quarter of tcMinN
   // when it has at least one front per SM (enough tiles to fill the GPU; 3D
   // 127^3 level 3: 512 fronts, N <= 1981), unless their panels fit one CTA's
@@ -1969,7 +1966,7 @@ int createFrom(std::unique_ptr<Schedule> sched, int n, const int* row_ptr, const
       H.dinvElems = cur;
       H.h_dinv_off = doff;
       H.d_Dinv = dalloc<unsigned char>(std::max<int64_t>(cur, 1) * H.esz, "alloc block inverses");
-      // task lists of the cooperative sweeps, per level
+      // task lists of the flag-ordered sweeps, per level
       std::vector<int> tab;
       H.flow.assign(s.levels, mfgpu_handle::FlowLevel());
       for (int ell = 0; ell < s.levels; ell++) {
@@ -2341,7 +2338,7 @@ int mfgpu_solve_device_noalloc(mfgpu_handle* h, const double* d_b, double* d_x, 
   return guarded(h, [&]() {
     double* W = noallocScratch(h->device);
     const int chunk = (int)std::min<int64_t>(16, (int64_t)kNoAllocScratchDoubles / per_rhs);
-    // the error word reports a cooperative sweep's grid barrier that gave up
+    // the error word reports a flag-ordered sweep's wait that gave up
     h->clearErr();
     ck(cudaEventRecord(h->ev0, h->stream), "event");
     for (int c0 = 0; c0 < nrhs; c0 += chunk) {
